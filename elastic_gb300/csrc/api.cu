@@ -197,8 +197,9 @@ void upload_structure(elx_ctx *c, bool prederived) {
   for (auto &row : c->tuned_unroll)
     for (int &u : row) u = 0;
   for (DBuf *v : {&c->node_count, &c->tstress, &c->tx0buf, &c->fbuf, &c->ld_node, &c->ld_ptr,
-                  &c->ld_ent, &c->ld_vec, &c->vtkbuf})
+                  &c->ld_ent, &c->ld_vec, &c->vtkbuf, &c->persist_cta, &c->persist_sync})
     c->release(*v);
+  c->persist_grid = 0;
   c->have_stress = false;
   release_partitions(c);
   c->have_fp32 = false;
@@ -452,6 +453,33 @@ void set_scalars(elx_ctx *c, double tol, int maxit) {
                            c->stream));
 }
 
+// The cooperative PCG, kPersistSteps iterations a launch, until it has stopped
+// (two launches in flight: the second returns at once when the first stopped).
+constexpr int kPersistSteps = 512;
+elx::PcgScalars run_persist(elx_ctx *c, int maxit) {
+  const int max_launches = maxit / kPersistSteps + 2;
+  int launched = 0, checked = 0;
+  auto launch = [&](int slot) {
+    persist_steps(c, kPersistSteps);
+    ELX_CUDA(cudaMemcpyAsync(&c->h_scal[slot], c->scal.p, sizeof(elx::PcgScalars),
+                             cudaMemcpyDeviceToHost, c->stream));
+    ELX_CUDA(cudaEventRecord(c->ev[slot], c->stream));
+    launched++;
+  };
+  launch(0);
+  for (;;) {
+    if (launched < max_launches) launch(launched & 1);
+    const int slot = checked & 1;
+    ELX_CUDA(cudaEventSynchronize(c->ev[slot]));
+    checked++;
+    if (c->h_scal[slot].done || checked == launched) {
+      const elx::PcgScalars last = c->h_scal[slot];
+      c->sync();
+      return last;
+    }
+  }
+}
+
 void pcg64(elx_ctx *c, double tol, int maxit, elx_info *info) {
   auto t0 = std::chrono::steady_clock::now();
   build_preconditioner(c);
@@ -461,9 +489,13 @@ void pcg64(elx_ctx *c, double tol, int maxit, elx_info *info) {
                                 c->scal.as<elx::PcgScalars>(), c->partials.as<double>(),
                                 c->counters.as<unsigned int>() + 2, c->stream);
   c->launches += 1;
-  capture_pcg_graph(c);
-  elx::PcgScalars last =
-      run_batches(c, c->pcg_graph, c->spmv_kind == elx::kSpmvTiled ? 4 : 3, maxit);
+  elx::PcgScalars last;
+  if (ensure_persist(c)) {
+    last = run_persist(c, maxit);
+  } else {
+    capture_pcg_graph(c);
+    last = run_batches(c, c->pcg_graph, c->spmv_kind == elx::kSpmvTiled ? 4 : 3, maxit);
+  }
   post_diagnostics(c);
   const double secs =
       std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -1177,6 +1209,7 @@ void elx_destroy(elx_ctx *c) {
                   &c->sell_val, &c->sell_val64, &c->sell_d16,
                   &c->node_count, &c->tstress, &c->tx0buf, &c->fbuf, &c->ld_node, &c->ld_ptr,
                   &c->ld_ent, &c->ld_vec, &c->vtkbuf,
+                  &c->persist_cta, &c->persist_sync,
                   &c->u, &c->b0, &c->b, &c->xs, &c->r, &c->p, &c->q, &c->m, &c->z,
                   &c->scal, &c->partials, &c->counters, &c->flags, &c->diag})
     c->release(*d);

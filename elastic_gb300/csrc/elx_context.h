@@ -95,6 +95,12 @@ struct elx_ctx {
   double *h_diag = nullptr;           // pinned
   int32_t *h_flags = nullptr;         // pinned
 
+  // cooperative PCG (persist.cu): blocks (0: not planned, -1: not used), their
+  // slices and the blocks' shared words
+  DBuf persist_cta, persist_sync;
+  int persist_grid = 0, persist_rows = 0, persist_slices = 0;
+  bool persist_smem = false;
+
   int64_t launches = 0;  // kernels of this library launched by this context
 
   cudaGraphExec_t pcg_graph = nullptr;    // kBatch FP64 PCG iterations
@@ -224,6 +230,9 @@ void upload_structure(elx_ctx *c, bool prederived = false);
 void assemble_resident(elx_ctx *c);
 void build_preconditioner(elx_ctx *c);
 void release_block(elx_ctx *c);
+// Cooperative PCG (persist.cu).
+bool ensure_persist(elx_ctx *c);
+void persist_steps(elx_ctx *c, int steps);
 // Row-block partitions on one device (partition.cu).
 void ensure_partitions(elx_ctx *c, int nparts);
 void release_partitions(elx_ctx *c);

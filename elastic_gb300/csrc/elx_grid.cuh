@@ -1,0 +1,272 @@
+// Grid-wide sums and barriers inside one cooperative launch (persist.cu).
+//
+// A sum over the blocks is one integer atomic per digit: every block adds its
+// partial, cut into five 32-bit digits of a 160-bit window, to five words in
+// L2, and polls them until all blocks have added (each word counts its
+// additions in its upper bits).  Integer adds commute, so the total is the same
+// whatever the order, and every block reads the same total one L2 round trip
+// after the slowest block arrives: 1,500 clocks on 152 blocks, where slots
+// written by every block and polled by all take 2,800 to 4,200 and a last
+// block that adds the partials a fence, an atomic and two more round trips.
+// The words are never reset: a total is their difference from the last one.
+//
+// The window reaches 32 bits above the sum's reference (the last residual's
+// norm) and 120 below.  A partial above it, an infinity or a NaN marks the
+// sum, and all blocks repeat it through slots, each with its own exponent.
+#pragma once
+
+#include <cstdint>
+
+#include "elx_ptx.cuh"
+#include "elx_reduce.cuh"
+
+namespace elx {
+
+constexpr int kGridMaxBlocks = 160;
+constexpr uint64_t kGridWaitNs = 2000000000ull;  // bound of every grid wait
+constexpr int kDigits = 5;
+
+// Shared by the blocks of a launch; zeroed before each launch.
+struct alignas(128) GridWords {
+  unsigned long long digit[16];  // kDigits used
+};
+struct alignas(16) GridSlot {
+  int64_t m;
+  uint64_t tag;  // epoch << 24 | exponent + 4096
+};
+struct GridSync {
+  GridWords sum[2];  // (p, q) and (r, z)
+  GridWords arrive;  // digit[0]: arrivals at the barrier
+  GridSlot slot[kGridMaxBlocks];
+};
+
+namespace grid {
+
+__device__ __forceinline__ unsigned long long load_relaxed(const unsigned long long *p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void red_add(unsigned long long *p, unsigned long long v) {
+  asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+__device__ __forceinline__ void store_slot(GridSlot *s, int64_t m, uint64_t tag) {
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\t"
+      "st.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(s),
+      "l"(m), "l"(tag)
+      : "memory");
+}
+
+__device__ __forceinline__ GridSlot load_slot(const GridSlot *s) {
+  GridSlot r;
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\t"
+      "mov.b128 {%0, %1}, t;\n\t}"
+      : "=l"(r.m), "=l"(r.tag)
+      : "l"(s)
+      : "memory");
+  return r;
+}
+
+__device__ __forceinline__ void fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
+// Counts polls and bounds them by the GPU's clock.
+struct Bound {
+  uint64_t t0 = 0;
+  uint32_t it = 0;
+  __device__ __forceinline__ bool over() {
+    if (++it & 1023u) return false;
+    const uint64_t now = ptx::global_ns();
+    if (!t0) t0 = now;
+    return now - t0 > kGridWaitNs;
+  }
+};
+
+// Every block's f through its slot (value, exponent and epoch in one 16-byte
+// store); warp 0.
+__device__ __forceinline__ bool slot_sum(GridSlot *slots, FixSum &f, uint64_t epoch) {
+  constexpr int K = kGridMaxBlocks / 32;
+  const int lane = threadIdx.x & 31;
+  if (lane == 0)
+    store_slot(slots + blockIdx.x, f.m, epoch << 24 | (uint64_t)(uint32_t)(f.e + 4096));
+  FixSum v[K];
+  bool ok = true;
+  Bound bound;
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    v[k].m = 0;
+    v[k].e = -4096;
+    const int b = lane + 32 * k;
+    while (b < (int)gridDim.x && ok) {
+      const GridSlot g = load_slot(slots + b);
+      if (g.tag >> 24 == epoch) {
+        v[k].m = g.m;
+        v[k].e = (int32_t)(g.tag & 0xffffffu) - 4096;
+        break;
+      }
+      ok = !bound.over();
+    }
+  }
+  ok = __all_sync(0xffffffffu, ok);
+  int e = v[0].e;
+#pragma unroll
+  for (int k = 1; k < K; k++) e = max(e, v[k].e);
+  FixSum t;
+  t.m = 0;
+#pragma unroll
+  for (int k = 0; k < K; k++) t.m += v[k].m >> min(e - v[k].e + 3, 63);
+  t.e = e + 3;
+  f = warp_sum(t);
+  return ok;
+}
+
+// Exponent of a window's lowest bit for sums near |ref|.
+__device__ __forceinline__ int window_of(double ref) {
+  const int ex = (int)((uint64_t)__double_as_longlong(ref) >> 52) & 0x7ff;
+  return ex - 1023 - 120;
+}
+
+// The blocks' sum of f (warp 0, every lane the same f): digits of 2^lo.
+// `seen` holds this lane's word after the last sum.  False in every lane when
+// the bound ran out.
+__device__ __forceinline__ bool digit_sum(GridSync *gs, GridWords *words, FixSum &f, int lo,
+                                          unsigned long long &seen, uint64_t epoch) {
+  constexpr unsigned long long kOne = 1ull << 48, kBias = 1ull << 33, kMark = 1ull << 56;
+  const int lane = threadIdx.x & 31;
+  const int n = gridDim.x;
+  if (lane < kDigits) {
+    uint64_t a = f.m < 0 ? -f.m : f.m;
+    int s = f.e - lo;  // place of a's lowest bit in the window
+    unsigned long long add = kOne + kBias;
+    if (f.m != 0 || f.e >= kFixBad) {
+      if (s > 32 * kDigits - 68) {  // 58 bits and 8 of 152 addends
+        add += kMark;
+      } else {
+        if (s < 0) {
+          a >>= min(-s, 63);
+          s = 0;
+        }
+        const int off = 32 * lane - s;
+        const uint64_t d = (off >= 64 || off <= -32 ? 0 : off >= 0 ? a >> off : a << -off) & 0xffffffffull;
+        add += f.m < 0 ? -d : d;
+      }
+    }
+    red_add(words->digit + lane, add);
+  }
+  unsigned long long w = 0;
+  bool ok = true;
+  if (lane < kDigits) {
+    Bound bound;
+    for (;;) {
+      w = load_relaxed(words->digit + lane);
+      if (((w - seen) >> 48 & 0xff) == (unsigned)n) break;
+      if (bound.over()) {
+        ok = false;
+        break;
+      }
+    }
+  }
+  if (!__all_sync(0xffffffffu, ok)) return false;
+  const unsigned long long diff = w - seen;
+  seen = w;
+  if (__any_sync(0xffffffffu, diff >> 56 != 0)) return slot_sum(gs->slot, f, epoch);
+  int64_t d = (int64_t)(diff & (kOne - 1)) - (int64_t)n * (int64_t)kBias;
+  if (lane >= kDigits) d = 0;
+  // carry upwards: digits of 32 bits, the top one signed
+  int64_t c[kDigits];
+#pragma unroll
+  for (int k = 0; k < kDigits; k++) c[k] = __shfl_sync(0xffffffffu, d, k);
+#pragma unroll
+  for (int k = 1; k < kDigits; k++) c[k] += c[k - 1] >> 32;
+  const bool neg = c[kDigits - 1] < 0;
+  uint32_t u[kDigits];
+  uint32_t carry = neg ? 1 : 0;  // |total|: two's complement
+#pragma unroll
+  for (int k = 0; k < kDigits; k++) {
+    const uint32_t x = neg ? ~(uint32_t)c[k] : (uint32_t)c[k];
+    u[k] = x + carry;
+    carry = carry && u[k] == 0;
+  }
+  // the 64 highest bits from the top digit that is not zero
+  uint64_t hi = 0;
+  int at = 0;
+#pragma unroll
+  for (int k = kDigits - 1; k >= 0; k--)
+    if (hi == 0 && u[k]) {
+      const uint32_t below = k > 0 ? u[k - 1] : 0, below2 = k > 1 ? u[k - 2] : 0;
+      const int z = __clz(u[k]);
+      hi = ((uint64_t)u[k] << 32 | below) << z | (z ? below2 >> (32 - z) : 0);
+      at = 32 * (k - 1) - z;
+    }
+  f.m = (int64_t)(hi >> 6);  // 58 bits
+  if (neg) f.m = -f.m;
+  f.e = hi ? lo + at + 6 : -4096;
+  return true;
+}
+
+template <int T>
+struct Scratch {
+  FixSum part[T / 32];
+  double value;
+  int32_t ok;
+};
+
+// The sum of v over the whole grid near |ref|: `then(total)` runs in lane 0 of
+// warp 0 and its result is returned in every thread (FP64 arithmetic on the
+// total costs the pipe once instead of once per warp); `meanwhile()` runs in
+// the other warps while warp 0 waits: work that does not need the total.  T:
+// threads of the block (a multiple of 32, at most 1024).  False in every
+// thread when a wait ran out (the caller returns).
+template <int T, class V, class F, class H>
+__device__ __forceinline__ bool sum(V v, GridSync *gs, int which, double ref,
+                                    unsigned long long &seen, uint64_t epoch, Scratch<T> &sh,
+                                    double &value, F then, H meanwhile) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const FixSum s = warp_sum(fix_of(v));
+  if (lane == 0) sh.part[w] = s;
+  __syncthreads();
+  if (w == 0) {
+    FixSum t;
+    t.m = 0;
+    t.e = -4096;
+    if (lane < T / 32) t = sh.part[lane];
+    t = warp_sum(t);
+    const bool ok = digit_sum(gs, &gs->sum[which], t, window_of(ref), seen, epoch);
+    if (lane == 0) {
+      sh.value = then(fix_value(t));
+      sh.ok = ok;
+    }
+  } else {
+    meanwhile();
+  }
+  __syncthreads();
+  value = sh.value;
+  return sh.ok != 0;
+}
+
+// Makes the blocks' global stores visible to one another.  The fences on both
+// sides order the data (and drop stale L1 lines).  `count`: barriers passed
+// in this launch, this one included.
+template <int T>
+__device__ __forceinline__ bool barrier(GridSync *gs, uint32_t count, Scratch<T> &sh) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    fence();
+    unsigned long long *p = gs->arrive.digit;
+    red_add(p, 1);
+    const unsigned long long want = (unsigned long long)count * gridDim.x;
+    bool ok = true;
+    Bound bound;
+    while (ok && load_relaxed(p) < want) ok = !bound.over();
+    fence();
+    sh.ok = ok;
+  }
+  __syncthreads();
+  return sh.ok != 0;
+}
+
+}  // namespace grid
+}  // namespace elx

@@ -1,0 +1,89 @@
+"""The FP64 PCG in one cooperative launch (persist.cu) where it can go wrong:
+one slice of block rows, a last slice that is not full, as many slices as
+blocks and one more, several launches per solve, loads at the ends of the
+exponent range (the digit window of the grid sums follows the residual), a
+matrix and a load whose norms differ by many orders, and a load with a NaN.
+
+Bars: the solver tests' (displacements within 1e-10 of the oracle, iterations
+within 2); a load scaled by a power of two gives the same iterates scaled
+exactly."""
+import numpy as np
+import pytest
+
+import elastic_gb300 as E
+import oracle as O
+from elastic_gb300 import meshgen as M
+from helpers import rel_inf
+
+pytestmark = pytest.mark.gpu
+
+# block rows: 24 (one slice), 32 = one full slice, 33, 152 * 32 and 153 * 32 of QUAD4
+CASES = {
+    "hexa8 one slice": lambda: M.box_hexa8(2, 3, 2),
+    "quad4 full slice": lambda: M.box2d(4, 7, etype=M.QUAD4_STRESS),
+    "quad4 two slices": lambda: M.box2d(3, 10, etype=M.QUAD4_STRAIN),
+    "quad4 152 slices": lambda: M.box2d(64, 75, etype=M.QUAD4_STRESS),
+    "tria3 153 slices": lambda: M.box2d(72, 67, etype=M.TRIA3_STRAIN),
+    "tetra4": lambda: M.box_tetra4(9, 8, 7, jitter=0.2, lognormal_E=True, nu_range=(0.25, 0.45)),
+}
+
+
+def _system(ctx, mesh, seed=3):
+    mesh.f = np.random.default_rng(seed).standard_normal(mesh.f.shape) * (mesh.id == 0)
+    ctx.set_mesh(mesh)
+    ctx.build_structure(True)
+    s = O.structure(mesh, True)
+    b0, u0 = O.loads(mesh, s)
+    ad, al, b = O.assemble(mesh, s, u0, b0)
+    ctx.assemble(u0, b0)
+    return s, ad, al, b
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_matches_oracle(gpu_ctx, name):
+    s, ad, al, b = _system(gpu_ctx, CASES[name]())
+    x_o, i_o = O.pcg(s, ad, al, b, tol=1e-12, maxit=20000)
+    x, i = gpu_ctx.solve(b, tol=1e-12, maxit=20000)
+    assert rel_inf(x_o, x) <= 1e-10
+    assert abs(i["iters"] - i_o["iters"]) <= 2
+    x2, i2 = gpu_ctx.solve(b, tol=1e-12, maxit=20000)
+    assert np.array_equal(x, x2) and i["iters"] == i2["iters"]
+
+
+@pytest.mark.parametrize("e", [-400, -60, 60, 400])
+def test_scaled_load_scales_exactly(gpu_ctx, e):
+    _, _, _, b = _system(gpu_ctx, M.box2d(40, 21, etype=M.QUAD4_STRAIN))
+    x, i = gpu_ctx.solve(b, tol=1e-11)
+    xs, js = gpu_ctx.solve(np.ldexp(b, e), tol=1e-11)
+    assert i["iters"] == js["iters"]
+    assert np.array_equal(np.ldexp(x, e), xs)
+
+
+def test_several_launches_and_maxit(gpu_ctx):
+    s, ad, al, b = _system(gpu_ctx, M.box2d(120, 60, etype=M.TRIA3_STRESS))
+    x, i = gpu_ctx.solve(b, tol=1e-11, maxit=20000)
+    assert i["iters"] > 1024  # more than two launches of 512 iterations
+    x_o, i_o = O.pcg(s, ad, al, b, tol=1e-11, maxit=20000)
+    assert rel_inf(x_o, x) <= 1e-10 and abs(i["iters"] - i_o["iters"]) <= 2
+    for maxit in (1, 511, 512, 513, 1024):
+        _, i = gpu_ctx.solve(b, tol=1e-11, maxit=maxit, raise_on_error=False)
+        assert i["status"] == E.ERR_NO_CONVERGENCE and i["iters"] == maxit
+
+
+def test_residual_far_from_the_matrix_scale(gpu_ctx):
+    m = M.box_hexa8(5, 4, 4, E=1e-90)
+    s, ad, al, b = _system(gpu_ctx, m)
+    x_o, i_o = O.pcg(s, ad, al, b, tol=1e-11, maxit=5000)
+    x, i = gpu_ctx.solve(b, tol=1e-11, maxit=5000)
+    assert rel_inf(x_o, x) <= 1e-10 and abs(i["iters"] - i_o["iters"]) <= 2
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_load_that_is_not_finite_does_not_converge(gpu_ctx, bad):
+    _, _, _, b = _system(gpu_ctx, M.box2d(30, 20, etype=M.QUAD4_STRESS))
+    c = b.copy()
+    c[17] = bad
+    _, i = gpu_ctx.solve(c, tol=1e-10, maxit=200, raise_on_error=False)
+    assert i["status"] == E.ERR_NO_CONVERGENCE
+    x, i = gpu_ctx.solve(b, tol=1e-10)
+    assert i["status"] == 0 and np.isfinite(x).all()

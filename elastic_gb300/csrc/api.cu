@@ -106,6 +106,9 @@ void upload_structure(elx_ctx *c, bool prederived) {
   if (const char *env = getenv("ELX_BLOCKS")) want_blocks = want_blocks && atoi(env) != 0;
   if (want_blocks && !prederived) elx::build_blocks(s, m.ndf);
   c->use_blocks = want_blocks && s.blocked;
+  c->want_blocks = want_blocks;
+  s.padded = false;
+  if (want_blocks && !s.blocked) elx::build_padded(s, m.ndf);
   for (DBuf *v : {&c->iat, &c->jat, &c->pt, &c->ja16, &c->jat16, &c->tile_tgt, &c->tile_out,
                   &c->tgt_col, &c->tgt_start, &c->tpos, &c->halo_ptr, &c->halo_slot,
                   &c->tile_desc, &c->part, &c->alt, &c->ja, &c->bia, &c->bt, &c->sell_ptr,
@@ -165,7 +168,6 @@ void upload_structure(elx_ctx *c, bool prederived) {
       for (size_t i = 0; i < ja0.size(); i++) ja0[i] = s.ja[i] - 1;
       c->upload(c->ja, ja0.data(), ja0.size());
     }
-    choose_tiles(s);
     elx::build_transpose(s);
     c->upload(c->iat, s.iat.data(), s.iat.size());
     c->upload(c->jat, s.jat.data(), s.jat.size());
@@ -174,16 +176,22 @@ void upload_structure(elx_ctx *c, bool prederived) {
       c->upload(c->ja16, s.ja16.data(), s.ja16.size());
       c->upload(c->jat16, s.jat16.data(), s.jat16.size());
     }
-    c->upload(c->tile_tgt, s.tile_tgt.data(), s.tile_tgt.size());
-    c->upload(c->tile_out, s.tile_out.data(), s.tile_out.size());
-    c->upload(c->tgt_col, s.tgt_col.data(), s.tgt_col.size());
-    c->upload(c->tgt_start, s.tgt_start.data(), s.tgt_start.size());
-    c->upload(c->tpos, s.tpos.data(), s.tpos.size());
-    c->upload(c->halo_ptr, s.halo_ptr.data(), s.halo_ptr.size());
-    c->upload(c->halo_slot, s.halo_slot.data(), s.halo_slot.size());
-    c->upload(c->tile_desc, s.tile_desc.data(), s.tile_desc.size());
-    c->alloc(c->part, (size_t)s.tile_out[s.ntiles] * 8);
-    elx::prepare_tile_kernels(c->tile_dev());
+    if (c->spmv_kind == elx::kSpmvTiled) {
+      choose_tiles(s);
+      c->upload(c->tile_tgt, s.tile_tgt.data(), s.tile_tgt.size());
+      c->upload(c->tile_out, s.tile_out.data(), s.tile_out.size());
+      c->upload(c->tgt_col, s.tgt_col.data(), s.tgt_col.size());
+      c->upload(c->tgt_start, s.tgt_start.data(), s.tgt_start.size());
+      c->upload(c->tpos, s.tpos.data(), s.tpos.size());
+      c->upload(c->halo_ptr, s.halo_ptr.data(), s.halo_ptr.size());
+      c->upload(c->halo_slot, s.halo_slot.data(), s.halo_slot.size());
+      c->upload(c->tile_desc, s.tile_desc.data(), s.tile_desc.size());
+      c->alloc(c->part, (size_t)s.tile_out[s.ntiles] * 8);
+      elx::prepare_tile_kernels(c->tile_dev());
+    } else {
+      s.tile_rows = s.ntiles = 0;
+      c->alloc(c->part, 16);
+    }
     c->alloc(c->alt, (size_t)s.nad * 8 + 64);
   }
   const size_t n = (size_t)s.neq, nad = (size_t)s.nad;
@@ -197,12 +205,13 @@ void upload_structure(elx_ctx *c, bool prederived) {
   for (auto &row : c->tuned_unroll)
     for (int &u : row) u = 0;
   for (DBuf *v : {&c->node_count, &c->tstress, &c->tx0buf, &c->fbuf, &c->ld_node, &c->ld_ptr,
-                  &c->ld_ent, &c->ld_vec, &c->vtkbuf, &c->persist_cta, &c->persist_sync})
+                  &c->ld_ent, &c->ld_vec, &c->vtkbuf, &c->persist_cta, &c->persist_sync, &c->persist_vec, &c->p_ptr,
+                  &c->p_col, &c->p_off, &c->p_eq, &c->p_val})
     c->release(*v);
   c->persist_grid = 0;
   c->have_stress = false;
   release_partitions(c);
-  c->have_fp32 = false;
+  c->have_fp32 = c->have_padded = false;
   c->alloc(c->u, (size_t)m.ndf * m.nnode * 8);
   ELX_CUDA(cudaMemsetAsync(c->u.p, 0, c->u.bytes, c->stream));
   c->alloc(c->b0, n * 8);
@@ -285,7 +294,7 @@ void assemble_resident(elx_ctx *c) {
   c->launches += (int64_t)s.segments.size();
   ELX_CUDA(cudaMemcpyAsync(c->h_flags, bad, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
   c->sync();
-  c->have_fp32 = false;
+  c->have_fp32 = c->have_padded = false;
   if (c->h_flags[0] != INT_MAX) {
     c->have_matrix = false;
     throw Error{ELX_ERR_BAD_DET, "non-positive Jacobian determinant in element " +
@@ -453,46 +462,35 @@ void set_scalars(elx_ctx *c, double tol, int maxit) {
                            c->stream));
 }
 
-// The cooperative PCG, kPersistSteps iterations a launch, until it has stopped
-// (two launches in flight: the second returns at once when the first stopped).
-constexpr int kPersistSteps = 512;
-elx::PcgScalars run_persist(elx_ctx *c, int maxit) {
-  const int max_launches = maxit / kPersistSteps + 2;
-  int launched = 0, checked = 0;
-  auto launch = [&](int slot) {
-    persist_steps(c, kPersistSteps);
-    ELX_CUDA(cudaMemcpyAsync(&c->h_scal[slot], c->scal.p, sizeof(elx::PcgScalars),
-                             cudaMemcpyDeviceToHost, c->stream));
-    ELX_CUDA(cudaEventRecord(c->ev[slot], c->stream));
-    launched++;
-  };
-  launch(0);
-  for (;;) {
-    if (launched < max_launches) launch(launched & 1);
-    const int slot = checked & 1;
-    ELX_CUDA(cudaEventSynchronize(c->ev[slot]));
-    checked++;
-    if (c->h_scal[slot].done || checked == launched) {
-      const elx::PcgScalars last = c->h_scal[slot];
-      c->sync();
-      return last;
-    }
-  }
-}
+// Iterations of a launch of the cooperative PCG: long solves stay in launches
+// of some ms, and the state's round trip between two is under 1 % of them.  A
+// server's block solve, whose batches are held back for small requests, takes
+// shorter ones.
+constexpr int kPersistSteps = 512, kPersistGatedSteps = 32;
 
 void pcg64(elx_ctx *c, double tol, int maxit, elx_info *info) {
   auto t0 = std::chrono::steady_clock::now();
   build_preconditioner(c);
-  set_scalars(c, tol, maxit);
-  elx::launch_pcg_start<double>(c->s.neq, c->b.as<double>(), c->m.as<double>(),
-                                c->xs.as<double>(), c->r.as<double>(), c->p.as<double>(),
-                                c->scal.as<elx::PcgScalars>(), c->partials.as<double>(),
-                                c->counters.as<unsigned int>() + 2, c->stream);
-  c->launches += 1;
-  elx::PcgScalars last;
+  elx::PcgScalars last{};
   if (ensure_persist(c)) {
-    last = run_persist(c, maxit);
+    // x's place holds x between launches too; r and p are the context's
+    elx::PersistCol col;
+    const size_t n = (size_t)persist_rows(c);
+    if (c->persist_vec.bytes < 3 * n * 8) c->alloc(c->persist_vec, 3 * n * 8);
+    persist_solve(c, 1, tol, maxit, c->b.as<double>(), c->xs.as<double>(),
+                  c->persist_vec.as<double>(), c->batch_gate ? kPersistGatedSteps : kPersistSteps,
+                  &col);
+    last.iters = col.iters;
+    last.status = col.status;
+    last.done = col.done;
+    last.conv = col.conv;
   } else {
+    set_scalars(c, tol, maxit);
+    elx::launch_pcg_start<double>(c->s.neq, c->b.as<double>(), c->m.as<double>(),
+                                  c->xs.as<double>(), c->r.as<double>(), c->p.as<double>(),
+                                  c->scal.as<elx::PcgScalars>(), c->partials.as<double>(),
+                                  c->counters.as<unsigned int>() + 2, c->stream);
+    c->launches += 1;
     capture_pcg_graph(c);
     last = run_batches(c, c->pcg_graph, c->spmv_kind == elx::kSpmvTiled ? 4 : 3, maxit);
   }
@@ -817,6 +815,73 @@ int autotune_block_width(elx_ctx *c, bool mixed, double *times_us = nullptr) {
   return best;
 }
 
+// FP64 load cases by the cooperative PCG, up to nc columns a launch (persist.cu):
+// the columns share the matrix reads and the waits, and none pads a block to a
+// width.  False: the matrix is too large for it.
+bool solve_block_persist(elx_ctx *c, int nrhs, double tol, int maxit, int width, const double *b,
+                         double *x, elx_info *infos, bool device_ptrs) {
+  // 3x3 blocks are FP64-bound either way: krylov's product over 8 or 16 columns
+  // is 5 % faster per column when none of its columns is padding (205,320
+  // equations, 16 columns: 388 against 405 ms; 6 columns: 206 against 152)
+  int w = 1;
+  while (w < 16 && w < nrhs && (width == 0 || w < width)) w *= 2;
+  if (c->s.bsize == 3 && nrhs > elx::kGridCols && 21 * nrhs > 20 * ((nrhs + w - 1) / w * w))
+    return false;
+  const int want = std::min(nrhs, width > 0 ? width : elx::kGridCols);
+  const int nc = persist_columns(c, want);
+  if (nc < std::min(want, 4)) return false;
+  auto t0 = std::chrono::steady_clock::now();
+  build_preconditioner(c);
+  const size_t n = (size_t)c->s.neq;
+  // per column: three work vectors, b and x
+  if (c->persist_vec.bytes < 5 * n * nc * 8) c->alloc(c->persist_vec, 5 * n * nc * 8);
+  double *work = c->persist_vec.as<double>(), *bs = work + 3 * n * nc, *xs = bs + n * nc;
+  const int chunks = (nrhs + nc - 1) / nc;
+  int status = ELX_OK;
+  for (int k = 0; k < chunks; k++) {
+    const int c0 = (int)((int64_t)nrhs * k / chunks), m = (int)((int64_t)nrhs * (k + 1) / chunks) - c0;
+    const double *bd = device_ptrs ? b + (size_t)c0 * n : bs;
+    double *xd = device_ptrs ? x + (size_t)c0 * n : xs;
+    if (!device_ptrs)
+      ELX_CUDA(cudaMemcpyAsync(bs, b + (size_t)c0 * n, n * m * 8, cudaMemcpyHostToDevice,
+                               c->stream));
+    elx::PersistCol cols[elx::kGridCols];
+    persist_solve(c, m, tol, maxit, bd, xd, work,
+                  c->batch_gate ? kPersistGatedSteps : kPersistSteps, cols);
+    if (!device_ptrs)
+      ELX_CUDA(cudaMemcpyAsync(x + (size_t)c0 * n, xs, n * m * 8, cudaMemcpyDeviceToHost,
+                               c->stream));
+    for (int j = 0; j < m; j++) {
+      spmv64(c, xd + (size_t)j * n, c->z.as<double>());
+      elx::launch_diagnostics(c->s.neq, xd + (size_t)j * n, c->z.as<double>(),
+                              bd + (size_t)j * n, c->m.as<double>(), c->diag.as<double>(),
+                              c->partials.as<double>(), c->counters.as<unsigned int>() + 3,
+                              c->stream);
+      c->launches += 1;
+      ELX_CUDA(cudaMemcpyAsync(c->h_diag, c->diag.p, 4 * sizeof(double), cudaMemcpyDeviceToHost,
+                               c->stream));
+      check_pipe_waits(c);
+      const int st = cols[j].done ? cols[j].status : ELX_ERR_NO_CONVERGENCE;
+      if (st != ELX_OK && status == ELX_OK) status = st;
+      if (!infos) continue;
+      elx_info &in = infos[c0 + j];
+      std::memset(&in, 0, sizeof(in));
+      in.iters = cols[j].iters;
+      in.status = st;
+      in.xkx = c->h_diag[0];
+      in.norm_x = std::sqrt(c->h_diag[1]);
+      in.norm_m_r = std::sqrt(std::fabs(c->h_diag[2]));
+      in.norm_r = std::sqrt(c->h_diag[3]);
+      in.conv = cols[j].conv;
+    }
+    const double secs =
+        std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    for (int j = 0; j < m && infos; j++) infos[c0 + j].seconds = secs;
+  }
+  if (status != ELX_OK) throw Error{status, "block PCG: a load case did not converge"};
+  return true;
+}
+
 // Solves nrhs load cases (b column-major, neq x nrhs, on the host or the
 // device) in blocks of `width` columns; x likewise; one elx_info per column.
 void solve_block(elx_ctx *c, int nrhs, int precision, double tol, int maxit, int width,
@@ -830,6 +895,7 @@ void solve_block(elx_ctx *c, int nrhs, int precision, double tol, int maxit, int
   require(c->use_blocks, ELX_ERR_ARG,
           "block solves need node blocks (every node all free or all fixed)");
   const bool mixed = precision == ELX_PREC_MIXED;
+  if (!mixed && solve_block_persist(c, nrhs, tol, maxit, width, b, x, infos, device_ptrs)) return;
   auto t0 = std::chrono::steady_clock::now();
   if (mixed) ensure_fp32(c);
   build_preconditioner(c);
@@ -1173,7 +1239,8 @@ int elx_create(elx_ctx **out, const elx_opts *opts) {
     c->pool_user = true;
     // h_scal (2 PcgScalars), h_diag (8 doubles), h_flags (4 ints) in one
     // recycled pinned block
-    static_assert(2 * sizeof(elx::PcgScalars) + 8 * sizeof(double) + 4 * sizeof(int32_t) <=
+    static_assert(2 * sizeof(elx::PcgScalars) + 8 * sizeof(double) + 4 * sizeof(int32_t) +
+                          12 * sizeof(elx::PersistCol) <=
                       elx::kPinnedBlock,
                   "pinned block too small");
     c->pinned = elx::pinned_block_get();
@@ -1181,6 +1248,8 @@ int elx_create(elx_ctx **out, const elx_opts *opts) {
     c->h_scal = reinterpret_cast<elx::PcgScalars *>(pb);
     c->h_diag = reinterpret_cast<double *>(pb + 2 * sizeof(elx::PcgScalars));
     c->h_flags = reinterpret_cast<int32_t *>(pb + 2 * sizeof(elx::PcgScalars) + 8 * sizeof(double));
+    c->h_cols = reinterpret_cast<elx::PersistCol *>(pb + 2 * sizeof(elx::PcgScalars) +
+                                                    8 * sizeof(double) + 4 * sizeof(int32_t));
     for (auto &e : c->ev) ELX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     for (auto &e : c->ev_t) ELX_CUDA(cudaEventCreate(&e));
   });
@@ -1209,7 +1278,8 @@ void elx_destroy(elx_ctx *c) {
                   &c->sell_val, &c->sell_val64, &c->sell_d16,
                   &c->node_count, &c->tstress, &c->tx0buf, &c->fbuf, &c->ld_node, &c->ld_ptr,
                   &c->ld_ent, &c->ld_vec, &c->vtkbuf,
-                  &c->persist_cta, &c->persist_sync,
+                  &c->persist_cta, &c->persist_sync, &c->persist_vec, &c->p_ptr,
+                  &c->p_col, &c->p_off, &c->p_eq, &c->p_val,
                   &c->u, &c->b0, &c->b, &c->xs, &c->r, &c->p, &c->q, &c->m, &c->z,
                   &c->scal, &c->partials, &c->counters, &c->flags, &c->diag})
     c->release(*d);
@@ -1530,7 +1600,7 @@ int elx_set_matrix(elx_ctx *c, const double *ad, const double *al) {
     refresh_derived_values(c);
     c->sync();
     c->have_matrix = true;
-    c->have_fp32 = false;
+    c->have_fp32 = c->have_padded = false;
   });
 }
 

@@ -97,6 +97,50 @@ __global__ void fill_sell_kernel(int nb, int nslices, const int32_t *__restrict_
   }
 }
 
+// The same for block rows with fixed dofs (build_padded): entry (a, b) of slot
+// (I, J) from the CSRC arrays, zero where row a or column b is fixed (eq -1).
+template <int B>
+__global__ void fill_padded_kernel(int nb, int nslices, const int32_t *__restrict__ ptr,
+                                   const int32_t *__restrict__ col,
+                                   const int32_t *__restrict__ off,
+                                   const int32_t *__restrict__ eq,
+                                   const int32_t *__restrict__ ia, const double *__restrict__ ad,
+                                   const double *__restrict__ al, double *__restrict__ val) {
+  constexpr int BB = B * B, R = kSliceRows;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nslices * R;
+       i += gridDim.x * blockDim.x) {
+    const int sl = i / R, t = i % R, I = i;
+    int ei[B];
+#pragma unroll
+    for (int a = 0; a < B; a++) ei[a] = I < nb ? eq[I * B + a] : -1;
+    for (int g = ptr[sl]; g < ptr[sl + 1]; g++) {
+      const size_t q = (size_t)g * R + t;
+      const int J = col[q], o = off[q];
+      double *grp = val + (size_t)g * BB * R;
+      int ej[B], first = -1;  // the lower node's first equation
+#pragma unroll
+      for (int b = 0; b < B; b++) ej[b] = eq[J * B + b];
+#pragma unroll
+      for (int b = B - 1; b >= 0; b--) {
+        const int e = J < I ? ej[b] : ei[b];
+        if (e >= 0) first = e;
+      }
+#pragma unroll
+      for (int a = 0; a < B; a++)
+#pragma unroll
+        for (int b = 0; b < B; b++) {
+          double v = 0.0;
+          if (o >= 0 && ei[a] >= 0 && ej[b] >= 0) {
+            const int hi = max(ei[a], ej[b]), lo = min(ei[a], ej[b]);
+            v = hi == lo ? ad[hi] : I == J ? al[ia[hi + 1] - (hi - lo)]
+                                           : al[ia[hi] + o + (lo - first)];
+          }
+          grp[sell_pos<double, B>(a * B + b, t)] = v;
+        }
+    }
+  }
+}
+
 // y = K x on a sliced copy: one warp per slice, one thread per block row.
 // Slot group g of a slice is one 128-byte line of column indices and B^2 / V
 // 512-byte runs (plus B^2 mod V lines) of values, so every load of the
@@ -263,6 +307,17 @@ double measure_fp64_fma_rate(int device, double *per_clock_per_sm) {
 
 void launch_fill_sell64(const CsrcDev &k, cudaStream_t st) { fill_sell<double>(k, k.sell_val64, st); }
 void launch_fill_sell32(const CsrcDev &k, cudaStream_t st) { fill_sell<float>(k, k.sell_val, st); }
+
+void launch_fill_padded64(const CsrcDev &k, int bsize, int nb, int nslices, const int32_t *ptr,
+                          const int32_t *col, const int32_t *off, const int32_t *eq, double *val,
+                          cudaStream_t st) {
+  const int g = fill_grid((int64_t)nslices * kSliceRows);
+  if (bsize == 3)
+    fill_padded_kernel<3><<<g, 256, 0, st>>>(nb, nslices, ptr, col, off, eq, k.ia, k.ad, k.al, val);
+  else
+    fill_padded_kernel<2><<<g, 256, 0, st>>>(nb, nslices, ptr, col, off, eq, k.ia, k.ad, k.al, val);
+  ELX_CUDA(cudaGetLastError());
+}
 
 void launch_sell64_local(int nb, int nslices, int bsize, const int32_t *sell_ptr,
                          const int32_t *sell_col, const double *sval, const double *x,

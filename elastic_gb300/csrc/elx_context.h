@@ -96,10 +96,16 @@ struct elx_ctx {
   int32_t *h_flags = nullptr;         // pinned
 
   // cooperative PCG (persist.cu): blocks (0: not planned, -1: not used), their
-  // slices and the blocks' shared words
-  DBuf persist_cta, persist_sync;
+  // slices and shared words, the vectors between launches, and per number of
+  // columns where the vectors live (0: too many, 1: L2, 2: shared memory)
+  DBuf persist_cta, persist_sync, persist_vec;
+  // its matrix when some nodes are only partly fixed (Structure::p_*)
+  DBuf p_ptr, p_col, p_off, p_eq, p_val;
+  bool have_padded = false;  // p_val was filled since the last assembly
+  bool want_blocks = true;   // node blocks are not switched off
   int persist_grid = 0, persist_rows = 0, persist_slices = 0;
-  bool persist_smem = false;
+  int persist_mode[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  elx::PersistCol *h_cols = nullptr;  // pinned, 2 slots of 6
 
   int64_t launches = 0;  // kernels of this library launched by this context
 
@@ -232,7 +238,10 @@ void build_preconditioner(elx_ctx *c);
 void release_block(elx_ctx *c);
 // Cooperative PCG (persist.cu).
 bool ensure_persist(elx_ctx *c);
-void persist_steps(elx_ctx *c, int steps);
+int persist_columns(elx_ctx *c, int want);
+int persist_rows(const elx_ctx *c);
+void persist_solve(elx_ctx *c, int nc, double tol, int maxit, const double *b, double *x,
+                   double *work, int steps, elx::PersistCol *out);
 // Row-block partitions on one device (partition.cu).
 void ensure_partitions(elx_ctx *c, int nparts);
 void release_partitions(elx_ctx *c);

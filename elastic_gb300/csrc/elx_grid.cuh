@@ -17,6 +17,7 @@
 
 #include <cstdint>
 
+#include "elx_krylov.h"
 #include "elx_ptx.cuh"
 #include "elx_reduce.cuh"
 
@@ -26,9 +27,10 @@ constexpr int kGridMaxBlocks = 160;
 constexpr uint64_t kGridWaitNs = 2000000000ull;  // bound of every grid wait
 constexpr int kDigits = 5;
 
+
 // Shared by the blocks of a launch; zeroed before each launch.
 struct alignas(128) GridWords {
-  unsigned long long digit[16];  // kDigits used
+  unsigned long long digit[32];  // kDigits for each sum
 };
 struct alignas(16) GridSlot {
   int64_t m;
@@ -37,7 +39,7 @@ struct alignas(16) GridSlot {
 struct GridSync {
   GridWords sum[2];  // (p, q) and (r, z)
   GridWords arrive;  // digit[0]: arrivals at the barrier
-  GridSlot slot[kGridMaxBlocks];
+  GridSlot slot[kGridCols][kGridMaxBlocks];
 };
 
 namespace grid {
@@ -73,6 +75,13 @@ __device__ __forceinline__ GridSlot load_slot(const GridSlot *s) {
 
 __device__ __forceinline__ void fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
+__device__ __forceinline__ FixSum fix_shfl(FixSum f, int lane) {
+  FixSum r;
+  r.m = __shfl_sync(0xffffffffu, f.m, lane);
+  r.e = __shfl_sync(0xffffffffu, f.e, lane);
+  return r;
+}
+
 // Counts polls and bounds them by the GPU's clock.
 struct Bound {
   uint64_t t0 = 0;
@@ -85,42 +94,46 @@ struct Bound {
   }
 };
 
-// Every block's f through its slot (value, exponent and epoch in one 16-byte
-// store); warp 0.
-__device__ __forceinline__ bool slot_sum(GridSlot *slots, FixSum &f, uint64_t epoch) {
+// The blocks' sums through a slot of each block (value, exponent and epoch in
+// one 16-byte store); warp 0, lane c holds sum c.
+template <int NC>
+__device__ __forceinline__ bool slot_sum(GridSync *gs, FixSum &f, uint64_t epoch) {
   constexpr int K = kGridMaxBlocks / 32;
   const int lane = threadIdx.x & 31;
-  if (lane == 0)
-    store_slot(slots + blockIdx.x, f.m, epoch << 24 | (uint64_t)(uint32_t)(f.e + 4096));
-  FixSum v[K];
+  if (lane < NC)
+    store_slot(gs->slot[lane] + blockIdx.x, f.m,
+               epoch << 24 | (uint64_t)(uint32_t)(f.e + 4096));
   bool ok = true;
   Bound bound;
+  for (int c = 0; c < NC; c++) {
+    FixSum v[K];
 #pragma unroll
-  for (int k = 0; k < K; k++) {
-    v[k].m = 0;
-    v[k].e = -4096;
-    const int b = lane + 32 * k;
-    while (b < (int)gridDim.x && ok) {
-      const GridSlot g = load_slot(slots + b);
-      if (g.tag >> 24 == epoch) {
-        v[k].m = g.m;
-        v[k].e = (int32_t)(g.tag & 0xffffffu) - 4096;
-        break;
+    for (int k = 0; k < K; k++) {
+      v[k].m = 0;
+      v[k].e = -4096;
+      const int b = lane + 32 * k;
+      while (b < (int)gridDim.x && ok) {
+        const GridSlot g = load_slot(gs->slot[c] + b);
+        if (g.tag >> 24 == epoch) {
+          v[k].m = g.m;
+          v[k].e = (int32_t)(g.tag & 0xffffffu) - 4096;
+          break;
+        }
+        ok = !bound.over();
       }
-      ok = !bound.over();
     }
+    int e = v[0].e;
+#pragma unroll
+    for (int k = 1; k < K; k++) e = max(e, v[k].e);
+    FixSum t;
+    t.m = 0;
+#pragma unroll
+    for (int k = 0; k < K; k++) t.m += v[k].m >> min(e - v[k].e + 3, 63);
+    t.e = e + 3;
+    t = warp_sum(t);
+    if (lane == c) f = t;
   }
-  ok = __all_sync(0xffffffffu, ok);
-  int e = v[0].e;
-#pragma unroll
-  for (int k = 1; k < K; k++) e = max(e, v[k].e);
-  FixSum t;
-  t.m = 0;
-#pragma unroll
-  for (int k = 0; k < K; k++) t.m += v[k].m >> min(e - v[k].e + 3, 63);
-  t.e = e + 3;
-  f = warp_sum(t);
-  return ok;
+  return __all_sync(0xffffffffu, ok);
 }
 
 // Exponent of a window's lowest bit for sums near |ref|.
@@ -129,19 +142,24 @@ __device__ __forceinline__ int window_of(double ref) {
   return ex - 1023 - 120;
 }
 
-// The blocks' sum of f (warp 0, every lane the same f): digits of 2^lo.
-// `seen` holds this lane's word after the last sum.  False in every lane when
-// the bound ran out.
+// The blocks' sums of f (warp 0, lane c holds sum c and `lo`, the exponent of
+// its lowest digit).  `seen`: this lane's word after the last sum.  False in
+// every lane when the bound ran out.
+template <int NC>
 __device__ __forceinline__ bool digit_sum(GridSync *gs, GridWords *words, FixSum &f, int lo,
                                           unsigned long long &seen, uint64_t epoch) {
+  static_assert(NC * kDigits <= 32, "one lane per digit");
   constexpr unsigned long long kOne = 1ull << 48, kBias = 1ull << 33, kMark = 1ull << 56;
-  const int lane = threadIdx.x & 31;
-  const int n = gridDim.x;
-  if (lane < kDigits) {
-    uint64_t a = f.m < 0 ? -f.m : f.m;
-    int s = f.e - lo;  // place of a's lowest bit in the window
+  const int lane = threadIdx.x & 31, n = gridDim.x;
+  const int col = min(lane / kDigits, NC - 1), k0 = lane - col * kDigits;
+  const FixSum g = fix_shfl(f, col);
+  const int glo = __shfl_sync(0xffffffffu, lo, col);
+  const bool on = lane < NC * kDigits;
+  if (on) {
+    uint64_t a = g.m < 0 ? -g.m : g.m;
+    int s = g.e - glo;  // place of a's lowest bit in the window
     unsigned long long add = kOne + kBias;
-    if (f.m != 0 || f.e >= kFixBad) {
+    if (g.m != 0 || g.e >= kFixBad) {
       if (s > 32 * kDigits - 68) {  // 58 bits and 8 of 152 addends
         add += kMark;
       } else {
@@ -149,16 +167,17 @@ __device__ __forceinline__ bool digit_sum(GridSync *gs, GridWords *words, FixSum
           a >>= min(-s, 63);
           s = 0;
         }
-        const int off = 32 * lane - s;
-        const uint64_t d = (off >= 64 || off <= -32 ? 0 : off >= 0 ? a >> off : a << -off) & 0xffffffffull;
-        add += f.m < 0 ? -d : d;
+        const int off = 32 * k0 - s;
+        const uint64_t d =
+            (off >= 64 || off <= -32 ? 0 : off >= 0 ? a >> off : a << -off) & 0xffffffffull;
+        add += g.m < 0 ? -d : d;
       }
     }
     red_add(words->digit + lane, add);
   }
   unsigned long long w = 0;
   bool ok = true;
-  if (lane < kDigits) {
+  if (on) {
     Bound bound;
     for (;;) {
       w = load_relaxed(words->digit + lane);
@@ -172,13 +191,13 @@ __device__ __forceinline__ bool digit_sum(GridSync *gs, GridWords *words, FixSum
   if (!__all_sync(0xffffffffu, ok)) return false;
   const unsigned long long diff = w - seen;
   seen = w;
-  if (__any_sync(0xffffffffu, diff >> 56 != 0)) return slot_sum(gs->slot, f, epoch);
-  int64_t d = (int64_t)(diff & (kOne - 1)) - (int64_t)n * (int64_t)kBias;
-  if (lane >= kDigits) d = 0;
-  // carry upwards: digits of 32 bits, the top one signed
+  if (__any_sync(0xffffffffu, diff >> 56 != 0)) return slot_sum<NC>(gs, f, epoch);
+  const int64_t d = (int64_t)(diff & (kOne - 1)) - (int64_t)n * (int64_t)kBias;
+  // lane c: its sum's digits, carried upwards (32 bits each, the top one signed)
   int64_t c[kDigits];
+  const int base = min(lane, NC - 1) * kDigits;
 #pragma unroll
-  for (int k = 0; k < kDigits; k++) c[k] = __shfl_sync(0xffffffffu, d, k);
+  for (int k = 0; k < kDigits; k++) c[k] = __shfl_sync(0xffffffffu, d, base + k);
 #pragma unroll
   for (int k = 1; k < kDigits; k++) c[k] += c[k - 1] >> 32;
   const bool neg = c[kDigits - 1] < 0;
@@ -207,51 +226,60 @@ __device__ __forceinline__ bool digit_sum(GridSync *gs, GridWords *words, FixSum
   return true;
 }
 
-template <int T>
+template <int T, int NC>
 struct Scratch {
-  FixSum part[T / 32];
-  double value;
+  FixSum part[NC][T / 32];
   int32_t ok;
 };
 
-// The sum of v over the whole grid near |ref|: `then(total)` runs in lane 0 of
-// warp 0 and its result is returned in every thread (FP64 arithmetic on the
-// total costs the pipe once instead of once per warp); `meanwhile()` runs in
-// the other warps while warp 0 waits: work that does not need the total.  T:
-// threads of the block (a multiple of 32, at most 1024).  False in every
+// The sums of v[c] over the whole grid, each near |ref[c]| (shared memory;
+// nullptr: of any size).  `then(total)` runs in lane c of warp 0 with sum c
+// (FP64 arithmetic on the totals costs the pipe once instead of once per
+// warp) and leaves what the block needs in shared memory; `meanwhile()` runs
+// in the other warps while warp 0 waits: work that does not need the totals.
+// T: threads of the block (a multiple of 32, at most 1024).  False in every
 // thread when a wait ran out (the caller returns).
-template <int T, class V, class F, class H>
-__device__ __forceinline__ bool sum(V v, GridSync *gs, int which, double ref,
-                                    unsigned long long &seen, uint64_t epoch, Scratch<T> &sh,
-                                    double &value, F then, H meanwhile) {
+template <int T, int NC, class V, class F, class H>
+__device__ __forceinline__ bool sum(const V (&v)[NC], GridSync *gs, int which, const double *ref,
+                                    unsigned long long &seen, uint64_t epoch, Scratch<T, NC> &sh,
+                                    F then, H meanwhile) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const FixSum s = warp_sum(fix_of(v));
-  if (lane == 0) sh.part[w] = s;
+#pragma unroll
+  for (int c = 0; c < NC; c++) {
+    const FixSum s = warp_sum(fix_of(v[c]));
+    if (lane == 0) sh.part[c][w] = s;
+  }
   __syncthreads();
   if (w == 0) {
-    FixSum t;
-    t.m = 0;
-    t.e = -4096;
-    if (lane < T / 32) t = sh.part[lane];
-    t = warp_sum(t);
-    const bool ok = digit_sum(gs, &gs->sum[which], t, window_of(ref), seen, epoch);
-    if (lane == 0) {
-      sh.value = then(fix_value(t));
-      sh.ok = ok;
+    FixSum mine;
+    mine.m = 0;
+    mine.e = -4096;
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+      FixSum t;
+      t.m = 0;
+      t.e = -4096;
+      if (lane < T / 32) t = sh.part[c][lane];
+      t = warp_sum(t);
+      if (lane == c) mine = t;
     }
+    const bool ok = ref ? digit_sum<NC>(gs, &gs->sum[which], mine,
+                                        window_of(ref[lane < NC ? lane : 0]), seen, epoch)
+                        : slot_sum<NC>(gs, mine, epoch);
+    if (lane < NC) then(fix_value(mine));
+    if (lane == 0) sh.ok = ok;
   } else {
     meanwhile();
   }
   __syncthreads();
-  value = sh.value;
   return sh.ok != 0;
 }
 
 // Makes the blocks' global stores visible to one another.  The fences on both
 // sides order the data (and drop stale L1 lines).  `count`: barriers passed
 // in this launch, this one included.
-template <int T>
-__device__ __forceinline__ bool barrier(GridSync *gs, uint32_t count, Scratch<T> &sh) {
+template <int T, int NC>
+__device__ __forceinline__ bool barrier(GridSync *gs, uint32_t count, Scratch<T, NC> &sh) {
   __syncthreads();
   if (threadIdx.x == 0) {
     fence();

@@ -120,6 +120,11 @@ struct Structure {
   // (padding slots: the row's own column, zero values).
   int32_t nslices = 0;
   std::vector<int32_t> sell_ptr, sell_col;
+  // The same with partly fixed nodes padded to whole blocks (build_padded):
+  // slices, columns, the slots' places in the CSRC arrays, rows' equations
+  bool padded = false;
+  int32_t p_nb = 0, p_bsize = 0;
+  std::vector<int32_t> p_ptr, p_col, p_off, p_eq;
 };
 
 constexpr int kSliceRows = 32;
@@ -175,6 +180,7 @@ void build_transpose(Structure &s);
 std::vector<int32_t> partition_bounds(const Structure &s, int ndf, int nparts);
 void build_partition(const Structure &s, int32_t eq0, int32_t eq1, Partition &p);
 void build_blocks(Structure &s, int bsize);
+void build_padded(Structure &s, int bsize);
 
 // ------------------------------------------------------------- kernels
 struct MeshDev {
@@ -295,6 +301,10 @@ void launch_transpose_values(const CsrcDev &k, cudaStream_t st);
 // FP32 (k.sell_val).
 void launch_fill_sell64(const CsrcDev &k, cudaStream_t st);
 void launch_fill_sell32(const CsrcDev &k, cudaStream_t st);
+// The sliced FP64 copy of a matrix with partly fixed nodes (build_padded).
+void launch_fill_padded64(const CsrcDev &k, int bsize, int nb, int nslices, const int32_t *ptr,
+                          const int32_t *col, const int32_t *off, const int32_t *eq, double *val,
+                          cudaStream_t st);
 // FP64 FMAs per second of the device (a register-only probe kernel, best of
 // five timed launches) and, optionally, per clock per SM at the device's
 // maximum SM clock.

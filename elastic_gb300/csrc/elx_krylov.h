@@ -30,6 +30,15 @@ struct PcgScalars {
   int32_t pad_;
 };
 
+// Columns that a cooperative PCG (persist.cu) takes together: five lanes of a
+// warp carry the digits of each one's sums.
+constexpr int kGridCols = 6;
+// One column of it, between and after launches.
+struct PersistCol {
+  double d, conv;
+  int32_t iters, done, status, pad;
+};
+
 // Progress watch of the mixed-precision solvers.  A matrix rounded to FP32
 // can lose definiteness when K is ill-conditioned (cond(K) near 1/eps32, as
 // in 2-D meshes of 10^6 dofs): the FP32 recurrence then stalls or diverges.

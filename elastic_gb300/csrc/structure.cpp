@@ -686,6 +686,120 @@ void build_blocks(Structure &s, int bsize) {
   });
 }
 
+// Node blocks with partly fixed nodes: every node that has an equation gets a
+// whole block row, a fixed dof a row and column of zeros in it (p_eq -1), so
+// that the sliced kernels run on meshes with symmetry planes and rollers too.
+// p_off locates a slot's entries in the CSRC arrays: the place of the lower
+// node's run inside the rows of the higher node (the same in each of its
+// rows), -1 in a padding slot.  Any other pattern leaves s.padded false.
+void build_padded(Structure &s, int bsize) {
+  s.padded = false;
+  const int B = bsize, R = kSliceRows;
+  const int nnode = (int)(s.id.size() / B);
+  if (B < 2 || B > 3 || s.neq < 1) return;
+  std::vector<int32_t> node_at(s.neq, -1);  // the node whose first equation it is
+  for (int no = 0; no < nnode; no++) {
+    int32_t first = 0, next = 0;
+    for (int d = 0; d < B; d++) {
+      const int32_t q = s.id[(size_t)no * B + d];
+      if (q <= 0) continue;
+      if (!first) first = next = q;
+      if (q != next++) return;
+    }
+    if (!first) continue;
+    if (node_at[first - 1] >= 0) return;
+    node_at[first - 1] = no;
+  }
+  std::vector<int32_t> first, count, blk(s.neq, -1);
+  s.p_eq.clear();
+  for (int32_t q = 0; q < s.neq;) {
+    const int no = node_at[q];
+    if (no < 0) return;
+    const int I = (int)first.size();
+    first.push_back(q);
+    int n = 0;
+    for (int d = 0; d < B; d++) {
+      const int32_t e = s.id[(size_t)no * B + d];
+      s.p_eq.push_back(e > 0 ? e - 1 : -1);
+      if (e <= 0) continue;
+      if (e - 1 >= s.neq || blk[e - 1] >= 0) return;
+      blk[e - 1] = I;
+      n++;
+    }
+    count.push_back(n);
+    q += n;
+  }
+  const int nb = (int)first.size();
+  struct Low { int32_t J, off; };
+  std::vector<std::vector<Low>> low(nb);
+  std::atomic<bool> bad{false};
+  parallel_chunks(nb, 4096, [&](int64_t I0, int64_t I1) {
+    for (int64_t I = I0; I < I1 && !bad.load(std::memory_order_relaxed); I++) {
+      const int32_t r0 = first[I], k0 = s.ia[r0] - 1, len0 = s.ia[r0 + 1] - s.ia[r0];
+      bool ok = true;
+      for (int32_t k = 0; ok && k < len0;) {
+        const int32_t c = s.ja[k0 + k] - 1;
+        const int32_t J = blk[c];
+        ok = J < I && first[J] == c && k + count[J] <= len0;
+        for (int b = 1; ok && b < count[J]; b++) ok = s.ja[k0 + k + b] - 1 == c + b;
+        if (!ok) break;
+        low[I].push_back({J, k});
+        k += count[J];
+      }
+      for (int a = 0; ok && a < count[I]; a++) {
+        const int32_t ka = s.ia[r0 + a] - 1;
+        ok = s.ia[r0 + a + 1] - s.ia[r0 + a] == len0 + a;
+        for (int32_t k = 0; ok && k < len0; k++) ok = s.ja[ka + k] == s.ja[k0 + k];
+        for (int t = 0; ok && t < a; t++) ok = s.ja[ka + len0 + t] - 1 == r0 + t;
+      }
+      if (!ok) bad = true;
+    }
+  });
+  if (bad) return;
+  std::vector<int32_t> bia(nb + 1, 0);
+  for (int I = 0; I < nb; I++) {
+    bia[I + 1] += (int32_t)low[I].size() + 1;
+    for (const Low &l : low[I]) bia[l.J + 1]++;
+  }
+  for (int I = 0; I < nb; I++) bia[I + 1] += bia[I];
+  std::vector<Low> row(bia[nb]);
+  std::vector<int32_t> up(nb);
+  for (int I = 0; I < nb; I++) up[I] = bia[I] + (int32_t)low[I].size() + 1;
+  for (int I = 0; I < nb; I++) {
+    int32_t k = bia[I];
+    for (const Low &l : low[I]) {
+      row[k++] = l;
+      row[up[l.J]++] = {I, l.off};
+    }
+    row[k] = {I, 0};
+  }
+  const int ns = (nb + R - 1) / R;
+  s.p_ptr.assign(ns + 1, 0);
+  for (int sl = 0; sl < ns; sl++) {
+    int w = 0;
+    for (int I = sl * R; I < std::min(nb, sl * R + R); I++) w = std::max(w, bia[I + 1] - bia[I]);
+    s.p_ptr[sl + 1] = s.p_ptr[sl] + w;
+  }
+  s.p_col.assign((size_t)s.p_ptr[ns] * R, 0);
+  s.p_off.assign((size_t)s.p_ptr[ns] * R, -1);
+  parallel_chunks(ns, 1024, [&](int64_t a, int64_t b) {
+    for (int64_t sl = a; sl < b; sl++)
+      for (int t = 0; t < R; t++) {
+        const int I = (int)sl * R + t;
+        const int n = I < nb ? bia[I + 1] - bia[I] : 0;
+        for (int g = s.p_ptr[sl]; g < s.p_ptr[sl + 1]; g++) {
+          const int k = g - s.p_ptr[sl];
+          const size_t q = (size_t)g * R + t;
+          s.p_col[q] = k < n ? row[bia[I] + k].J : (I < nb ? I : 0);
+          if (k < n) s.p_off[q] = row[bia[I] + k].off;
+        }
+      }
+  });
+  s.p_nb = nb;
+  s.p_bsize = B;
+  s.padded = true;
+}
+
 }  // namespace elx
 
 namespace elx {

@@ -1,6 +1,8 @@
 """The FP64 PCG in one cooperative launch (persist.cu) where it can go wrong:
 one slice of block rows, a last slice that is not full, as many slices as
-blocks and one more, several launches per solve, loads at the ends of the
+blocks and one more, partly fixed nodes (padded to whole blocks), blocks of
+one to six columns, some of them stopped long before the others, several
+launches per solve, loads at the ends of the
 exponent range (the digit window of the grid sums follows the residual), a
 matrix and a load whose norms differ by many orders, and a load with a NaN.
 
@@ -13,7 +15,7 @@ import pytest
 import elastic_gb300 as E
 import oracle as O
 from elastic_gb300 import meshgen as M
-from helpers import rel_inf
+from helpers import rel_inf, rollers
 
 pytestmark = pytest.mark.gpu
 
@@ -25,6 +27,11 @@ CASES = {
     "quad4 152 slices": lambda: M.box2d(64, 75, etype=M.QUAD4_STRESS),
     "tria3 153 slices": lambda: M.box2d(72, 67, etype=M.TRIA3_STRAIN),
     "tetra4": lambda: M.box_tetra4(9, 8, 7, jitter=0.2, lognormal_E=True, nu_range=(0.25, 0.45)),
+    # partly fixed nodes: one, two and three dofs free, on lower and upper neighbours
+    "hexa8 rollers": lambda: rollers(rollers(M.box_hexa8(7, 5, 6), 0), 1),
+    "tetra4 rollers": lambda: rollers(M.box_tetra4(5, 6, 4, jitter=0.15), 1),
+    "quad4 rollers": lambda: rollers(M.box2d(23, 17, etype=M.QUAD4_STRAIN), 1),
+    "tria3 rollers": lambda: rollers(M.box2d(90, 71, etype=M.TRIA3_STRESS), 1),
 }
 
 
@@ -87,3 +94,27 @@ def test_load_that_is_not_finite_does_not_converge(gpu_ctx, bad):
     assert i["status"] == E.ERR_NO_CONVERGENCE
     x, i = gpu_ctx.solve(b, tol=1e-10)
     assert i["status"] == 0 and np.isfinite(x).all()
+
+
+@pytest.mark.parametrize("name", ["hexa8 one slice", "quad4 152 slices", "tetra4"])
+@pytest.mark.parametrize("nrhs", [1, 2, 3, 5, 6, 7])
+def test_columns_match_single_solves(gpu_ctx, name, nrhs):
+    """Each column's iterates are those of the single solve; a zero column and
+    one that is solved early do not disturb the others."""
+    _, _, _, b = _system(gpu_ctx, CASES[name]())
+    rng = np.random.default_rng(nrhs)
+    B = rng.standard_normal((b.size, nrhs))
+    if nrhs > 2:
+        B[:, 1] = 0.0
+    X, infos = gpu_ctx.solve_block(B, precision=E.PREC_FP64, tol=1e-11, maxit=20000)
+    for c in range(nrhs):
+        x, i = gpu_ctx.solve(B[:, c], tol=1e-11, maxit=20000)
+        assert infos[c]["status"] == 0 and abs(infos[c]["iters"] - i["iters"]) <= 2
+        assert rel_inf(x, X[:, c]) <= 1e-10 if x.any() else not X[:, c].any()
+        np.testing.assert_allclose(infos[c]["xkx"], i["xkx"], rtol=1e-10)
+    # a column of another magnitude leaves the others' bits alone
+    B[:, 0] *= 1e-30
+    X2, infos2 = gpu_ctx.solve_block(B, precision=E.PREC_FP64, tol=1e-11, maxit=20000)
+    assert rel_inf(1e-30 * X[:, 0], X2[:, 0]) <= 1e-10
+    for c in range(1, nrhs):
+        assert np.array_equal(X[:, c], X2[:, c]) and infos2[c]["iters"] == infos[c]["iters"]

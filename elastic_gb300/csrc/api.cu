@@ -367,20 +367,19 @@ void capture_pcg_graph(elx_ctx *c) {
   c->pcg_graph_iters = kBatch;
 }
 
-// Launches batches of `graph` until the scalars' stopping flag is set (two
-// batches in flight; the host reads the flag of the older one).
-elx::PcgScalars run_batches(elx_ctx *c, cudaGraphExec_t graph, double kernels_per_iter,
-                            int maxit) {
+// Launches batches of `size` iterations (`launch`) until the scalars' stopping
+// flag is set (two batches in flight; the host reads the flag of the older one).
+template <class F>
+elx::PcgScalars run_batches(elx_ctx *c, int size, int maxit, F launch) {
   elx::PcgScalars *d_sc = c->scal.as<elx::PcgScalars>();
   int launched = 0, checked = 0;
   auto launch_batch = [&](int slot) {
-    ELX_CUDA(cudaGraphLaunch(graph, c->stream));
-    c->launches += (int64_t)(kernels_per_iter * kBatch + 0.5);
+    launch();
     ELX_CUDA(cudaMemcpyAsync(&c->h_scal[slot], d_sc, sizeof(elx::PcgScalars),
                              cudaMemcpyDeviceToHost, c->stream));
     ELX_CUDA(cudaEventRecord(c->ev[slot], c->stream));
   };
-  const int max_batches = maxit / kBatch + 2;
+  const int max_batches = maxit / size + 2;
   launch_batch(0);
   launched = 1;
   if (max_batches > 1) {
@@ -400,6 +399,14 @@ elx::PcgScalars run_batches(elx_ctx *c, cudaGraphExec_t graph, double kernels_pe
   elx::PcgScalars last;
   ELX_CUDA(cudaMemcpy(&last, d_sc, sizeof(last), cudaMemcpyDeviceToHost));
   return last;
+}
+
+elx::PcgScalars run_batches(elx_ctx *c, cudaGraphExec_t graph, double kernels_per_iter,
+                            int maxit) {
+  return run_batches(c, kBatch, maxit, [&] {
+    ELX_CUDA(cudaGraphLaunch(graph, c->stream));
+    c->launches += (int64_t)(kernels_per_iter * kBatch + 0.5);
+  });
 }
 
 void fill_info(elx_ctx *c, elx_info *info, const elx::PcgScalars &sc, double secs) {
@@ -513,7 +520,8 @@ void pcg_mixed(elx_ctx *c, double tol, int maxit, elx_info *info) {
   auto t0 = std::chrono::steady_clock::now();
   ensure_fp32(c);
   build_preconditioner(c);
-  if (!c->pcg32_graph) c->pcg32_graph = capture_batch(c, true);
+  const bool persist = mixed_persist(c);
+  if (!persist && !c->pcg32_graph) c->pcg32_graph = capture_batch(c, true);
   const int n = c->s.neq;
   double *bmb_d = c->diag.as<double>() + 4;
   // r_hi = b (x = 0), r = (float) b, (b, M b) in FP64
@@ -540,7 +548,10 @@ void pcg_mixed(elx_ctx *c, double tol, int maxit, elx_info *info) {
                         c->p32.as<float>(), c->scal.as<elx::PcgScalars>(),
                         c->partials.as<double>(), c->counters.as<unsigned int>() + 2, c->stream);
   c->launches += 2;
-  elx::PcgScalars last = run_batches(c, c->pcg32_graph, 3 + 3.0 / kReplaceEvery, maxit);
+  elx::PcgScalars last =
+      persist ? run_batches(c, kPersistSteps, maxit,
+                            [&] { mixed_persist_steps(c, kReplaceEvery, kPersistSteps); })
+              : run_batches(c, c->pcg32_graph, 3 + 3.0 / kReplaceEvery, maxit);
   // fold the last FP32 piece (zero unless maxit stopped the iteration)
   elx::launch_refine_accumulate(n, c->xs.as<double>(), c->x32.as<float>(), false, c->stream);
   c->launches += 1;

@@ -240,6 +240,8 @@ void release_block(elx_ctx *c);
 bool ensure_persist(elx_ctx *c);
 int persist_columns(elx_ctx *c, int want);
 int persist_rows(const elx_ctx *c);
+bool mixed_persist(elx_ctx *c);
+void mixed_persist_steps(elx_ctx *c, int replace_every, int steps);
 void persist_solve(elx_ctx *c, int nc, double tol, int maxit, const double *b, double *x,
                    double *work, int steps, elx::PersistCol *out);
 // Row-block partitions on one device (partition.cu).

@@ -532,6 +532,19 @@ void persist_solve(elx_ctx *c, int nc, double tol, int maxit, const double *b, d
     ELX_CUDA(cudaEventRecord(c->ev[slot], c->stream));
     launched++;
   };
+  // a server's block solve asks the gate before each launch and polls it
+  auto gate = [&](int enter) {
+    if (c->batch_gate) c->batch_gate(c->batch_gate_user, enter);
+  };
+  struct Leave {  // also when a launch or a poll throws
+    decltype(gate) &g;
+    bool in = false;
+    ~Leave() {
+      if (in) g(0);
+    }
+  } leave{gate};
+  gate(1);
+  leave.in = true;
   go();
   for (;;) {
     if (launched < max_launches && !c->batch_gate) go();
@@ -544,7 +557,13 @@ void persist_solve(elx_ctx *c, int nc, double tol, int maxit, const double *b, d
       std::copy(h, h + nc, out);
       break;
     }
-    if (c->batch_gate) go();
+    if (c->batch_gate) {
+      leave.in = false;
+      gate(0);
+      gate(1);
+      leave.in = true;
+      go();
+    }
   }
   c->sync();
 }

@@ -118,3 +118,27 @@ def test_columns_match_single_solves(gpu_ctx, name, nrhs):
     assert rel_inf(1e-30 * X[:, 0], X2[:, 0]) <= 1e-10
     for c in range(1, nrhs):
         assert np.array_equal(X[:, c], X2[:, c]) and infos2[c]["iters"] == infos[c]["iters"]
+
+
+@pytest.mark.parametrize("name", sorted(k for k in CASES if "rollers" not in k))
+def test_mixed_meets_the_fp64_test(gpu_ctx, name):
+    s, ad, al, b = _system(gpu_ctx, CASES[name]())
+    x_o, _ = O.pcg(s, ad, al, b, tol=1e-13, maxit=20000)
+    x, i = gpu_ctx.solve(b, precision=E.PREC_MIXED, tol=1e-10, maxit=20000)
+    assert i["status"] == 0 and i["norm_m_r"] <= 3.16 * i["conv"]
+    assert rel_inf(x_o, x) <= 1e-6
+    x2, i2 = gpu_ctx.solve(b, precision=E.PREC_MIXED, tol=1e-10, maxit=20000)
+    assert np.array_equal(x, x2) and i["inner_iters"] == i2["inner_iters"]
+
+
+def test_mixed_maxit_and_bad_load(gpu_ctx):
+    _, _, _, b = _system(gpu_ctx, M.box_hexa8(9, 8, 8, jitter=0.1))
+    for maxit in (1, 6, 8):  # the test is made at every fourth iteration
+        _, i = gpu_ctx.solve(b, precision=E.PREC_MIXED, tol=1e-12, maxit=maxit, raise_on_error=False)
+        assert i["status"] == E.ERR_NO_CONVERGENCE and maxit <= i["iters"] < maxit + 4
+    c = b.copy()
+    c[5] = np.nan
+    _, i = gpu_ctx.solve(c, precision=E.PREC_MIXED, tol=1e-10, maxit=100, raise_on_error=False)
+    assert i["status"] == E.ERR_NO_CONVERGENCE
+    _, i = gpu_ctx.solve(b, precision=E.PREC_MIXED, tol=1e-10)
+    assert i["status"] == 0

@@ -128,8 +128,8 @@ __device__ __forceinline__ bool slot_sum(GridSync *gs, FixSum &f, uint64_t epoch
     FixSum t;
     t.m = 0;
 #pragma unroll
-    for (int k = 0; k < K; k++) t.m += v[k].m >> min(e - v[k].e + 3, 63);
-    t.e = e + 3;
+    for (int k = 0; k < K; k++) t.m += fix_align(v[k], e, 3);
+    t.e = e >= kFixBad ? e : e + 3;
     t = warp_sum(t);
     if (lane == c) f = t;
   }
@@ -159,7 +159,7 @@ __device__ __forceinline__ bool digit_sum(GridSync *gs, GridWords *words, FixSum
     uint64_t a = g.m < 0 ? -g.m : g.m;
     int s = g.e - glo;  // place of a's lowest bit in the window
     unsigned long long add = kOne + kBias;
-    if (g.m != 0 || g.e >= kFixBad) {
+    if (g.m != 0) {
       if (s > 32 * kDigits - 68) {  // 58 bits and 8 of 152 addends
         add += kMark;
       } else {

@@ -330,6 +330,7 @@ enum GatherEpi : int {
   kEpiBicgAlpha = 2,  // pq = (w, y), alpha = rho / pq, iters += 1   (w = r0)
   kEpiBicgOmega = 3,  // omega = (w, y) / (y, y)                      (w = r)
   kEpiScale = 4,      // y = w .* (K x), no dot                       (w = M)
+  kEpiDot = 5,        // *dot = (x, y)                                (no solve)
 };
 void launch_gather_epi64(const CsrcDev &k, int epi, const double *x, double *y, const double *w,
                          PcgScalars *sc, double *partials, unsigned int *counter,

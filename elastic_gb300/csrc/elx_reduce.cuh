@@ -1,5 +1,5 @@
 // Deterministic block and grid reductions used by the solver kernels: each
-// block reduces its threads in a fixed tree, writes one partial per block,
+// block adds its threads' values in integers, writes one partial per block,
 // and the last block to arrive (atomic ticket) sums the partials in a fixed
 // order.  Same grid, same inputs -> bitwise the same result.
 #pragma once
@@ -9,13 +9,6 @@
 namespace elx {
 
 constexpr int kThreads = 256;
-
-template <class T>
-__device__ __forceinline__ T warp_sum(T v) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-  return v;
-}
 
 // A sum in integer form: value = m 2^e with |m| < 2^58.  GB300 runs an FP64
 // instruction of a warp in 64 clocks per SM quarter, however few lanes are
@@ -28,16 +21,33 @@ struct FixSum {
   int64_t m;
   int32_t e;
 };
-constexpr int32_t kFixBad = 1 << 20;  // exponent of a sum with an infinity or NaN
+// Exponent of a sum with an infinity or NaN: m then counts the +infinities
+// (from bit 0), -infinities (bit 20) and NaNs (bit 40) among its terms.
+constexpr int32_t kFixBad = 1 << 20;
+
+__device__ __forceinline__ int64_t fix_class(bool nan, bool neg) {
+  return nan ? 1ll << 40 : neg ? 1ll << 20 : 1ll;
+}
+
+// m of a term in a sum with exponent e, k bits lower.
+__device__ __forceinline__ int64_t fix_align(FixSum f, int e, int k) {
+  if (e >= kFixBad) return f.e >= kFixBad ? f.m : 0;
+  return f.m >> min(e - f.e + k, 63);
+}
 
 __device__ __forceinline__ FixSum fix_of(double v) {
   const int64_t b = __double_as_longlong(v);
   const int ex = (int)((uint64_t)b >> 52) & 0x7ff;
   int64_t m = b & 0xfffffffffffffll;
-  if (ex) m |= 0x10000000000000ll;
   FixSum f;
+  if (ex == 0x7ff) {
+    f.m = fix_class(m != 0, b < 0);
+    f.e = kFixBad;
+    return f;
+  }
+  if (ex) m |= 0x10000000000000ll;
   f.m = (b < 0 ? -m : m) << 5;
-  f.e = ex == 0x7ff ? kFixBad : m ? max(ex, 1) - 1080 : -4096;
+  f.e = m ? max(ex, 1) - 1080 : -4096;
   return f;
 }
 
@@ -45,18 +55,23 @@ __device__ __forceinline__ FixSum fix_of(float v) {
   const uint32_t b = __float_as_uint(v);
   const int ex = (int)(b >> 23) & 0xff;
   int64_t m = b & 0x7fffffu;
+  FixSum f;
+  if (ex == 0xff) {
+    f.m = fix_class(m != 0, (int32_t)b < 0);
+    f.e = kFixBad;
+    return f;
+  }
   if (ex) m |= 0x800000;
   m <<= 34;
-  FixSum f;
   f.m = (int32_t)b < 0 ? -m : m;
-  f.e = ex == 0xff ? kFixBad : m ? max(ex, 1) - 184 : -4096;
+  f.e = m ? max(ex, 1) - 184 : -4096;
   return f;
 }
 
 // The sum over the 32 lanes, in every lane.
 __device__ __forceinline__ FixSum warp_sum(FixSum f) {
   const int e = __reduce_max_sync(0xffffffffu, f.e);
-  const int64_t m = f.m >> min(e - f.e, 63);
+  const int64_t m = fix_align(f, e, 0);
   const uint32_t lo = __reduce_add_sync(0xffffffffu, (uint32_t)m & 0x7ffffffu);
   const uint32_t mid = __reduce_add_sync(0xffffffffu, (uint32_t)(m >> 27) & 0x7ffffffu);
   const int32_t hi = __reduce_add_sync(0xffffffffu, (int32_t)(m >> 54));
@@ -64,13 +79,22 @@ __device__ __forceinline__ FixSum warp_sum(FixSum f) {
   // back to 58 bits (leading zeros of |t| to 6), so that no stage loses bits
   const int sh = 6 - __clzll(t < 0 ? -t : t);
   FixSum r;
+  if (e >= kFixBad) {
+    r.m = t;
+    r.e = kFixBad;
+    return r;
+  }
   r.m = sh > 0 ? t >> sh : t << -sh;
   r.e = t ? e + sh : -4096;
   return r;
 }
 
 __device__ __forceinline__ double fix_value(FixSum f) {
-  if (f.e >= kFixBad) return __longlong_as_double(0x7ff8000000000000ll);
+  if (f.e >= kFixBad) {
+    const bool pos = f.m & 0xfffff, neg = f.m >> 20 & 0xfffff;
+    return __longlong_as_double(f.m >> 40 || (pos && neg) ? 0x7ff8000000000000ll
+                                : neg ? (int64_t)0xfff0000000000000ull : 0x7ff0000000000000ll);
+  }
   if (f.m == 0) return 0.0;
   // 58 bits rounded to 53; the carry of a rounding up runs into the exponent
   const uint64_t a = (uint64_t)(f.m < 0 ? -f.m : f.m) + 16 >> 5;
@@ -86,38 +110,18 @@ __device__ __forceinline__ double fix_value(FixSum f) {
   return v;
 }
 
-// Block-wide sum of NV values (fixed order); result valid in thread 0.
-template <int NV>
-__device__ __forceinline__ void block_sum(double (&v)[NV]) {
-  __shared__ double sh[NV][kThreads / 32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int i = 0; i < NV; i++) {
-    v[i] = warp_sum(v[i]);
-    if (lane == 0) sh[i][w] = v[i];
-  }
-  __syncthreads();
-  if (w == 0) {
-#pragma unroll
-    for (int i = 0; i < NV; i++) {
-      double t = lane < kThreads / 32 ? sh[i][lane] : 0.0;
-      v[i] = warp_sum(t);
-    }
-  }
-}
-
-// Block-wide sum of NV per-thread values of type T (float in the FP32
-// kernels): the warp stage adds in T, the per-warp sums are widened to double
-// and added in a fixed order.  Keeps the FP32 kernels off the (narrow) FP64
-// pipe except for a handful of additions per block.  Result in thread 0.
+// Block-wide sum of NV per-thread values (double or float; kThreads threads);
+// result valid in thread 0.  In integers (FixSum): as FP64 shuffle trees the
+// two stages were 45 FP64 warp instructions a block, 12 us of 95 in a product
+// of 64 rows per block, and 1,200 clocks at the end of every fused dot.
 template <int NV, class T>
 __device__ __forceinline__ void block_sum_widen(const T (&v)[NV], double (&out)[NV]) {
-  __shared__ double sh[NV][kThreads / 32];
+  __shared__ FixSum sh[NV][kThreads / 32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
   for (int i = 0; i < NV; i++) {
-    const T s = warp_sum(v[i]);
-    if (lane == 0) sh[i][w] = (double)s;
+    const FixSum s = warp_sum(fix_of(v[i]));
+    if (lane == 0) sh[i][w] = s;
   }
   __syncthreads();
 #pragma unroll
@@ -125,10 +129,21 @@ __device__ __forceinline__ void block_sum_widen(const T (&v)[NV], double (&out)[
   if (w == 0) {
 #pragma unroll
     for (int i = 0; i < NV; i++) {
-      double t = lane < kThreads / 32 ? sh[i][lane] : 0.0;
-      out[i] = warp_sum(t);
+      FixSum t;
+      t.m = 0;
+      t.e = -4096;
+      if (lane < kThreads / 32) t = sh[i][lane];
+      out[i] = fix_value(warp_sum(t));
     }
   }
+}
+
+template <int NV>
+__device__ __forceinline__ void block_sum(double (&v)[NV]) {
+  double out[NV];
+  block_sum_widen<NV>(v, out);
+#pragma unroll
+  for (int i = 0; i < NV; i++) v[i] = out[i];
 }
 
 // Writes this block's NV partials and returns true in thread 0 of the last

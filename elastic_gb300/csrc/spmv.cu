@@ -285,10 +285,10 @@ gather_spmv_kernel(int neq, const int32_t *__restrict__ ia, const int32_t *__res
                    const T *__restrict__ w, PcgScalars *sc, double *partials,
                    unsigned int *counter, const int32_t *gate,
                    const uint16_t *__restrict__ ja16 = nullptr,
-                   const uint16_t *__restrict__ jat16 = nullptr) {
-  constexpr bool DOT = EPI == kEpiPcg || EPI == kEpiBicgAlpha || EPI == kEpiBicgOmega;
+                   const uint16_t *__restrict__ jat16 = nullptr, double *dot = nullptr) {
+  constexpr bool DOT = EPI != kEpiNone && EPI != kEpiScale;
   constexpr int NV = EPI == kEpiBicgOmega ? 2 : 1;
-  if (DOT && sc->done) return;
+  if (DOT && EPI != kEpiDot && sc->done) return;
   if (gate && *gate == 0) return;
   constexpr int RPB = 256 / LANES;  // rows per block pass
   const int lane = threadIdx.x % LANES, sub = threadIdx.x / LANES;
@@ -336,7 +336,7 @@ gather_spmv_kernel(int neq, const int32_t *__restrict__ ia, const int32_t *__res
       T yi = ad[row] * xi + s;
       if (EPI == kEpiScale) yi = yi * w[row];
       y[row] = yi;
-      if (EPI == kEpiPcg) v[0] += xi * yi;
+      if (EPI == kEpiPcg || EPI == kEpiDot) v[0] += xi * yi;
       if (EPI == kEpiBicgAlpha) v[0] += yi * w[row];
       if (EPI == kEpiBicgOmega) {
         v[0] += yi * w[row];
@@ -360,6 +360,8 @@ gather_spmv_kernel(int neq, const int32_t *__restrict__ ia, const int32_t *__res
       sc->iters += 1;
     } else if (EPI == kEpiBicgOmega) {
       sc->omega = tot[0] / tot[NV - 1];
+    } else if (EPI == kEpiDot) {
+      *dot = tot[0];
     }
   }
 }
@@ -550,13 +552,19 @@ void launch_gather_epi64(const CsrcDev &k, int epi, const double *x, double *y, 
 namespace elx {
 namespace {
 
-constexpr int kNoAllocMaxBlocks = 16384;          // partial sums in the scratch
-constexpr int kNoAllocRowsPerBlock = 256 / 4;     // rows per block of the kernel
-constexpr int64_t kNoAllocMaxRows = (int64_t)kNoAllocMaxBlocks * kNoAllocRowsPerBlock;
+constexpr int kNoAllocMaxBlocks = 16384;       // partial sums in the scratch
+constexpr int64_t kNoAllocMaxRows = 1 << 20;   // the documented limit
+// Two lanes per row, eight entries in flight each: the columns are 32-bit here
+// (no offsets), and fewer lanes per row idle less in a row's last step and need
+// one shuffle add instead of two (330,750 rows of 74 entries: 99.5 us; lanes x
+// entries 4 x 4 102.5, 4 x 2 106.7, 2 x 4 108.9, 1 x 8 120, 8 x 4 149; 85.4 as one
+// launch with integer block sums)
+constexpr int kNoAllocLanes = 2;
+constexpr int kNoAllocRowsPerBlock = 256 / kNoAllocLanes;
+static_assert(kNoAllocMaxRows / kNoAllocRowsPerBlock <= kNoAllocMaxBlocks, "scratch too small");
 
 struct NoAllocScratch {
   double partials[kNoAllocMaxBlocks];
-  PcgScalars scalars;
   unsigned int counter;
 };
 
@@ -588,18 +596,12 @@ extern "C" int elx_spmv_dot_noalloc(int32_t neq, const int32_t *ia, const int32_
     g_noalloc_addr[dev].store(sc, std::memory_order_release);
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // the scalars and the ticket must start at zero (done = 0 lets the kernel
-  // run; the ticket counts the blocks that have published their partials)
-  if (cudaMemsetAsync(&sc->scalars, 0, sizeof(PcgScalars), st) != cudaSuccess ||
-      cudaMemsetAsync(&sc->counter, 0, sizeof(unsigned int), st) != cudaSuccess)
-    return ELX_ERR_CUDA;
+  // one launch: the ticket starts at zero, every launch leaves it there, and
+  // the last block writes *xy
   const int grid = (neq + kNoAllocRowsPerBlock - 1) / kNoAllocRowsPerBlock;
-  gather_spmv_kernel<double, 4, 4, kEpiPcg, 1><<<grid, 256, 0, st>>>(
-      neq, ia, ja, al, iat, jat, alt, ad, x, y, nullptr, &sc->scalars, sc->partials,
-      &sc->counter, nullptr);
+  gather_spmv_kernel<double, kNoAllocLanes, 8, kEpiDot, 1><<<grid, 256, 0, st>>>(
+      neq, ia, ja, al, iat, jat, alt, ad, x, y, nullptr, nullptr, sc->partials, &sc->counter,
+      nullptr, nullptr, nullptr, xy);
   if (cudaGetLastError() != cudaSuccess) return ELX_ERR_CUDA;
-  if (cudaMemcpyAsync(xy, &sc->scalars.pq, sizeof(double), cudaMemcpyDeviceToDevice, st) !=
-      cudaSuccess)
-    return ELX_ERR_CUDA;
   return ELX_OK;
 }

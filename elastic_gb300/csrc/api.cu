@@ -650,12 +650,29 @@ void bicgstab64(elx_ctx *c, double tol, int maxit, elx_info *info, bool plain) {
 void gmres64(elx_ctx *c, int kdim, double tol, int maxit, elx_info *info) {
   auto t0 = std::chrono::steady_clock::now();
   require(kdim >= 1 && kdim <= kMaxGmresK, ELX_ERR_ARG, "GMRES restart length out of range");
-  const size_t n = (size_t)c->s.neq;
-  if (c->gmres_k != kdim || !c->gbasis.p) {
+  bool persist = ensure_gmres_persist(c, kdim);
+  // the basis by equations, or by rows of the sliced matrix
+  size_t n = persist ? (size_t)persist_rows(c) : (size_t)c->s.neq;
+  if (c->gmres_k == kdim && c->gbasis.p) {
+    persist = c->gmres_persist;
+    n = persist ? (size_t)persist_rows(c) : (size_t)c->s.neq;
+  } else {
     if (c->gmres_graph) cudaGraphExecDestroy(c->gmres_graph);
     c->gmres_graph = nullptr;
-    c->alloc(c->gbasis, n * 8 * (size_t)(kdim + 1));
-    c->alloc(c->garrays, elx::gmres_array_doubles(kdim) * 8);
+    c->gmres_k = 0;
+    try {
+      c->alloc(c->gbasis, n * 8 * (size_t)(kdim + 1));
+      c->alloc(c->garrays,
+               persist ? gmres_persist_bytes(kdim) : elx::gmres_array_doubles(kdim) * 8);
+    } catch (const Error &e) {
+      if (e.code != ELX_ERR_OOM || !persist) throw;
+      // a memory budget without room for the cooperative cycle's words
+      persist = false;
+      n = (size_t)c->s.neq;
+      c->alloc(c->gbasis, n * 8 * (size_t)(kdim + 1));
+      c->alloc(c->garrays, elx::gmres_array_doubles(kdim) * 8);
+    }
+    c->gmres_persist = persist;
     if (!c->gstate.p) c->alloc(c->gstate, sizeof(elx::GmresState));
     c->gmres_k = kdim;
   }
@@ -670,7 +687,8 @@ void gmres64(elx_ctx *c, int kdim, double tol, int maxit, elx_info *info) {
                          c->gbasis.as<double>(), gs, c->partials.as<double>(),
                          c->counters.as<unsigned int>() + 2, c->stream);
   c->launches += 1;
-  if (!c->gmres_graph) {
+  if (persist) ELX_CUDA(cudaMemsetAsync(c->persist_vec.p, 0, n * 8, c->stream));  // x by rows
+  if (!persist && !c->gmres_graph) {
     cudaGraph_t g;
     ELX_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     try {
@@ -692,6 +710,12 @@ void gmres64(elx_ctx *c, int kdim, double tol, int maxit, elx_info *info) {
     ELX_CUDA(cudaMemcpyAsync(&st, gs, sizeof(st), cudaMemcpyDeviceToHost, c->stream));
     c->sync();
     if (!st.live) break;
+    if (persist) {
+      gmres_persist_cycle(c, kdim, c->gbasis.as<double>(), c->persist_vec.as<double>(),
+                          c->garrays.p);
+      check_pipe_waits(c);
+      continue;
+    }
     ELX_CUDA(cudaGraphLaunch(c->gmres_graph, c->stream));
     c->launches += c->gmres_launches;
   }

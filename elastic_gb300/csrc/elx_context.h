@@ -115,6 +115,7 @@ struct elx_ctx {
   bool bicg_plain = false;                // bicg_graph has M = I (no preconditioner)
   cudaGraphExec_t gmres_graph = nullptr;  // one GMRES(gmres_k) restart cycle
   int gmres_k = 0, gmres_launches = 0;
+  bool gmres_persist = false;  // gbasis and garrays are the cooperative cycle's
   int pcg_graph_iters = 0;
   cudaEvent_t ev[2] = {nullptr, nullptr};
   cudaEvent_t ev_t[2] = {nullptr, nullptr};  // timing (autotuner)
@@ -241,6 +242,9 @@ bool ensure_persist(elx_ctx *c);
 int persist_columns(elx_ctx *c, int want);
 int persist_rows(const elx_ctx *c);
 bool mixed_persist(elx_ctx *c);
+bool ensure_gmres_persist(elx_ctx *c, int k);
+size_t gmres_persist_bytes(int k);
+void gmres_persist_cycle(elx_ctx *c, int k, double *basis, double *xr, void *dots);
 void mixed_persist_steps(elx_ctx *c, int replace_every, int steps);
 void persist_solve(elx_ctx *c, int nc, double tol, int maxit, const double *b, double *x,
                    double *work, int steps, elx::PersistCol *out);

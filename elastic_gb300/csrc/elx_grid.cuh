@@ -94,14 +94,20 @@ struct Bound {
   }
 };
 
+// The blocks that work together: all of a launch, or some.
+struct Team {
+  int me, n;
+};
+
 // The blocks' sums through a slot of each block (value, exponent and epoch in
-// one 16-byte store); warp 0, lane c holds sum c.
+// one 16-byte store); one warp, lane c holds sum c.
 template <int NC>
-__device__ __forceinline__ bool slot_sum(GridSync *gs, FixSum &f, uint64_t epoch) {
+__device__ __forceinline__ bool slot_sum(Team t, GridSlot (*slots)[kGridMaxBlocks], FixSum &f,
+                                         uint64_t epoch) {
   constexpr int K = kGridMaxBlocks / 32;
   const int lane = threadIdx.x & 31;
   if (lane < NC)
-    store_slot(gs->slot[lane] + blockIdx.x, f.m,
+    store_slot(slots[lane] + t.me, f.m,
                epoch << 24 | (uint64_t)(uint32_t)(f.e + 4096));
   bool ok = true;
   Bound bound;
@@ -112,8 +118,8 @@ __device__ __forceinline__ bool slot_sum(GridSync *gs, FixSum &f, uint64_t epoch
       v[k].m = 0;
       v[k].e = -4096;
       const int b = lane + 32 * k;
-      while (b < (int)gridDim.x && ok) {
-        const GridSlot g = load_slot(gs->slot[c] + b);
+      while (b < t.n && ok) {
+        const GridSlot g = load_slot(slots[c] + b);
         if (g.tag >> 24 == epoch) {
           v[k].m = g.m;
           v[k].e = (int32_t)(g.tag & 0xffffffu) - 4096;
@@ -125,13 +131,13 @@ __device__ __forceinline__ bool slot_sum(GridSync *gs, FixSum &f, uint64_t epoch
     int e = v[0].e;
 #pragma unroll
     for (int k = 1; k < K; k++) e = max(e, v[k].e);
-    FixSum t;
-    t.m = 0;
+    FixSum q;
+    q.m = 0;
 #pragma unroll
-    for (int k = 0; k < K; k++) t.m += fix_align(v[k], e, 3);
-    t.e = e >= kFixBad ? e : e + 3;
-    t = warp_sum(t);
-    if (lane == c) f = t;
+    for (int k = 0; k < K; k++) q.m += fix_align(v[k], e, 3);
+    q.e = e >= kFixBad ? e : e + 3;
+    q = warp_sum(q);
+    if (lane == c) f = q;
   }
   return __all_sync(0xffffffffu, ok);
 }
@@ -142,42 +148,49 @@ __device__ __forceinline__ int window_of(double ref) {
   return ex - 1023 - 120;
 }
 
-// The blocks' sums of f (warp 0, lane c holds sum c and `lo`, the exponent of
-// its lowest digit).  `seen`: this lane's word after the last sum.  False in
-// every lane when the bound ran out.
+constexpr unsigned long long kOne = 1ull << 48, kBias = 1ull << 33, kMark = 1ull << 56;
+
+// Adds this block's f to the digits (one warp; lane c holds sum c and `lo`,
+// the exponent of its lowest digit).
 template <int NC>
-__device__ __forceinline__ bool digit_sum(GridSync *gs, GridWords *words, FixSum &f, int lo,
-                                          unsigned long long &seen, uint64_t epoch) {
+__device__ __forceinline__ void digit_add(GridWords *words, FixSum f, int lo) {
   static_assert(NC * kDigits <= 32, "one lane per digit");
-  constexpr unsigned long long kOne = 1ull << 48, kBias = 1ull << 33, kMark = 1ull << 56;
-  const int lane = threadIdx.x & 31, n = gridDim.x;
+  const int lane = threadIdx.x & 31;
   const int col = min(lane / kDigits, NC - 1), k0 = lane - col * kDigits;
   const FixSum g = fix_shfl(f, col);
   const int glo = __shfl_sync(0xffffffffu, lo, col);
-  const bool on = lane < NC * kDigits;
-  if (on) {
-    uint64_t a = g.m < 0 ? -g.m : g.m;
-    int s = g.e - glo;  // place of a's lowest bit in the window
-    unsigned long long add = kOne + kBias;
-    if (g.m != 0) {
-      if (s > 32 * kDigits - 68) {  // 58 bits and 8 of 152 addends
-        add += kMark;
-      } else {
-        if (s < 0) {
-          a >>= min(-s, 63);
-          s = 0;
-        }
-        const int off = 32 * k0 - s;
-        const uint64_t d =
-            (off >= 64 || off <= -32 ? 0 : off >= 0 ? a >> off : a << -off) & 0xffffffffull;
-        add += g.m < 0 ? -d : d;
+  if (lane >= NC * kDigits) return;
+  uint64_t a = g.m < 0 ? -g.m : g.m;
+  int s = g.e - glo;  // place of a's lowest bit in the window
+  unsigned long long add = kOne + kBias;
+  if (g.m != 0) {
+    if (s > 32 * kDigits - 68) {  // 58 bits and 8 of 152 addends
+      add += kMark;
+    } else {
+      if (s < 0) {
+        a >>= min(-s, 63);
+        s = 0;
       }
+      const int off = 32 * k0 - s;
+      const uint64_t d =
+          (off >= 64 || off <= -32 ? 0 : off >= 0 ? a >> off : a << -off) & 0xffffffffull;
+      add += g.m < 0 ? -d : d;
     }
-    red_add(words->digit + lane, add);
   }
+  red_add(words->digit + lane, add);
+}
+
+// Waits for the n blocks' additions and replaces f by the sums (the same warp).
+// `seen`: this lane's word after the last sum.  False in every lane when the
+// bound ran out.
+template <int NC>
+__device__ __forceinline__ bool digit_read(Team t, GridSlot (*slots)[kGridMaxBlocks],
+                                           GridWords *words, FixSum &f, int lo,
+                                           unsigned long long &seen, uint64_t epoch) {
+  const int lane = threadIdx.x & 31, n = t.n;
   unsigned long long w = 0;
   bool ok = true;
-  if (on) {
+  if (lane < NC * kDigits) {
     Bound bound;
     for (;;) {
       w = load_relaxed(words->digit + lane);
@@ -191,7 +204,7 @@ __device__ __forceinline__ bool digit_sum(GridSync *gs, GridWords *words, FixSum
   if (!__all_sync(0xffffffffu, ok)) return false;
   const unsigned long long diff = w - seen;
   seen = w;
-  if (__any_sync(0xffffffffu, diff >> 56 != 0)) return slot_sum<NC>(gs, f, epoch);
+  if (__any_sync(0xffffffffu, diff >> 56 != 0)) return slot_sum<NC>(t, slots, f, epoch);
   const int64_t d = (int64_t)(diff & (kOne - 1)) - (int64_t)n * (int64_t)kBias;
   // lane c: its sum's digits, carried upwards (32 bits each, the top one signed)
   int64_t c[kDigits];
@@ -232,7 +245,7 @@ struct Scratch {
   int32_t ok;
 };
 
-// The sums of v[c] over the whole grid, each near |ref[c]| (shared memory;
+// The sums of v[c] over the team's blocks, each near |ref[c]| (shared memory;
 // nullptr: of any size).  `then(total)` runs in lane c of warp 0 with sum c
 // (FP64 arithmetic on the totals costs the pipe once instead of once per
 // warp) and leaves what the block needs in shared memory; `meanwhile()` runs
@@ -240,8 +253,8 @@ struct Scratch {
 // T: threads of the block (a multiple of 32, at most 1024).  False in every
 // thread when a wait ran out (the caller returns).
 template <int T, int NC, class V, class F, class H>
-__device__ __forceinline__ bool sum(const V (&v)[NC], GridSync *gs, int which, const double *ref,
-                                    unsigned long long &seen, uint64_t epoch, Scratch<T, NC> &sh,
+__device__ __forceinline__ bool sum(Team team, const V (&v)[NC], GridSync *gs, int which,
+                                    const double *ref, unsigned long long &seen, uint64_t epoch, Scratch<T, NC> &sh,
                                     F then, H meanwhile) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
@@ -263,9 +276,14 @@ __device__ __forceinline__ bool sum(const V (&v)[NC], GridSync *gs, int which, c
       t = warp_sum(t);
       if (lane == c) mine = t;
     }
-    const bool ok = ref ? digit_sum<NC>(gs, &gs->sum[which], mine,
-                                        window_of(ref[lane < NC ? lane : 0]), seen, epoch)
-                        : slot_sum<NC>(gs, mine, epoch);
+    bool ok;
+    if (ref) {
+      const int lo = window_of(ref[lane < NC ? lane : 0]);
+      digit_add<NC>(&gs->sum[which], mine, lo);
+      ok = digit_read<NC>(team, gs->slot, &gs->sum[which], mine, lo, seen, epoch);
+    } else {
+      ok = slot_sum<NC>(team, gs->slot, mine, epoch);
+    }
     if (lane < NC) then(fix_value(mine));
     if (lane == 0) sh.ok = ok;
   } else {
@@ -279,13 +297,14 @@ __device__ __forceinline__ bool sum(const V (&v)[NC], GridSync *gs, int which, c
 // sides order the data (and drop stale L1 lines).  `count`: barriers passed
 // in this launch, this one included.
 template <int T, int NC>
-__device__ __forceinline__ bool barrier(GridSync *gs, uint32_t count, Scratch<T, NC> &sh) {
+__device__ __forceinline__ bool barrier(Team team, GridSync *gs, uint32_t count,
+                                        Scratch<T, NC> &sh) {
   __syncthreads();
   if (threadIdx.x == 0) {
     fence();
     unsigned long long *p = gs->arrive.digit;
     red_add(p, 1);
-    const unsigned long long want = (unsigned long long)count * gridDim.x;
+    const unsigned long long want = (unsigned long long)count * team.n;
     bool ok = true;
     Bound bound;
     while (ok && load_relaxed(p) < want) ok = !bound.over();

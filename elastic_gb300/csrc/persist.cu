@@ -85,6 +85,7 @@ pcg_persist_kernel(PersistArgs a, int start, int steps) {
   int32_t *sptr = reinterpret_cast<int32_t *>(shead + kPW * RBC);  // group pointers of the slices
   int32_t *sga = sptr + a.slices + 1, *swsl = sga + kPW + 1;  // warps' first groups and slices
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const grid::Team team{(int)blockIdx.x, (int)gridDim.x};
   // every block reads the columns' states before the first wait, and block 0
   // writes them after the last
   int left = start;
@@ -176,7 +177,7 @@ pcg_persist_kernel(PersistArgs a, int start, int steps) {
       }
     }
     epoch++;
-    if (!grid::sum<kPT, NC>(v, a.gs, 0, nullptr, seen_pq, epoch, sred,
+    if (!grid::sum<kPT, NC>(team, v, a.gs, 0, nullptr, seen_pq, epoch, sred,
                             [&](double t) {
                               sd[lane] = t;
                               sconv[lane] = a.tol * sqrt(fabs(t));
@@ -189,7 +190,7 @@ pcg_persist_kernel(PersistArgs a, int start, int steps) {
       if (tid == 0) atomicExch(a.err, 2);
       return;
     }
-    if (!grid::barrier<kPT, NC>(a.gs, ++barriers, sred)) {
+    if (!grid::barrier<kPT, NC>(team, a.gs, ++barriers, sred)) {
       if (tid == 0) atomicExch(a.err, 2);
       return;
     }
@@ -247,7 +248,7 @@ pcg_persist_kernel(PersistArgs a, int start, int steps) {
       }
     }
     // alpha = d / (p, q); meanwhile the slices cut between warps are put together
-    if (!grid::sum<kPT, NC>(v, a.gs, 0, sd, seen_pq, epoch, sred,
+    if (!grid::sum<kPT, NC>(team, v, a.gs, 0, sd, seen_pq, epoch, sred,
                             [&](double t) {
                               // p = 0: no step; a stopped column stays as it is
                               salpha[lane] = son[lane] && t != 0.0 ? sd[lane] / t : 0.0;
@@ -280,7 +281,7 @@ pcg_persist_kernel(PersistArgs a, int start, int steps) {
         v[c] += ri * zi;
       }
     }
-    if (!grid::sum<kPT, NC>(v, a.gs, 1, sd, seen_rz, epoch + 1, sred,
+    if (!grid::sum<kPT, NC>(team, v, a.gs, 1, sd, seen_rz, epoch + 1, sred,
                             [&](double t) {
                               if (son[lane]) {
                                 sbeta[lane] = t / sd[lane];
@@ -322,7 +323,7 @@ pcg_persist_kernel(PersistArgs a, int start, int steps) {
       if (SMEM) sp[e] = pi;
       gp[e] = pi;
     }
-    if (!grid::barrier<kPT, NC>(a.gs, ++barriers, sred)) {
+    if (!grid::barrier<kPT, NC>(team, a.gs, ++barriers, sred)) {
       if (tid == 0) atomicExch(a.err, 2);
       return;
     }

@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(kMT, 1) mixed_persist_kernel(MixedArgs a, int 
   int32_t *sptr = reinterpret_cast<int32_t *>(shead + kMW * RB);
   int32_t *sga = sptr + a.slices + 1, *swsl = sga + kMW + 1;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const grid::Team team{(int)blockIdx.x, (int)gridDim.x};
   // block 0 writes the scalars after the last wait
   if (a.sc->done) return;
   const int s0 = a.cta[blockIdx.x], s1 = a.cta[blockIdx.x + 1], ns = s1 - s0;
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(kMT, 1) mixed_persist_kernel(MixedArgs a, int 
         sl++;
       }
     }
-    if (!grid::sum<kMT, 1>(v, a.gs, 0, sd, seen_pq, epoch, sred,
+    if (!grid::sum<kMT, 1>(team, v, a.gs, 0, sd, seen_pq, epoch, sred,
                            [&](double t) {
                              S.pq = t;
                              S.alpha = t != 0.0 ? sd[0] / t : 0.0;
@@ -189,7 +190,7 @@ __global__ void __launch_bounds__(kMT, 1) mixed_persist_kernel(MixedArgs a, int 
         v[0] += ri * zi;
       }
     }
-    if (!grid::sum<kMT, 1>(v, a.gs, 1, sd, seen_rz, epoch + 1, sred,
+    if (!grid::sum<kMT, 1>(team, v, a.gs, 1, sd, seen_rz, epoch + 1, sred,
                            [&](double t) {
                              // an FP32 residual of exactly zero: beta = 0, and
                              // the next replacement point takes over
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(kMT, 1) mixed_persist_kernel(MixedArgs a, int 
         a.p[row0 + i] = pi;
       }
     }
-    if (!grid::barrier<kMT, 1>(a.gs, ++barriers, sred)) ELX_GIVE_UP;
+    if (!grid::barrier<kMT, 1>(team, a.gs, ++barriers, sred)) ELX_GIVE_UP;
     if (S.done || !S.update || S.iters % replace_every) continue;
     // replacement (rel_accumulate, FP64 product, rel_residual): x_hi += x_lo,
     // r = b - K x_hi in FP64
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(kMT, 1) mixed_persist_kernel(MixedArgs a, int 
       a.xhi[row0 + i] += (double)sx[i];
       sx[i] = 0.0f;
     }
-    if (!grid::barrier<kMT, 1>(a.gs, ++barriers, sred)) ELX_GIVE_UP;
+    if (!grid::barrier<kMT, 1>(team, a.gs, ++barriers, sred)) ELX_GIVE_UP;
     double vd[1] = {0.0};
     for (int sl = w; sl < ns; sl += kMW) {
       double acc[B];
@@ -260,7 +261,7 @@ __global__ void __launch_bounds__(kMT, 1) mixed_persist_kernel(MixedArgs a, int 
           vd[0] += ri * (ri * a.m[row0 + i + b]);
         }
     }
-    if (!grid::sum<kMT, 1>(vd, a.gs, 1, sd, seen_rz, epoch + 2, sred,
+    if (!grid::sum<kMT, 1>(team, vd, a.gs, 1, sd, seen_rz, epoch + 2, sred,
                            [&](double t) {
                              const double rt = sqrt(fabs(t));
                              S.update = 0;

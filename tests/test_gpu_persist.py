@@ -142,3 +142,22 @@ def test_mixed_maxit_and_bad_load(gpu_ctx):
     assert i["status"] == E.ERR_NO_CONVERGENCE
     _, i = gpu_ctx.solve(b, precision=E.PREC_MIXED, tol=1e-10)
     assert i["status"] == 0
+
+
+# restart lengths around the 16 warps that share the basis vectors; k = 250
+# does not fit the block's shared memory and takes the launches
+@pytest.mark.parametrize("name,k", [("quad4 full slice", 1), ("quad4 two slices", 16),
+                                    ("tetra4", 33), ("tria3 153 slices", 17),
+                                    ("hexa8 rollers", 7), ("tetra4 rollers", 17),
+                                    ("quad4 152 slices", 250)])
+def test_gmres_cycle_matches_oracle(gpu_ctx, name, k):
+    s, ad, al, b = _system(gpu_ctx, CASES[name]())
+    k = min(k, s.neq)
+    x_o, _ = O.gmres(s, ad, al, b, k=k, tol=1e-14, maxit=1)
+    x, i = gpu_ctx.solve(b, solver=E.SOLVER_GMRES, tol=1e-14, maxit=1, ngram=k,
+                         raise_on_error=False)
+    assert i["refinements"] == 1 and i["iters"] <= k
+    assert rel_inf(x_o, x) <= 1e-9
+    x2, _ = gpu_ctx.solve(b, solver=E.SOLVER_GMRES, tol=1e-14, maxit=1, ngram=k,
+                          raise_on_error=False)
+    assert np.array_equal(x, x2)

@@ -36,8 +36,10 @@ constexpr int kGridCols = 6;
 // One column of it, between and after launches.
 struct PersistCol {
   double d, conv;
-  int32_t iters, done, status, pad;
+  int32_t iters, done, status, started;
 };
+// Cuts slices into one run per block with equal numbers of slot groups.
+std::vector<int32_t> persist_cuts(const std::vector<int32_t> &sell_ptr, int grid);
 
 // Progress watch of the mixed-precision solvers.  A matrix rounded to FP32
 // can lose definiteness when K is ill-conditioned (cond(K) near 1/eps32, as

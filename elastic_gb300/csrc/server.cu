@@ -13,11 +13,13 @@
 //     (matrix, preconditioner, Krylov vectors stay resident until it is
 //     done) and assembles it on the context's stream, overlapping the
 //     iterations of the others;
-//   * runs one PCG iteration of every active (request, load case) slot as
-//     three packed launches -- the SpMV with (p, q), the update with (r, M r)
-//     and the direction -- over all slots at once, each slot with its own
-//     scalars and its own stopping test (a converged slot's blocks return at
-//     once and the slot leaves the pack at the next poll);
+//   * runs the PCG iterations of every active (request, load case) slot in
+//     cooperative launches over all slots at once, a team of blocks for each
+//     slot with its own scalars and its own stopping test (a converged slot's
+//     blocks return at once and the slot leaves the pack at the next poll);
+//     slots too large for a team (above 122,880 rows, when large requests are
+//     packed too) as three packed launches an iteration -- the SpMV with
+//     (p, q), the update with (r, M r) and the direction;
 //   * lets new requests join the pack between polls (every few iterations),
 //     so that slots and memory freed by finished requests are reused at once.
 //
@@ -29,6 +31,7 @@
 #include <chrono>
 #include <cmath>
 #include <condition_variable>
+#include <cstddef>
 #include <cstdlib>
 #include <cstring>
 #include <deque>
@@ -40,6 +43,7 @@
 
 #include "elx_context.h"
 #include "elx_gate.h"
+#include "elx_persist.cuh"
 #include "elx_reduce.cuh"
 
 namespace elx {
@@ -61,7 +65,70 @@ struct SlotDesc {
   int32_t scta0, sncta;  // and in the packed product (8 slices per block)
 };
 
+// A load case in the cooperative pack: its solve and its blocks.
+struct PackSlot {
+  PersistArgs a;
+  int32_t cta0, ncta, bsize;
+  int32_t share;  // iterations of a launch, in 1/16 of its steps
+};
+
 namespace {
+
+// The pack as one cooperative launch: a team of kPackThreads-thread blocks for
+// each load case, `steps` PCG iterations of every one (elx_persist.cuh).
+// Teams wait only for their own blocks, so load cases of every size go on at
+// their own pace; three blocks share an SM, and one team's arithmetic runs in
+// another's waits.  A team has a block per kPackRows rows of its matrix,
+// whatever else is in the pack: a result is bitwise the same alone and in a
+// mix.  As three launches an iteration over all slots (48 us on a burst of 27
+// load cases, 20 us for the last of them alone) the pack waited for its
+// slowest slot three times an iteration: the burst took 153 ms, here 113
+// (blocks per SM x rows: 3 x 960 121, 2 x 960 123, 4 x 960 116, 4 x 576 117,
+// 3 x 576 126; 128 threads: 6 x 576 120, 8 x 384 151).
+constexpr int kPackThreads = 256;
+constexpr int kPackPerSm = 4;
+constexpr int kPackRows = 768;  // five vectors of it in shared memory: 37 KB a block
+
+__global__ void __launch_bounds__(kPackThreads, kPackPerSm)
+packed_pcg_kernel(const PackSlot *d, int nslots, int steps, uint64_t epoch) {
+  int lo = 0, hi = nslots - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (d[mid].cta0 <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+  }
+  const PackSlot &S = d[lo];
+  const grid::Team team{(int)blockIdx.x - S.cta0, S.ncta};
+  // every block reads the state before its first wait, and the team's first
+  // block writes it after the last
+  const int start = !S.a.cols[0].started;
+  const PersistArgs a = S.a;
+  if (S.bsize == 3)
+    persist_pcg<kPackThreads, 3, 1, true>(a, team, start, steps * S.share / 16, epoch);
+  else
+    persist_pcg<kPackThreads, 2, 1, true>(a, team, start, steps * S.share / 16, epoch);
+}
+
+int pack_slices(int bsize) { return kPackRows / (kSliceRows * bsize); }
+
+// A launch lasts as long as its slowest team, so a team takes iterations in
+// inverse proportion to what one costs: its DFMAs per row and 10 more for the
+// vectors, and 20 for the waits (HEXA8: 16/16, TETRA4 24/16, plane meshes up
+// to 36/16).  How many a launch takes does not change the iterates.
+int pack_share(const Structure &s) {
+  const double row = (double)s.sell_ptr[s.nslices] * kSliceRows * s.bsize / s.nb;
+  return (int)std::min(48.0, std::max(8.0, 16.0 * (81 + 30) / (row + 30)));
+}
+
+size_t pack_smem() {
+  return std::max(persist_smem<kPackThreads, 3, 1, true>(kPackRows, pack_slices(3)),
+                  persist_smem<kPackThreads, 2, 1, true>(kPackRows, pack_slices(2)));
+}
+
+// Blocks of a load case of the cooperative pack; 0: too many (packed launches).
+int pack_blocks(const Structure &s) {
+  const int S = pack_slices(s.bsize), n = (s.nslices + S - 1) / S;
+  return n <= kGridMaxBlocks ? n : 0;
+}
 
 constexpr int kRowsPerCta = kThreads;  // one row per thread
 
@@ -269,6 +336,8 @@ struct SrvRequest {
   // device state
   elx_ctx *ctx = nullptr;
   DBuf vecs;  // b (nrhs x neq), then per load case x, r, p, q
+  int blocks = 0;  // of each load case in the cooperative pack (0: packed launches)
+  DBuf cuts;       // its slices' cuts between them
   cudaEvent_t ready = nullptr;
   std::vector<int> slots;  // indices into the server's slot scalars
   // result
@@ -313,6 +382,14 @@ struct elx_server {
   std::vector<std::shared_ptr<SrvRequest>> active;
   void *d_desc = nullptr, *d_part = nullptr;
   size_t desc_bytes = 0, part_bytes = 0;
+  // the cooperative pack: slot states (the error word first), the grids'
+  // words, descriptors; blocks that fit the GPU at once
+  elx::PersistCol *d_col = nullptr, *h_col = nullptr;  // 1 + max_slots
+  elx::GridSync *d_sync = nullptr;
+  int sync_slots = 0;
+  elx::PackSlot *d_pack = nullptr, *h_pack = nullptr;  // max_slots
+  int pack_capacity = 0;
+  uint64_t epoch = 0;
   SlotScalars *d_sc = nullptr;   // max_slots
   SlotScalars *h_sc = nullptr;   // pinned copy
   SlotDesc *h_desc = nullptr;    // pinned, max_slots
@@ -471,6 +548,7 @@ void release_request(elx_server *sv, SrvRequest &q) {
   q.small_counted = false;
   if (q.ctx) {
     q.ctx->release(q.vecs);
+    q.ctx->release(q.cuts);
     elx_destroy(q.ctx);
     q.ctx = nullptr;
   }
@@ -534,16 +612,28 @@ void admit(elx_server *sv, SrvRequest &q) {
   c->alloc(q.vecs, 5 * n * q.nrhs * 8);
   ELX_CUDA(cudaMemcpyAsync(q.vecs.p, q.b0.data(), n * q.nrhs * 8, cudaMemcpyHostToDevice,
                            c->stream));
-  double *base = q.vecs.as<double>();
-  for (int k = 0; k < q.nrhs; k++) {
-    double *b = base + (size_t)k * n;
-    double *x = base + n * q.nrhs + (size_t)k * 4 * n;
-    elx::slot_start_kernel<<<elx::vector_grid((int)n), elx::kThreads, 0, c->stream>>>(
-        (int)n, b, c->m.as<double>(), x, x + n, x + 2 * n, sv->d_sc + q.slots[k], q.tol,
-        q.maxit, c->partials.as<double>(), c->counters.as<unsigned int>() + 7);
+  q.blocks = sv->pack_capacity > 0 ? elx::pack_blocks(c->s) : 0;
+  if (q.blocks > sv->pack_capacity) q.blocks = 0;
+  if (q.blocks > 0) {
+    const int nsl = c->s.nslices;
+    std::vector<int32_t> cuts(q.blocks + 1);
+    for (int k = 0; k <= q.blocks; k++) cuts[k] = (int32_t)((int64_t)nsl * k / q.blocks);
+    c->upload(q.cuts, cuts.data(), cuts.size());
+    for (int k = 0; k < q.nrhs; k++)
+      ELX_CUDA(cudaMemsetAsync(sv->d_col + 1 + q.slots[k], 0, sizeof(elx::PersistCol), c->stream));
+    c->sync();  // the cuts' host copy
+  } else {
+    double *base = q.vecs.as<double>();
+    for (int k = 0; k < q.nrhs; k++) {
+      double *b = base + (size_t)k * n;
+      double *x = base + n * q.nrhs + (size_t)k * 4 * n;
+      elx::slot_start_kernel<<<elx::vector_grid((int)n), elx::kThreads, 0, c->stream>>>(
+          (int)n, b, c->m.as<double>(), x, x + n, x + 2 * n, sv->d_sc + q.slots[k], q.tol,
+          q.maxit, c->partials.as<double>(), c->counters.as<unsigned int>() + 7);
+    }
+    ELX_CUDA(cudaGetLastError());
+    c->launches += q.nrhs;
   }
-  ELX_CUDA(cudaGetLastError());
-  c->launches += q.nrhs;
   ELX_CUDA(cudaEventCreateWithFlags(&q.ready, cudaEventDisableTiming));
   ELX_CUDA(cudaEventRecord(q.ready, c->stream));
   ELX_CUDA(cudaEventSynchronize(q.ready));  // this thread only; the pack runs on
@@ -575,7 +665,15 @@ void collect(elx_server *sv, SrvRequest &q) {
       const int e = c->s.id[j];
       q.u[k * nd + j] = e > 0 ? x[(size_t)k * n + e - 1] : 0.0;
     }
-    const SlotScalars &S = sv->h_sc[q.slots[k]];
+    SlotScalars S = sv->h_sc[q.slots[k]];
+    if (q.blocks > 0) {
+      const elx::PersistCol &o = sv->h_col[1 + q.slots[k]];
+      S.d = o.d;
+      S.conv = o.conv;
+      S.iters = o.iters;
+      S.done = o.done;
+      S.status = o.status;
+    }
     elx_info &in = q.infos[k];
     in.iters = S.iters;
     in.status = S.done ? S.status : ELX_ERR_NO_CONVERGENCE;
@@ -732,6 +830,12 @@ void gpu_loop(elx_server *sv) {
   try {
     ELX_CUDA(cudaSetDevice(sv->device));
     int nslots = 0, grid = 0, sgrid = 0;
+    // the cooperative pack's launches: (first slot, slots, blocks) of each
+    struct PackLaunch {
+      int first, n, blocks;
+    };
+    std::vector<PackLaunch> packs;
+    int npack = 0, ncol = 0;
     bool repack = false;
     for (;;) {
       // 1. admitted requests join the pack
@@ -752,8 +856,52 @@ void gpu_loop(elx_server *sv) {
         nslots = 0;
         grid = 0;
         sgrid = 0;
+        packs.clear();
+        npack = 0;
+        ncol = 0;
         for (auto &q : sv->active) {
           elx_ctx *c = q->ctx;
+          for (int k : q->slots) ncol = std::max(ncol, k + 1);
+          if (q->blocks > 0) {
+            const size_t n = (size_t)c->s.neq;
+            double *b = q->vecs.as<double>();
+            for (int k = 0; k < q->nrhs; k++) {
+              // a launch takes the teams that fit the GPU together
+              if (packs.empty() || packs.back().blocks + q->blocks > sv->pack_capacity)
+                packs.push_back({npack, 0, 0});
+              PackLaunch &L = packs.back();
+              elx::PackSlot &d = sv->h_pack[npack];
+              double *x = b + n * q->nrhs + (size_t)k * 4 * n;
+              elx::PersistArgs &a = d.a;
+              a.n = a.neq = (int)n;
+              a.sell_ptr = c->sell_ptr.as<int32_t>();
+              a.sell_col = c->sell_col.as<int32_t>();
+              a.sval = c->sell_val64.as<double>();
+              a.cta = q->cuts.as<int32_t>();
+              a.eq = nullptr;
+              a.m = c->m.as<double>();
+              a.b = b + (size_t)k * n;
+              a.x = x;
+              a.sx = x + 3 * n;
+              a.sr = x + n;
+              a.p = x + 2 * n;
+              a.cols = sv->d_col + 1 + q->slots[k];
+              a.gs = nullptr;  // below, once there is one for each slot
+              a.err = reinterpret_cast<int32_t *>(sv->d_col);
+              a.tol = q->tol;
+              a.maxit = q->maxit;
+              a.rows = elx::kPackRows;
+              a.slices = elx::pack_slices(c->s.bsize);
+              d.bsize = c->s.bsize;
+              d.cta0 = L.blocks;
+              d.ncta = q->blocks;
+              d.share = elx::pack_share(c->s);
+              L.blocks += q->blocks;
+              L.n++;
+              npack++;
+            }
+            continue;
+          }
           const size_t n = (size_t)c->s.neq;
           double *base = q->vecs.as<double>() + n * q->nrhs;
           const int per_cta = elx::kThreads / elx::kSliceRows;
@@ -779,7 +927,20 @@ void gpu_loop(elx_server *sv) {
             grid += d.ncta;
           }
         }
-        sv->peak_slots = std::max<int64_t>(sv->peak_slots.load(), nslots);
+        sv->peak_slots = std::max<int64_t>(sv->peak_slots.load(), nslots + npack);
+        if (npack > sv->sync_slots) {
+          if (sv->d_sync) cudaFree(sv->d_sync);
+          sv->d_sync = nullptr;
+          sv->sync_slots = 0;
+          const int want = std::min(sv->max_slots, std::max(64, 2 * npack));
+          ELX_CUDA(cudaMalloc(&sv->d_sync, sizeof(elx::GridSync) * want));
+          ELX_CUDA(cudaMemsetAsync(sv->d_sync, 0, sizeof(elx::GridSync) * want, sv->stream));
+          sv->sync_slots = want;
+        }
+        for (int k = 0; k < npack; k++) sv->h_pack[k].a.gs = sv->d_sync + k;
+        if (npack)
+          ELX_CUDA(cudaMemcpyAsync(sv->d_pack, sv->h_pack, npack * sizeof(elx::PackSlot),
+                                   cudaMemcpyHostToDevice, sv->stream));
         const int pgrid = std::max(grid, sgrid);
         if ((size_t)pgrid * 8 > sv->part_bytes) {
           if (sv->d_part) cudaFree(sv->d_part);
@@ -788,29 +949,55 @@ void gpu_loop(elx_server *sv) {
           ELX_CUDA(cudaMalloc(&sv->d_part, (size_t)pgrid * 8 * 2));
           sv->part_bytes = (size_t)pgrid * 8 * 2;
         }
-        ELX_CUDA(cudaMemcpyAsync(sv->d_desc, sv->h_desc, nslots * sizeof(SlotDesc),
-                                 cudaMemcpyHostToDevice, sv->stream));
+        if (nslots)
+          ELX_CUDA(cudaMemcpyAsync(sv->d_desc, sv->h_desc, nslots * sizeof(SlotDesc),
+                                   cudaMemcpyHostToDevice, sv->stream));
         repack = false;
       }
-      // 3. poll_steps packed PCG iterations of every active load case
+      // 3. PCG iterations of every active load case, then the poll: poll_steps
+      // of packed launches, four times as many in cooperative ones (a team's
+      // vectors come from and go to L2 once a launch)
+      const int steps = npack ? 4 * sv->poll_steps : sv->poll_steps;
+      if (npack) {
+        // the words (not the slots) of each team's sums
+        ELX_CUDA(cudaMemset2DAsync(sv->d_sync, sizeof(elx::GridSync), 0,
+                                   offsetof(elx::GridSync, slot), npack, sv->stream));
+        for (const PackLaunch &L : packs) {
+          const elx::PackSlot *d = sv->d_pack + L.first;
+          int n = L.n, st = steps;
+          uint64_t ep = sv->epoch;
+          void *args[] = {&d, &n, &st, &ep};
+          ELX_CUDA(cudaLaunchCooperativeKernel((const void *)elx::packed_pcg_kernel,
+                                               dim3(L.blocks), dim3(elx::kPackThreads), args,
+                                               elx::pack_smem(), sv->stream));
+        }
+        sv->epoch += 2 * 3 * (uint64_t)steps + 2;  // shares are at most 48/16
+      }
       const SlotDesc *dd = static_cast<const SlotDesc *>(sv->d_desc);
       double *part = static_cast<double *>(sv->d_part);
-      for (int it = 0; it < sv->poll_steps; it++) {
+      for (int it = 0; it < steps && nslots; it++) {
         elx::packed_spmv_kernel<<<sgrid, elx::kThreads, 0, sv->stream>>>(dd, nslots, part);
         elx::packed_update_kernel<<<grid, elx::kThreads, 0, sv->stream>>>(dd, nslots, part);
         elx::packed_direction_kernel<<<grid, elx::kThreads, 0, sv->stream>>>(dd, nslots);
       }
       ELX_CUDA(cudaGetLastError());
-      sv->iterations += sv->poll_steps;
-      ELX_CUDA(cudaMemcpyAsync(sv->h_sc, sv->d_sc, sizeof(SlotScalars) * sv->max_slots,
-                               cudaMemcpyDeviceToHost, sv->stream));
+      sv->iterations += steps;
+      if (npack)
+        ELX_CUDA(cudaMemcpyAsync(sv->h_col, sv->d_col, sizeof(elx::PersistCol) * (1 + ncol),
+                                 cudaMemcpyDeviceToHost, sv->stream));
+      if (nslots)
+        ELX_CUDA(cudaMemcpyAsync(sv->h_sc, sv->d_sc, sizeof(SlotScalars) * ncol,
+                                 cudaMemcpyDeviceToHost, sv->stream));
       ELX_CUDA(cudaEventRecord(sv->ev_poll, sv->stream));
       ELX_CUDA(cudaEventSynchronize(sv->ev_poll));
+      if (npack && *reinterpret_cast<const int32_t *>(sv->h_col) != 0)
+        throw Error{ELX_ERR_TIMEOUT, "a bounded device wait of the pack gave up"};
       // 4. retire the requests whose load cases have all stopped
       for (size_t i = 0; i < sv->active.size();) {
         auto q = sv->active[i];
         bool all = true;
-        for (int k : q->slots) all = all && sv->h_sc[k].done;
+        for (int k : q->slots)
+          all = all && (q->blocks > 0 ? sv->h_col[1 + k].done : sv->h_sc[k].done);
         if (!all) {
           i++;
           continue;
@@ -880,6 +1067,23 @@ int elx_server_create(elx_server **out, const elx_server_opts *opts) {
     e = cudaHostAlloc(&sv->h_sc, sizeof(SlotScalars) * sv->max_slots, cudaHostAllocDefault);
   if (e == cudaSuccess)
     e = cudaHostAlloc(&sv->h_desc, sizeof(SlotDesc) * sv->max_slots, cudaHostAllocDefault);
+  const size_t col_bytes = sizeof(elx::PersistCol) * (1 + (size_t)sv->max_slots);
+  if (e == cudaSuccess) e = cudaMalloc(&sv->d_col, col_bytes);
+  if (e == cudaSuccess) e = cudaMemset(sv->d_col, 0, col_bytes);
+  if (e == cudaSuccess) e = cudaMalloc(&sv->d_pack, sizeof(elx::PackSlot) * sv->max_slots);
+  if (e == cudaSuccess) e = cudaHostAlloc(&sv->h_col, col_bytes, cudaHostAllocDefault);
+  if (e == cudaSuccess)
+    e = cudaHostAlloc(&sv->h_pack, sizeof(elx::PackSlot) * sv->max_slots, cudaHostAllocDefault);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(elx::packed_pcg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)elx::pack_smem());
+  int per_sm = 0, sms = 0;
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, elx::packed_pcg_kernel,
+                                                      elx::kPackThreads, elx::pack_smem());
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, sv->device);
+  sv->pack_capacity = per_sm * sms;
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sv->ev_poll, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
@@ -927,6 +1131,11 @@ void elx_server_destroy(elx_server *sv) {
   if (sv->d_sc) cudaFree(sv->d_sc);
   if (sv->d_desc) cudaFree(sv->d_desc);
   if (sv->d_part) cudaFree(sv->d_part);
+  if (sv->d_col) cudaFree(sv->d_col);
+  if (sv->d_sync) cudaFree(sv->d_sync);
+  if (sv->d_pack) cudaFree(sv->d_pack);
+  if (sv->h_col) cudaFreeHost(sv->h_col);
+  if (sv->h_pack) cudaFreeHost(sv->h_pack);
   if (sv->h_sc) cudaFreeHost(sv->h_sc);
   if (sv->h_desc) cudaFreeHost(sv->h_desc);
   if (sv->ev_poll) cudaEventDestroy(sv->ev_poll);

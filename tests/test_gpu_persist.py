@@ -161,3 +161,29 @@ def test_gmres_cycle_matches_oracle(gpu_ctx, name, k):
     x2, _ = gpu_ctx.solve(b, solver=E.SOLVER_GMRES, tol=1e-14, maxit=1, ngram=k,
                           raise_on_error=False)
     assert np.array_equal(x, x2)
+
+
+def test_pack_with_teams_and_packed_launches(built_lib):
+    """A load case too large for a team of the cooperative pack (above 160
+    blocks of 768 rows) iterates in packed launches beside teams of one block
+    and of several; each equals its own single solve."""
+    meshes = [M.box2d(255, 250, etype=M.QUAD4_STRESS), M.box_hexa8(2, 2, 2),
+              M.box_tetra4(9, 9, 9), M.box2d(40, 20, etype=M.TRIA3_STRAIN)]
+    with E.Server(device=0, large_mode=-1) as srv, E.Context(device=0) as ctx:
+        tickets = []
+        for k, m in enumerate(meshes):
+            F = np.random.default_rng(k).standard_normal((2,) + m.f.shape) * (m.id == 0)
+            tickets.append((m, F, srv.submit(m, F, tol=1e-10, maxit=50000)))
+        for m, F, t in tickets:
+            U, infos, _, status = srv.wait(t, timeout=300)
+            assert status == 0
+            ctx.set_mesh(m)
+            ctx.build_structure(True)
+            st = ctx.structure()
+            ctx.assemble(None, None)
+            for k in range(2):
+                m.f = F[k]
+                b, u0 = E.pload(m, st.id)
+                x, i = ctx.solve(b, tol=1e-10, maxit=50000)
+                assert abs(infos[k]["iters"] - i["iters"]) <= max(2, 0.01 * i["iters"])
+                assert rel_inf(ctx.update(x, u0), U[k]) <= 1e-8

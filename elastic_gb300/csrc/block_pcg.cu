@@ -43,10 +43,20 @@ __device__ __forceinline__ double gather_columns(const double *partials, int nbl
   constexpr int S = kThreads / NC;
   __shared__ double sh[kThreads];
   const int c = threadIdx.x % NC, sl = threadIdx.x / NC;
-  double t = 0.0;
-#pragma unroll 4
-  for (int b = sl; b < nblocks; b += S) t += __ldcg(partials + (size_t)c * nblocks + b);
-  sh[threadIdx.x] = t;
+  // eight loads in flight, four chains of adds (76 adds a thread of 1216 blocks'
+  // partials: a chain of FP64 adds is 64 clocks each)
+  double t0 = 0.0, t1 = 0.0, t2 = 0.0, t3 = 0.0;
+  const double *pc = partials + (size_t)c * nblocks;
+  int b = sl;
+#pragma unroll 2
+  for (; b + 3 * S < nblocks; b += 4 * S) {
+    t0 += __ldcg(pc + b);
+    t1 += __ldcg(pc + b + S);
+    t2 += __ldcg(pc + b + 2 * S);
+    t3 += __ldcg(pc + b + 3 * S);
+  }
+  for (; b < nblocks; b += S) t0 += __ldcg(pc + b);
+  sh[threadIdx.x] = (t0 + t1) + (t2 + t3);
   __syncthreads();
   double u = 0.0;
   if (threadIdx.x < NC)
@@ -207,6 +217,48 @@ __device__ __forceinline__ bool column_reduce_v(double (&v)[VC], double *partial
   return true;
 }
 
+// The same for FP32 values, in integers (FixSum): the FP64 shuffle trees of
+// eight blocks per SM held its FP64 pipe for 8 of the update's 50 us.  Warp w
+// adds columns w, w + 8, ... of the block's values from shared memory.
+template <int W, int VC>
+__device__ __forceinline__ bool column_reduce_v(const float (&v)[VC], double *partials,
+                                                unsigned int *counter, double &out) {
+  constexpr int G = W / VC, N = kThreads / G, K = N / 32;  // values of a column, per lane
+  __shared__ float sv[VC][kThreads];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int j = 0; j < VC; j++) sv[j][threadIdx.x] = v[j];
+  __syncthreads();
+  for (int c = warp; c < W; c += kThreads / 32) {
+    FixSum f[K];
+    int e = -4096;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      f[k] = fix_of(sv[c % VC][c / VC + G * (lane + 32 * k)]);
+      e = max(e, f[k].e);
+    }
+    FixSum t;
+    t.m = 0;
+#pragma unroll
+    for (int k = 0; k < K; k++) t.m += fix_align(f[k], e, 3);
+    t.e = e >= kFixBad ? e : e + 3;
+    const double s = fix_value(warp_sum(t));
+    if (lane == 0) {
+      partials[(size_t)c * gridDim.x + blockIdx.x] = s;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  out = gather_columns<W>(partials, gridDim.x);
+  if (threadIdx.x == 0) *counter = 0u;
+  return true;
+}
+
 // Y = K X for W columns on a sliced copy of the node blocks.  A group of
 // G = W / VC lanes works on one block row, each lane on VC consecutive
 // columns (one 16-byte x load per row of a block); G warps take one slice
@@ -305,11 +357,8 @@ sell_spmm_kernel(int nb, int nslices, const int32_t *__restrict__ sell_ptr,
     }
   }
   if constexpr (DOT) {
-    double vd[VC];
-#pragma unroll
-    for (int j = 0; j < VC; j++) vd[j] = (double)v[j];
     double tot;
-    if (!column_reduce_v<W, VC>(vd, partials, counter, tot)) return;
+    if (!column_reduce_v<W, VC>(v, partials, counter, tot)) return;
     if (threadIdx.x < W) {
       ColScalars &s = cols[threadIdx.x];
       if (!s.done) {
@@ -469,13 +518,15 @@ brel_start_kernel(int n, const double *__restrict__ b, const double *__restrict_
   }
 }
 
-// FP32 step: x_lo += alpha p, r -= alpha q, d' = (r, M r); beta; flag a
-// replacement when ||r||_M < delta rmax, < conv, or at maxit.  Each thread
-// takes VC consecutive columns of a row (16-byte accesses).
+// FP32 step: r -= alpha q, d' = (r, M r); beta; flag a replacement when
+// ||r||_M < delta rmax, < conv, or at maxit.  x_lo += alpha p waits for the
+// direction pass, which reads p anyway: 8 passes over the multi-vectors in an
+// iteration instead of 9 (87 MB each at 1,354,896 equations x 16).  Each
+// thread takes VC consecutive columns of a row (16-byte accesses), two rows in
+// flight.
 template <int W>
 __global__ void __launch_bounds__(kThreads)
-brel_update_kernel(int n, const float *__restrict__ p, const float *__restrict__ qv,
-                   const float *__restrict__ m32, float *__restrict__ xlo,
+brel_update_kernel(int n, const float *__restrict__ qv, const float *__restrict__ m32,
                    float *__restrict__ r, ColScalars *cols, BlockHeader *hdr,
                    double *partials, unsigned int *counter) {
   constexpr int VC = W < 4 ? W : 4;
@@ -493,28 +544,36 @@ brel_update_kernel(int n, const float *__restrict__ p, const float *__restrict__
   bool any = false;
 #pragma unroll
   for (int j = 0; j < VC; j++) any = any || on[j];
-  const size_t ng = (size_t)n * G;
-  if (any)
-    for (size_t t = (size_t)blockIdx.x * kThreads + threadIdx.x; t < ng;
-         t += (size_t)gridDim.x * kThreads) {
-      const size_t row = t / G, q = row * W + c0;
-      const float mi = m32[row];
-      ColVec<float, VC> pv = load_cols<float, VC>(p + q), qq = load_cols<float, VC>(qv + q);
-      ColVec<float, VC> xv = load_cols<float, VC>(xlo + q), rv = load_cols<float, VC>(r + q);
+  const size_t ng = (size_t)n * G, step = (size_t)gridDim.x * kThreads;
+  auto one = [&](size_t row, ColVec<float, VC> &rv, const ColVec<float, VC> &qq, float mi) {
 #pragma unroll
-      for (int j = 0; j < VC; j++) {
-        xv.v[j] += alpha[j] * pv.v[j];
-        rv.v[j] -= alpha[j] * qq.v[j];
-        v[j] += rv.v[j] * (rv.v[j] * mi);
-      }
-      store_cols<float, VC>(xlo + q, xv);
-      store_cols<float, VC>(r + q, rv);
+    for (int j = 0; j < VC; j++) {
+      rv.v[j] -= alpha[j] * qq.v[j];
+      v[j] += rv.v[j] * (rv.v[j] * mi);
     }
-  double vd[VC];
-#pragma unroll
-  for (int j = 0; j < VC; j++) vd[j] = (double)v[j];
+    store_cols<float, VC>(r + row * W + c0, rv);
+  };
+  if (any) {
+    size_t t = (size_t)blockIdx.x * kThreads + threadIdx.x;
+    for (; t + step < ng; t += 2 * step) {
+      const size_t row0 = t / G, row1 = (t + step) / G;
+      const ColVec<float, VC> q0 = load_cols<float, VC>(qv + row0 * W + c0);
+      const ColVec<float, VC> q1 = load_cols<float, VC>(qv + row1 * W + c0);
+      ColVec<float, VC> r0 = load_cols<float, VC>(r + row0 * W + c0);
+      ColVec<float, VC> r1 = load_cols<float, VC>(r + row1 * W + c0);
+      const float m0 = m32[row0], m1 = m32[row1];
+      one(row0, r0, q0, m0);
+      one(row1, r1, q1, m1);
+    }
+    if (t < ng) {
+      const size_t row = t / G;
+      const ColVec<float, VC> q0 = load_cols<float, VC>(qv + row * W + c0);
+      ColVec<float, VC> r0 = load_cols<float, VC>(r + row * W + c0);
+      one(row, r0, q0, m32[row]);
+    }
+  }
   double tot;
-  if (!column_reduce_v<W, VC>(vd, partials, counter, tot)) return;
+  if (!column_reduce_v<W, VC>(v, partials, counter, tot)) return;
   if (threadIdx.x < W) {
     ColScalars &s = cols[threadIdx.x];
     if (!s.done) {
@@ -528,7 +587,12 @@ brel_update_kernel(int n, const float *__restrict__ p, const float *__restrict__
         const double rn = sqrt(fabs(tot));
         s.beta = s.d != 0.0 ? tot / s.d : 0.0;
         s.d = tot;
-        if (rn < hdr->delta * s.rmax || rn < s.conv || s.iters >= hdr->maxit ||
+        // a column that looks converged waits for the others to, or for the
+        // next replacement: its FP64 product is a full-width one, and the 16
+        // columns of the 96x96x48 plate end within 28 iterations of each other
+        // (8 products of 2.9 ms)
+        if (rn < s.conv) s.update = 1;
+        if (rn < hdr->delta * s.rmax || s.iters >= hdr->maxit ||
             s.iters - s.last_rep >= kMixedCheckEvery || rn > kMixedDiverge * s.rmax) {
           s.update = 1;
           hdr->any_update = 1;
@@ -538,9 +602,68 @@ brel_update_kernel(int n, const float *__restrict__ p, const float *__restrict__
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    int act = 0;
-    for (int k = 0; k < W; k++) act += cols[k].done ? 0 : 1;
+    int act = 0, due = 0;
+    for (int k = 0; k < W; k++) {
+      act += cols[k].done ? 0 : 1;
+      due += !cols[k].done && cols[k].update ? 1 : 0;
+    }
     hdr->active = act;
+    if (due == act) hdr->any_update = 1;
+  }
+}
+
+// p = M r + beta p and x_lo += alpha p (the old p) for the active columns.
+template <int W>
+__global__ void __launch_bounds__(kThreads)
+brel_direction_kernel(int n, const float *__restrict__ r, const float *__restrict__ m32,
+                      float *__restrict__ p, float *__restrict__ xlo, const ColScalars *cols,
+                      const BlockHeader *hdr) {
+  constexpr int VC = W < 4 ? W : 4;
+  constexpr int G = W / VC;
+  if (hdr->active == 0) return;
+  const int c0 = (threadIdx.x % G) * VC;
+  bool on[VC], any = false, all = true;
+  float alpha[VC], beta[VC];
+#pragma unroll
+  for (int j = 0; j < VC; j++) {
+    on[j] = !cols[c0 + j].done;
+    alpha[j] = (float)cols[c0 + j].alpha;
+    beta[j] = (float)cols[c0 + j].beta;
+    any = any || on[j];
+    all = all && on[j];
+  }
+  if (!any) return;
+  const size_t ng = (size_t)n * G, step = (size_t)gridDim.x * kThreads;
+  auto one = [&](size_t row, ColVec<float, VC> &pv, ColVec<float, VC> &xv,
+                 const ColVec<float, VC> &rv, float mi) {
+#pragma unroll
+    for (int j = 0; j < VC; j++)
+      if (all || on[j]) {
+        xv.v[j] += alpha[j] * pv.v[j];
+        pv.v[j] = rv.v[j] * mi + beta[j] * pv.v[j];
+      }
+    store_cols<float, VC>(p + row * W + c0, pv);
+    store_cols<float, VC>(xlo + row * W + c0, xv);
+  };
+  size_t t = (size_t)blockIdx.x * kThreads + threadIdx.x;
+  for (; t + step < ng; t += 2 * step) {
+    const size_t row0 = t / G, row1 = (t + step) / G;
+    ColVec<float, VC> p0 = load_cols<float, VC>(p + row0 * W + c0);
+    ColVec<float, VC> p1 = load_cols<float, VC>(p + row1 * W + c0);
+    const ColVec<float, VC> r0 = load_cols<float, VC>(r + row0 * W + c0);
+    const ColVec<float, VC> r1 = load_cols<float, VC>(r + row1 * W + c0);
+    ColVec<float, VC> x0 = load_cols<float, VC>(xlo + row0 * W + c0);
+    ColVec<float, VC> x1 = load_cols<float, VC>(xlo + row1 * W + c0);
+    const float m0 = m32[row0], m1 = m32[row1];
+    one(row0, p0, x0, r0, m0);
+    one(row1, p1, x1, r1, m1);
+  }
+  if (t < ng) {
+    const size_t row = t / G;
+    ColVec<float, VC> p0 = load_cols<float, VC>(p + row * W + c0);
+    const ColVec<float, VC> r0 = load_cols<float, VC>(r + row * W + c0);
+    ColVec<float, VC> x0 = load_cols<float, VC>(xlo + row * W + c0);
+    one(row, p0, x0, r0, m32[row]);
   }
 }
 
@@ -779,10 +902,10 @@ void iteration_w(const CsrcDev &k, const BlockVecs &v, bool mixed, bool replacem
   } else {
     spmm_w<float, W>(k, v.p32, v.q32, v.cols, v.hdr, v.partials, cnt + 0, nullptr, true,
                      st);
-    brel_update_kernel<W><<<g, kThreads, 0, st>>>(n, v.p32, v.q32, v.m32, v.xlo, v.r32, v.cols,
-                                                  v.hdr, v.partials, cnt + 1);
-    bpcg_direction_kernel<float, W><<<g, kThreads, 0, st>>>(n, v.r32, v.m32, v.p32, v.cols,
-                                                            v.hdr);
+    brel_update_kernel<W><<<g, kThreads, 0, st>>>(n, v.q32, v.m32, v.r32, v.cols, v.hdr,
+                                                  v.partials, cnt + 1);
+    brel_direction_kernel<W><<<g, kThreads, 0, st>>>(n, v.r32, v.m32, v.p32, v.xlo, v.cols,
+                                                     v.hdr);
     if (replacement_point) {
       brel_accumulate_kernel<W><<<g, kThreads, 0, st>>>(n, v.x, v.xlo, v.cols, v.hdr);
       spmm_w<double, W>(k, v.x, v.z, v.cols, v.hdr, v.partials, cnt + 2,

@@ -28,6 +28,7 @@
 // well below 1e-13 relative.
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 
 #include "elx_internal.h"
 
@@ -474,19 +475,33 @@ hexa8_kernel(MeshDev m, CsrcDev k, int begin, int end, const double *__restrict_
 #undef SG
 }
 
-// HEXA8 with a team of 8 threads per element.  One thread per element
+// HEXA8 with a team of 4 threads per element.  One thread per element
 // (hexa8_kernel, ELX_HEX_TEAM=0) left each colour's launch with 32,768 long
-// serial threads on the 64^3 cube: 8.45 ms per assembly, latency bound.
-// Here thread g of a team first forms integration point g (Jacobian, one
-// reciprocal of its determinant, the 8 nodes' gradients and weighted
-// gradients into shared memory; the natural derivatives come from a table)
-// and stages node g's equations and displacements, then the team splits the
-// 36 node pairs (lane i: pairs i, i+8, ...), each pair's block formed as in
-// hexa8_kernel; the element vector K u is summed over the team by a fixed
-// shuffle tree and lane g subtracts node g's part from b.  5.30 ms per
-// assembly, the FP64 pipe 77 % busy (FP64-bound: ~7,000 FP64 operations per
-// element).
-constexpr int kTeamElems = 8;  // elements per 64-thread block
+// serial threads on the 64^3 cube: 8.45 ms per assembly, latency bound.  The
+// FP64 pipe bounds a team (an instruction of a warp costs the same however few
+// of its lanes work), so its lanes are filled and its operations counted:
+//
+//   * Each lane forms two of the 8 integration points.  With G = a c the shear
+//     modulus and s = b / c, the block of nodes (i, j) at a point is
+//       G det (s g_i g_j^T + g_j g_i^T + (g_i . g_j) I),
+//     so one array of gradients scaled by sqrt(G det) serves both sides: the
+//     adjugate of the Jacobian times sqrt(G / det), one root and one quotient
+//     a point.
+//   * The 36 node pairs are nine a lane with no lane idle: lane l takes nodes
+//     a = 2l and 2l + 1 with b = a .. a + 3 (mod 8), and the pair (l, l + 4).
+//     A block is 72 FMAs (48 on the diagonal) and 11 more operations.
+//   * K u needs no sums over the team at the end: for a given step the part of
+//     node b belongs to the same neighbour lane in every team, which gets it
+//     by a shuffle.
+//   * The entries a pair adds to are loaded before its FMAs and stored after
+//     them (a read-modify-write at a time waits for L2 nine times a pair).
+//
+// 64^3 elements: 2.49 ms with u = 0 (8 threads per element, blocks in pair order
+// with a read-modify-write at a time and a shuffle tree for K u: 3.76), 61 x 66 x
+// 58 with K u 2.65 (4.20).
+constexpr int kTeamThreads = 64;
+constexpr int kTeamElems = kTeamThreads / 4;
+constexpr int kTeamStride = 8 * 8 * 3 + 5;  // doubles of an element, odd: spreads the banks
 
 // Natural derivatives (d/dr, d/ds, d/dt) of the 8 shape functions at the 8
 // points (sfhexa8_m, Elmlib.f:1151-1258; point g = lx + 2 ly + 4 lz), the
@@ -494,175 +509,235 @@ constexpr int kTeamElems = 8;  // elements per 64-thread block
 // expressions (exact: the node signs are +-1 and 0.125 a power of two).
 __device__ __constant__ double kHexDh[8][3][8];
 
-__device__ __constant__ unsigned char kPairA[36] = {0, 1, 1, 2, 2, 2, 3, 3, 3, 3, 4, 4,
-                                                    4, 4, 4, 5, 5, 5, 5, 5, 5, 6, 6, 6,
-                                                    6, 6, 6, 6, 7, 7, 7, 7, 7, 7, 7, 7};
-__device__ __constant__ unsigned char kPairB[36] = {0, 0, 1, 0, 1, 2, 0, 1, 2, 3, 0, 1,
-                                                    2, 3, 4, 0, 1, 2, 3, 4, 5, 0, 1, 2,
-                                                    3, 4, 5, 6, 0, 1, 2, 3, 4, 5, 6, 7};
-
-__global__ void __launch_bounds__(64)
+__global__ void __launch_bounds__(kTeamThreads, 6)
 hexa8_team_kernel(MeshDev m, CsrcDev k, int begin, int end, const double *__restrict__ u,
                   double *__restrict__ b, int32_t *bad) {
-  __shared__ double sg[kTeamElems][8][8][3];   // [element][point][node][d]: gradients
-  __shared__ double swg[kTeamElems][8][8][3];  // the same times the point's weight
+  __shared__ double sg[kTeamElems * kTeamStride];  // [element][point][node][d], scaled
+  __shared__ double sdh[8 * 24];
   __shared__ double su[kTeamElems][8][3];
   __shared__ int seq[kTeamElems][8][3];
   __shared__ int sfirst[kTeamElems][8];
-  const int le = threadIdx.x >> 3, lane = threadIdx.x & 7;
+  const int le = threadIdx.x >> 2, lane = threadIdx.x & 3;
   const int t = begin + blockIdx.x * kTeamElems + le;
   const bool active = t < end;
   const int te = active ? t : begin;  // inactive teams read a valid element, write nothing
-  int node[8];
-#pragma unroll
-  for (int a = 0; a < 8; a++) node[a] = m.conn[(size_t)a * m.numel + te];
-  const Law L = make_law(HEXA8, m.e + (size_t)m.mat[te] * m.prop);
+  for (int i = threadIdx.x; i < 8 * 24; i += kTeamThreads) sdh[i] = (&kHexDh[0][0][0])[i];
+  double *ge = sg + le * kTeamStride;
+  // a c and b / c of Elmlib02.f:1697-1705
+  const double *em = m.e + (size_t)m.mat[te] * m.prop;
+  const double G = 0.5 * em[0] / (1.0 + em[1]), sig = 2.0 * em[1] / (1.0 - 2.0 * em[1]);
+  const bool neg = G < 0.0;
+  __syncthreads();
   {
-    // integration point `lane`
-    double hr[8], hs[8], ht[8];
+    double xl[8][3];
 #pragma unroll
     for (int a = 0; a < 8; a++) {
-      hr[a] = kHexDh[lane][0][a];
-      hs[a] = kHexDh[lane][1][a];
-      ht[a] = kHexDh[lane][2][a];
+      const int no = m.conn[(size_t)a * m.numel + te];
+#pragma unroll
+      for (int d = 0; d < 3; d++) xl[a][d] = m.x[(size_t)no * 3 + d];
     }
-    double xj[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+#pragma unroll 1
+    for (int half = 0; half < 2; half++) {
+      const int gp = lane + 4 * half;
+      const double *h = sdh + gp * 24;
+      double xj[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
 #pragma unroll
-    for (int a = 0; a < 8; a++)
+      for (int a = 0; a < 8; a++)
 #pragma unroll
-      for (int d = 0; d < 3; d++) {
-        const double xa = m.x[(size_t)node[a] * 3 + d];
-        xj[0][d] += hr[a] * xa;
-        xj[1][d] += hs[a] * xa;
-        xj[2][d] += ht[a] * xa;
-      }
-    const double det = xj[0][0] * xj[1][1] * xj[2][2] + xj[0][1] * xj[1][2] * xj[2][0] +
-                       xj[0][2] * xj[1][0] * xj[2][1] - xj[2][0] * xj[1][1] * xj[0][2] -
-                       xj[1][0] * xj[0][1] * xj[2][2] - xj[0][0] * xj[2][1] * xj[1][2];
-    if (active && det <= 1.e-14) mark_bad(bad, m.elnum[t]);
-    // the inverse Jacobian through one reciprocal of det (one FP64 division
-    // instead of nine; the FP64 pipe bounds this kernel)
-    const double rd = 1.0 / det;
-    double ji[3][3];
-    ji[0][0] = (xj[1][1] * xj[2][2] - xj[1][2] * xj[2][1]) * rd;
-    ji[1][0] = -(xj[1][0] * xj[2][2] - xj[1][2] * xj[2][0]) * rd;
-    ji[2][0] = (xj[1][0] * xj[2][1] - xj[1][1] * xj[2][0]) * rd;
-    ji[0][1] = -(xj[0][1] * xj[2][2] - xj[0][2] * xj[2][1]) * rd;
-    ji[1][1] = (xj[0][0] * xj[2][2] - xj[0][2] * xj[2][0]) * rd;
-    ji[2][1] = -(xj[0][0] * xj[2][1] - xj[0][1] * xj[2][0]) * rd;
-    ji[0][2] = (xj[0][1] * xj[1][2] - xj[0][2] * xj[1][1]) * rd;
-    ji[1][2] = -(xj[0][0] * xj[1][2] - xj[0][2] * xj[1][0]) * rd;
-    ji[2][2] = (xj[0][0] * xj[1][1] - xj[0][1] * xj[1][0]) * rd;
-    const double w = det * L.a;  // wg^3 = 1
+        for (int r = 0; r < 3; r++)
 #pragma unroll
-    for (int a = 0; a < 8; a++)
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        const double g = ji[d][0] * hr[a] + ji[d][1] * hs[a] + ji[d][2] * ht[a];
-        sg[le][lane][a][d] = g;
-        swg[le][lane][a][d] = w * g;
-      }
-    // node `lane`: its equations, the smallest of them, its displacements
-    int f = -1;
-#pragma unroll
-    for (int d = 2; d >= 0; d--) {
-      const int q = m.eq[(size_t)node[lane] * 3 + d];
-      seq[le][lane][d] = q;
-      if (q >= 0) f = q;
-      su[le][lane][d] = u ? u[(size_t)node[lane] * 3 + d] : 0.0;
-    }
-    sfirst[le][lane] = f;
-  }
-  __syncthreads();
-  // K u only where the element has a non-zero displacement (an element with
-  // u = 0 adds nothing to b; the first solvm pass has u = 0 away from
-  // prescribed values): decided per team, from its 8 lanes' nodes
-  const unsigned team_mask = 0xffu << (threadIdx.x & 24);
-  const bool nz = su[le][lane][0] != 0.0 || su[le][lane][1] != 0.0 || su[le][lane][2] != 0.0;
-  const bool with_u = u != nullptr && (__ballot_sync(0xffffffffu, nz) & team_mask) != 0u;
-  double p[8][3];
-#pragma unroll
-  for (int a = 0; a < 8; a++)
-#pragma unroll
-    for (int d = 0; d < 3; d++) p[a][d] = 0.0;
-  for (int q = lane; q < 36; q += 8) {
-    const int a = kPairA[q], bb = kPairB[q];
-    double M[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, K[3][3];
-#pragma unroll
-    for (int gp = 0; gp < 8; gp++) {
-      const double s0 = swg[le][gp][a][0], s1 = swg[le][gp][a][1], s2 = swg[le][gp][a][2];
-      const double g0 = sg[le][gp][bb][0], g1 = sg[le][gp][bb][1], g2 = sg[le][gp][bb][2];
-      M[0][0] += s0 * g0; M[0][1] += s0 * g1; M[0][2] += s0 * g2;
-      M[1][0] += s1 * g0; M[1][1] += s1 * g1; M[1][2] += s1 * g2;
-      M[2][0] += s2 * g0; M[2][1] += s2 * g1; M[2][2] += s2 * g2;
-    }
-    block3d(L, M, K);
-    if (with_u) {
+          for (int d = 0; d < 3; d++) xj[r][d] += h[r * 8 + a] * xl[a][d];
+      double ad[3][3];  // adjugate
+      ad[0][0] = xj[1][1] * xj[2][2] - xj[1][2] * xj[2][1];
+      ad[1][0] = -(xj[1][0] * xj[2][2] - xj[1][2] * xj[2][0]);
+      ad[2][0] = xj[1][0] * xj[2][1] - xj[1][1] * xj[2][0];
+      ad[0][1] = -(xj[0][1] * xj[2][2] - xj[0][2] * xj[2][1]);
+      ad[1][1] = xj[0][0] * xj[2][2] - xj[0][2] * xj[2][0];
+      ad[2][1] = -(xj[0][0] * xj[2][1] - xj[0][1] * xj[2][0]);
+      ad[0][2] = xj[0][1] * xj[1][2] - xj[0][2] * xj[1][1];
+      ad[1][2] = -(xj[0][0] * xj[1][2] - xj[0][2] * xj[1][0]);
+      ad[2][2] = xj[0][0] * xj[1][1] - xj[0][1] * xj[1][0];
+      const double det = xj[0][0] * xj[1][1] * xj[2][2] + xj[0][1] * xj[1][2] * xj[2][0] +
+                         xj[0][2] * xj[1][0] * xj[2][1] - xj[2][0] * xj[1][1] * xj[0][2] -
+                         xj[1][0] * xj[0][1] * xj[2][2] - xj[0][0] * xj[2][1] * xj[1][2];
+      if (active && det <= 1.e-14) mark_bad(bad, m.elnum[t]);
+      const double f = sqrt(fabs(G) / det);  // wg^3 = 1
 #pragma unroll
       for (int r = 0; r < 3; r++)
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          p[a][r] += K[r][c] * su[le][bb][c];
-          if (a != bb) p[bb][c] += K[r][c] * su[le][a][r];
-        }
-    }
-    if (!active) continue;
-    if (a == bb) {
+        for (int d = 0; d < 3; d++) ad[r][d] *= f;
 #pragma unroll
-      for (int r = 0; r < 3; r++) {
-        const int row = seq[le][a][r];
-        if (row < 0) continue;
-        k.ad[row] += K[r][r];
-        const int endr = k.ia[row + 1];
+      for (int a = 0; a < 8; a++)
 #pragma unroll
-        for (int c = 0; c < r; c++) {
-          const int col = seq[le][a][c];
-          if (col >= 0) k.al[endr - (row - col)] += K[r][c];
-        }
-      }
-    } else {
-      const int fa = sfirst[le][a], fb = sfirst[le][bb];
-      if (fa < 0 || fb < 0) continue;
-      const int off = m.slot[(size_t)pair_index(m.nen, bb, a) * m.numel + t];
-      if (fa > fb) {  // rows of a, columns of bb
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-          const int row = seq[le][a][r];
-          if (row < 0) continue;
-          const int base = k.ia[row] + off - fb;
-#pragma unroll
-          for (int c = 0; c < 3; c++)
-            if (seq[le][bb][c] >= 0) k.al[base + seq[le][bb][c]] += K[r][c];
-        }
-      } else {  // rows of bb, columns of a: entry (bb c, a r) = K[r][c]
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-          const int row = seq[le][bb][c];
-          if (row < 0) continue;
-          const int base = k.ia[row] + off - fa;
-#pragma unroll
-          for (int r = 0; r < 3; r++)
-            if (seq[le][a][r] >= 0) k.al[base + seq[le][a][r]] += K[r][c];
-        }
-      }
+        for (int d = 0; d < 3; d++)
+          ge[gp * 24 + a * 3 + d] =
+              ad[d][0] * h[a] + ad[d][1] * h[8 + a] + ad[d][2] * h[16 + a];
     }
   }
-  if (!with_u || b == nullptr) return;
-  // K u over the team: fixed shuffle tree within the team's 8 lanes (other
-  // teams of the warp may have left above)
+  // nodes lane and lane + 4: equations, the smallest of them, displacements
+  bool nz = false;
 #pragma unroll
-  for (int off = 4; off > 0; off >>= 1)
+  for (int half = 0; half < 2; half++) {
+    const int a = lane + 4 * half;
+    const int no = m.conn[(size_t)a * m.numel + te];
+    int f = -1;
 #pragma unroll
-    for (int a = 0; a < 8; a++)
+    for (int d = 2; d >= 0; d--) {
+      const int q = m.eq[(size_t)no * 3 + d];
+      seq[le][a][d] = q;
+      if (q >= 0) f = q;
+      const double ud = u ? u[(size_t)no * 3 + d] : 0.0;
+      su[le][a][d] = ud;
+      nz = nz || ud != 0.0;
+    }
+    sfirst[le][a] = f;
+  }
+  __syncwarp();
+  // K u only where the element has a non-zero displacement (an element with
+  // u = 0 adds nothing to b; the first solvm pass has u = 0 away from
+  // prescribed values): decided per team
+  const unsigned team_mask = 0xfu << (threadIdx.x & 28);
+  const bool with_u = u != nullptr && (__ballot_sync(0xffffffffu, nz) & team_mask) != 0u;
+  const bool any_u = __any_sync(0xffffffffu, with_u);
+  double p[2][3] = {{0, 0, 0}, {0, 0, 0}};  // K u of nodes 2 lane, 2 lane + 1
+  // one pair: its block K (rows a, columns c), added to the CSRC arrays
+  auto pair = [&](int a, int c, double (&K)[3][3], auto is_diag) {
+    const int *qa = seq[le][a], *qc = seq[le][c];
+    const int fa = sfirst[le][a], fc = sfirst[le][c];
+    constexpr bool diag = decltype(is_diag)::value;
+    const bool lower = fa > fc;  // rows of a; else rows of c, entry (c d, a r) = K[r][d]
+    const bool on = active && fa >= 0 && fc >= 0;
+    // where the entries go, and what is there
+    int base[3];
+    double old[3][3];
+    if (on && !diag) {
+      const int lo = min(a, c), hi = max(a, c);
+      const int off = m.slot[(size_t)pair_index(m.nen, lo, hi) * m.numel + t] - (lower ? fc : fa);
 #pragma unroll
-      for (int d = 0; d < 3; d++) p[a][d] += __shfl_xor_sync(team_mask, p[a][d], off, 8);
-  if (!active) return;
+      for (int r = 0; r < 3; r++) {
+        const int row = lower ? qa[r] : qc[r];
+        base[r] = row >= 0 ? k.ia[row] + off : 0;
+      }
 #pragma unroll
-  for (int a = 0; a < 8; a++)
-    if (a == lane)
+      for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          const int row = lower ? qa[r] : qc[r], cl = lower ? qc[d] : qa[d];
+          old[r][d] = row >= 0 && cl >= 0 ? k.al[base[r] + cl] : 0.0;
+        }
+    } else if (on) {
+#pragma unroll
+      for (int r = 0; r < 3; r++) {
+        const int row = qa[r];
+        base[r] = row >= 0 ? k.ia[row + 1] : 0;
+        old[r][r] = row >= 0 ? k.ad[row] : 0.0;
+#pragma unroll
+        for (int d = 0; d < r; d++)
+          old[r][d] = row >= 0 && qa[d] >= 0 ? k.al[base[r] - (row - qa[d])] : 0.0;
+      }
+    }
+    double M[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    const double *pa = ge + a * 3, *pc = ge + c * 3;
+#pragma unroll
+    for (int gp = 0; gp < 8; gp++) {
+      const double s0 = pa[gp * 24], s1 = pa[gp * 24 + 1], s2 = pa[gp * 24 + 2];
+      const double g0 = pc[gp * 24], g1 = pc[gp * 24 + 1], g2 = pc[gp * 24 + 2];
+      M[0][0] += s0 * g0; M[0][1] += s0 * g1; M[0][2] += s0 * g2;
+      if (!diag) M[1][0] += s1 * g0;
+      M[1][1] += s1 * g1; M[1][2] += s1 * g2;
+      if (!diag) { M[2][0] += s2 * g0; M[2][1] += s2 * g1; }
+      M[2][2] += s2 * g2;
+    }
+    if (diag) {
+      M[1][0] = M[0][1];
+      M[2][0] = M[0][2];
+      M[2][1] = M[1][2];
+    }
+    const double tr = M[0][0] + M[1][1] + M[2][2];
+#pragma unroll
+    for (int r = 0; r < 3; r++)
 #pragma unroll
       for (int d = 0; d < 3; d++)
-        if (seq[le][a][d] >= 0) b[seq[le][a][d]] -= p[a][d];
+        K[r][d] = r == d ? (sig + 1.0) * M[r][r] + tr : sig * M[r][d] + M[d][r];
+    if (neg)
+#pragma unroll
+      for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) K[r][d] = -K[r][d];
+    if (on && !diag) {
+#pragma unroll
+      for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          const int row = lower ? qa[r] : qc[r], cl = lower ? qc[d] : qa[d];
+          if (row >= 0 && cl >= 0) k.al[base[r] + cl] = old[r][d] + (lower ? K[r][d] : K[d][r]);
+        }
+    } else if (on) {
+#pragma unroll
+      for (int r = 0; r < 3; r++) {
+        const int row = qa[r];
+        if (row < 0) continue;
+        k.ad[row] = old[r][r] + K[r][r];
+#pragma unroll
+        for (int d = 0; d < r; d++)
+          if (qa[d] >= 0) k.al[base[r] - (row - qa[d])] = old[r][d] + K[r][d];
+      }
+    }
+  };
+  // K u_c (for node a) and K^T u_a (for node c)
+  auto products = [&](int a, int c, const double (&K)[3][3], double (&pa)[3], double (&pc)[3]) {
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      pa[r] = K[r][0] * su[le][c][0] + K[r][1] * su[le][c][1] + K[r][2] * su[le][c][2];
+      pc[r] = K[0][r] * su[le][a][0] + K[1][r] * su[le][a][1] + K[2][r] * su[le][a][2];
+    }
+  };
+#pragma unroll
+  for (int s = 0; s < 2; s++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int a = 2 * lane + s, c = (a + q) & 7;
+      double K[3][3];
+      if (q == 0) pair(a, a, K, std::true_type()); else pair(a, c, K, std::false_type());
+      if (any_u) {
+        double pa[3], pc[3];
+        products(a, c, K, pa, pc);
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+          p[s][r] += pa[r];
+          // node c is node (s + q) & 1 of the lane (s + q) >> 1 further on
+          if (q > 0)
+            p[(s + q) & 1][r] +=
+                __shfl_sync(0xffffffffu, pc[r], (lane - ((s + q) >> 1)) & 3, 4);
+        }
+      }
+    }
+  {
+    double K[3][3];
+    pair(lane, lane + 4, K, std::false_type());
+    if (any_u) {
+      double pa[3], pc[3];
+      products(lane, lane + 4, K, pa, pc);
+#pragma unroll
+      for (int s = 0; s < 2; s++)
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+          // node 2 lane + s: node a of lane 2 lane + s, or node c of that - 4
+          const int from = (2 * lane + s) & 3;
+          const double va = __shfl_sync(0xffffffffu, pa[r], from, 4);
+          const double vc = __shfl_sync(0xffffffffu, pc[r], from, 4);
+          p[s][r] += lane < 2 ? va : vc;
+        }
+    }
+  }
+  if (!with_u || b == nullptr || !active) return;
+#pragma unroll
+  for (int s = 0; s < 2; s++)
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      const int q = seq[le][2 * lane + s][r];
+      if (q >= 0) b[q] -= p[s][r];
+    }
 }
 
 // kHexDh for the current device, once per device.
@@ -714,7 +789,7 @@ void launch_assembly(const MeshDev &m, const CsrcDev &k, const Segment &seg,
       static const bool team = !getenv("ELX_HEX_TEAM") || atoi(getenv("ELX_HEX_TEAM")) != 0;
       if (team) {
         fill_hex_table(st);
-        hexa8_team_kernel<<<(n + kTeamElems - 1) / kTeamElems, 8 * kTeamElems, 0, st>>>(
+        hexa8_team_kernel<<<(n + kTeamElems - 1) / kTeamElems, kTeamThreads, 0, st>>>(
             m, k, seg.begin, seg.end, u, b, bad);
       } else {
         ELX_CUDA(cudaFuncSetAttribute(hexa8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

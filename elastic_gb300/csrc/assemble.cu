@@ -79,10 +79,372 @@ __device__ __forceinline__ int pair_index(int nen, int lo, int hi) {
   return lo * (nen - 1) - (lo * (lo - 1)) / 2 + (hi - lo - 1);
 }
 
+// The matrix entries an element adds to: their places and present values, all
+// loaded before the geometry is computed and stored at the end.  One thread
+// per element has few others to hide behind (20,000 threads a colour on the
+// 48^3 TETRA4 mesh), and a read-modify-write at a time waited for L2 once per
+// entry: 94 us a colour there, 40 here; QUAD4 64 x 16: 62 us, 28 here; TRIA3 301
+// x 150: 26 us, 13 here.
+template <int NEN, int NDF>
+struct Entries {
+  static constexpr int NP = NEN * (NEN - 1) / 2;
+  int base[NP][NDF];  // row starts plus the run's offset, less its first column
+  bool on[NP], rows_a[NP];
+  double old[NP][NDF][NDF], dold[NEN][NDF][NDF];
+  int dend[NEN][NDF];
+
+  // pair (a, b), b < a: the rows of the higher node, the columns of the lower
+  static __device__ __forceinline__ constexpr int at(int a, int b) { return a * (a - 1) / 2 + b; }
+
+  __device__ __forceinline__ void load(const Elem<NEN, NDF> &E, const CsrcDev &k,
+                                       const MeshDev &m, int t) {
+#pragma unroll
+    for (int a = 1; a < NEN; a++)
+#pragma unroll
+      for (int b = 0; b < a; b++) {
+        const int q = at(a, b), fa = E.first[a], fb = E.first[b];
+        on[q] = fa >= 0 && fb >= 0;
+        rows_a[q] = fa > fb;
+        const int off = m.slot[(size_t)pair_index(m.nen, b, a) * m.numel + t] -
+                        (rows_a[q] ? fb : fa);
+#pragma unroll
+        for (int r = 0; r < NDF; r++) {
+          const int row = rows_a[q] ? E.eq[a][r] : E.eq[b][r];
+          base[q][r] = on[q] && row >= 0 ? k.ia[row] + off : 0;
+        }
+      }
+#pragma unroll
+    for (int a = 0; a < NEN; a++)
+#pragma unroll
+      for (int r = 0; r < NDF; r++) {
+        const int row = E.eq[a][r];
+        dend[a][r] = row >= 0 ? k.ia[row + 1] : 0;
+        dold[a][r][r] = row >= 0 ? k.ad[row] : 0.0;
+      }
+#pragma unroll
+    for (int a = 1; a < NEN; a++)
+#pragma unroll
+      for (int b = 0; b < a; b++) {
+        const int q = at(a, b);
+#pragma unroll
+        for (int r = 0; r < NDF; r++)
+#pragma unroll
+          for (int c = 0; c < NDF; c++) {
+            const int row = rows_a[q] ? E.eq[a][r] : E.eq[b][r];
+            const int col = rows_a[q] ? E.eq[b][c] : E.eq[a][c];
+            old[q][r][c] = on[q] && row >= 0 && col >= 0 ? k.al[base[q][r] + col] : 0.0;
+          }
+      }
+    // a node's own lower columns are the last entries of its rows (column c of
+    // row r at ia[r + 1] - (r - c))
+#pragma unroll
+    for (int a = 0; a < NEN; a++)
+#pragma unroll
+      for (int r = 0; r < NDF; r++)
+#pragma unroll
+        for (int c = 0; c < r; c++) {
+          const int row = E.eq[a][r], col = E.eq[a][c];
+          dold[a][r][c] = row >= 0 && col >= 0 ? k.al[dend[a][r] - (row - col)] : 0.0;
+        }
+  }
+};
+
+// Adds the block K_ab (rows = dofs of local node a, columns = dofs of b) of a
+// node pair b < a to al, and both directions of K u to p.
+template <int NEN, int NDF>
+__device__ __forceinline__ void scatter_pair(Elem<NEN, NDF> &E, const Entries<NEN, NDF> &N,
+                                             const CsrcDev &k, int a, int b,
+                                             const double (&K)[NDF][NDF], bool with_u) {
+  if (with_u) {
+#pragma unroll
+    for (int r = 0; r < NDF; r++)
+#pragma unroll
+      for (int c = 0; c < NDF; c++) {
+        E.p[a][r] += K[r][c] * E.u[b][c];
+        E.p[b][c] += K[r][c] * E.u[a][r];
+      }
+  }
+  const int q = Entries<NEN, NDF>::at(a, b);
+  if (!N.on[q]) return;
+#pragma unroll
+  for (int r = 0; r < NDF; r++)
+#pragma unroll
+    for (int c = 0; c < NDF; c++) {
+      const int row = N.rows_a[q] ? E.eq[a][r] : E.eq[b][r];
+      const int col = N.rows_a[q] ? E.eq[b][c] : E.eq[a][c];
+      if (row >= 0 && col >= 0)
+        k.al[N.base[q][r] + col] = N.old[q][r][c] + (N.rows_a[q] ? K[r][c] : K[c][r]);
+    }
+}
+
+// Diagonal block of node a: ad and the node's own lower entries.
+template <int NEN, int NDF>
+__device__ __forceinline__ void scatter_diag(Elem<NEN, NDF> &E, const Entries<NEN, NDF> &N,
+                                             const CsrcDev &k, int a,
+                                             const double (&K)[NDF][NDF], bool with_u) {
+  if (with_u) {
+#pragma unroll
+    for (int r = 0; r < NDF; r++)
+#pragma unroll
+      for (int c = 0; c < NDF; c++) E.p[a][r] += K[r][c] * E.u[a][c];
+  }
+#pragma unroll
+  for (int r = 0; r < NDF; r++) {
+    const int row = E.eq[a][r];
+    if (row < 0) continue;
+    k.ad[row] = N.dold[a][r][r] + K[r][r];
+#pragma unroll
+    for (int c = 0; c < r; c++) {
+      const int col = E.eq[a][c];
+      if (col >= 0) k.al[N.dend[a][r] - (row - col)] = N.dold[a][r][c] + K[r][c];
+    }
+  }
+}
+
+// Returns whether the element has a non-zero displacement (one without adds
+// nothing to b; the first solvm pass has u = 0 away from prescribed values).
+template <int NEN, int NDF>
+__device__ __forceinline__ bool load_elem(Elem<NEN, NDF> &E, const MeshDev &m, int t,
+                                          const int (&node)[NEN], const double *u) {
+  bool nz = false;
+#pragma unroll
+  for (int a = 0; a < NEN; a++) {
+    int f = -1;
+#pragma unroll
+    for (int d = NDF - 1; d >= 0; d--) {
+      const int q = m.eq[(size_t)node[a] * NDF + d];
+      E.eq[a][d] = q;
+      if (q >= 0) f = q;
+      E.u[a][d] = u ? u[(size_t)node[a] * NDF + d] : 0.0;
+      E.p[a][d] = 0.0;
+      nz = nz || E.u[a][d] != 0.0;
+    }
+    E.first[a] = f;
+  }
+  return nz;
+}
+
+// b(k) = b(k) - p(i) for free dofs (Assbly.f:118).
+template <int NEN, int NDF>
+__device__ __forceinline__ void finish_rhs(const Elem<NEN, NDF> &E, double *b) {
+  if (b == nullptr) return;
+#pragma unroll
+  for (int a = 0; a < NEN; a++)
+#pragma unroll
+    for (int d = 0; d < NDF; d++)
+      if (E.eq[a][d] >= 0) b[E.eq[a][d]] -= E.p[a][d];
+}
+
+__device__ __forceinline__ void mark_bad(int32_t *bad, int elnum) { atomicMin(bad, elnum); }
+
+// 2-D block from M = sum wt g_i g_j^T (rows x, y).
+__device__ __forceinline__ void block2d(const Law &L, const double (&M)[2][2],
+                                        double (&K)[2][2]) {
+  K[0][0] = L.d11 * M[0][0] + L.d33 * M[1][1];
+  K[0][1] = L.d12 * M[0][1] + L.d33 * M[1][0];
+  K[1][0] = L.d12 * M[1][0] + L.d33 * M[0][1];
+  K[1][1] = L.d22 * M[1][1] + L.d33 * M[0][0];
+}
+
+// 3-D block from M = sum wt1 g_i g_j^T: b M + c M^T + c tr(M) I.
+__device__ __forceinline__ void block3d(const Law &L, const double (&M)[3][3],
+                                        double (&K)[3][3]) {
+  const double tr = L.c * (M[0][0] + M[1][1] + M[2][2]);
+#pragma unroll
+  for (int r = 0; r < 3; r++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) K[r][c] = L.b * M[r][c] + L.c * M[c][r] + (r == c ? tr : 0.0);
+}
+
+// ---------------------------------------------------------------- TRIA3
+// elmt02_mec / elmt03_mec (Elmlib02.f:50-627): constant-strain triangle,
+// wt1 = det/2; the plane-stress thickness is not applied to K (as there).
+__global__ void __launch_bounds__(64) tria3_kernel(MeshDev m, CsrcDev k, int begin, int end, int iel,
+                             const double *__restrict__ u, double *__restrict__ b,
+                             int32_t *bad) {
+  const int t = begin + blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= end) return;
+  int node[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) node[a] = m.conn[(size_t)a * m.numel + t];
+  Elem<3, 2> E;
+  const bool with_u = load_elem<3, 2>(E, m, t, node, u);
+  Entries<3, 2> N;
+  N.load(E, k, m, t);
+  double xl[3][2];
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    xl[a][0] = m.x[(size_t)node[a] * m.ndm + 0];
+    xl[a][1] = m.x[(size_t)node[a] * m.ndm + 1];
+  }
+  const double xj11 = xl[0][0] - xl[2][0], xj12 = xl[0][1] - xl[2][1];
+  const double xj21 = xl[1][0] - xl[2][0], xj22 = xl[1][1] - xl[2][1];
+  const double det = xj11 * xj22 - xj12 * xj21;
+  if (det <= 0.0) { mark_bad(bad, m.elnum[t]); return; }
+  const double xji11 = xj22 / det, xji12 = -xj12 / det;
+  const double xji21 = -xj21 / det, xji22 = xj11 / det;
+  const double g[3][2] = {{xji11, xji21}, {xji12, xji22},
+                          {-xji11 - xji12, -xji21 - xji22}};
+  const Law L = make_law(iel, m.e + (size_t)m.mat[t] * m.prop);
+  const double wt1 = 0.5 * det;
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+#pragma unroll
+    for (int bb = 0; bb <= a; bb++) {
+      double M[2][2], K[2][2];
+#pragma unroll
+      for (int r = 0; r < 2; r++)
+#pragma unroll
+        for (int c = 0; c < 2; c++) M[r][c] = wt1 * g[a][r] * g[bb][c];
+      block2d(L, M, K);
+      if (a == bb) scatter_diag<3, 2>(E, N, k, a, K, with_u);
+      else scatter_pair<3, 2>(E, N, k, a, bb, K, with_u);
+    }
+  if (with_u) finish_rhs<3, 2>(E, b);
+}
+
+// ---------------------------------------------------------------- QUAD4
+// elmt04_mec / elmt05_mec (Elmlib02.f:629-1230): 2x2 Gauss with sfquad4_m
+// (Elmlib.f:815-886) and jacob2d_m (Elmlib.f:1769-1852).
+__global__ void __launch_bounds__(64) quad4_kernel(MeshDev m, CsrcDev k, int begin, int end, int iel,
+                             const double *__restrict__ u, double *__restrict__ b,
+                             int32_t *bad) {
+  const int t = begin + blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= end) return;
+  int node[4];
+#pragma unroll
+  for (int a = 0; a < 4; a++) node[a] = m.conn[(size_t)a * m.numel + t];
+  Elem<4, 2> E;
+  const bool with_u = load_elem<4, 2>(E, m, t, node, u);
+  Entries<4, 2> N;
+  N.load(E, k, m, t);
+  double xl[4][2];
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+    xl[a][0] = m.x[(size_t)node[a] * m.ndm + 0];
+    xl[a][1] = m.x[(size_t)node[a] * m.ndm + 1];
+  }
+  const Law L = make_law(iel, m.e + (size_t)m.mat[t] * m.prop);
+  double g[4][4][2];  // [gp][node][x,y]
+  double wt[4];
+#pragma unroll
+  for (int ly = 0; ly < 2; ly++)
+#pragma unroll
+    for (int lx = 0; lx < 2; lx++) {
+      const int gp = ly * 2 + lx;
+      const double r = kPg2[lx], s = kPg2[ly];
+      const double opr = 1.0 + r, ops = 1.0 + s, omr = 1.0 - r, oms = 1.0 - s;
+      const double hr[4] = {ops * 0.25, -(ops * 0.25), -(oms * 0.25), oms * 0.25};
+      const double hs[4] = {opr * 0.25, omr * 0.25, -(omr * 0.25), -(opr * 0.25)};
+      double j11 = 0, j12 = 0, j21 = 0, j22 = 0;
+#pragma unroll
+      for (int a = 0; a < 4; a++) {
+        j11 += hr[a] * xl[a][0];
+        j12 += hr[a] * xl[a][1];
+        j21 += hs[a] * xl[a][0];
+        j22 += hs[a] * xl[a][1];
+      }
+      const double det = j11 * j22 - j21 * j12;
+      if (det <= 1.e-14) { mark_bad(bad, m.elnum[t]); return; }
+      const double i11 = j22 / det, i12 = -j12 / det, i21 = -j21 / det, i22 = j11 / det;
+#pragma unroll
+      for (int a = 0; a < 4; a++) {
+        g[gp][a][0] = i11 * hr[a] + i12 * hs[a];
+        g[gp][a][1] = i21 * hr[a] + i22 * hs[a];
+      }
+      wt[gp] = det * L.thic;  // wg(lx)*wg(ly) = 1
+    }
+#pragma unroll
+  for (int a = 0; a < 4; a++)
+#pragma unroll
+    for (int bb = 0; bb <= a; bb++) {
+      double M[2][2] = {{0, 0}, {0, 0}}, K[2][2];
+#pragma unroll
+      for (int gp = 0; gp < 4; gp++) {
+        const double s0 = wt[gp] * g[gp][a][0], s1 = wt[gp] * g[gp][a][1];
+        M[0][0] += s0 * g[gp][bb][0];
+        M[0][1] += s0 * g[gp][bb][1];
+        M[1][0] += s1 * g[gp][bb][0];
+        M[1][1] += s1 * g[gp][bb][1];
+      }
+      block2d(L, M, K);
+      if (a == bb) scatter_diag<4, 2>(E, N, k, a, K, with_u);
+      else scatter_pair<4, 2>(E, N, k, a, bb, K, with_u);
+    }
+  if (with_u) finish_rhs<4, 2>(E, b);
+}
+
+// --------------------------------------------------------------- TETRA4
+// elmt06_mec (Elmlib02.f:1232-1573) with jtetra4 (Elmlib.f:2636-2713):
+// constant strain, wt1 = a * det * div6 with the literal div6.
+__global__ void __launch_bounds__(64) tetra4_kernel(MeshDev m, CsrcDev k, int begin, int end,
+                              const double *__restrict__ u, double *__restrict__ b,
+                              int32_t *bad) {
+  const int t = begin + blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= end) return;
+  int node[4];
+#pragma unroll
+  for (int a = 0; a < 4; a++) node[a] = m.conn[(size_t)a * m.numel + t];
+  Elem<4, 3> E;
+  const bool with_u = load_elem<4, 3>(E, m, t, node, u);
+  Entries<4, 3> N;
+  N.load(E, k, m, t);
+  double xl[4][3];
+#pragma unroll
+  for (int a = 0; a < 4; a++)
+#pragma unroll
+    for (int d = 0; d < 3; d++) xl[a][d] = m.x[(size_t)node[a] * 3 + d];
+  double xj[3][3];
+#pragma unroll
+  for (int r = 0; r < 3; r++)
+#pragma unroll
+    for (int d = 0; d < 3; d++) xj[r][d] = xl[r][d] - xl[3][d];
+  const double det = xj[0][0] * xj[1][1] * xj[2][2] + xj[0][1] * xj[1][2] * xj[2][0] +
+                     xj[0][2] * xj[1][0] * xj[2][1] - xj[2][0] * xj[1][1] * xj[0][2] -
+                     xj[0][1] * xj[1][0] * xj[2][2] - xj[0][0] * xj[2][1] * xj[1][2];
+  if (det <= 1.e-14) { mark_bad(bad, m.elnum[t]); return; }
+  const double deti = 1.0 / det;
+  double g[4][3];
+  g[0][0] = (xj[1][1] * xj[2][2] - xj[1][2] * xj[2][1]) * deti;
+  g[1][0] = (xj[0][2] * xj[2][1] - xj[0][1] * xj[2][2]) * deti;
+  g[2][0] = (xj[0][1] * xj[1][2] - xj[0][2] * xj[1][1]) * deti;
+  g[0][1] = (xj[1][2] * xj[2][0] - xj[1][0] * xj[2][2]) * deti;
+  g[1][1] = (xj[0][0] * xj[2][2] - xj[0][2] * xj[2][0]) * deti;
+  g[2][1] = (xj[0][2] * xj[1][0] - xj[0][0] * xj[1][2]) * deti;
+  g[0][2] = (xj[1][0] * xj[2][1] - xj[1][1] * xj[2][0]) * deti;
+  g[1][2] = (xj[0][1] * xj[2][0] - xj[0][0] * xj[2][1]) * deti;
+  g[2][2] = (xj[0][0] * xj[1][1] - xj[0][1] * xj[1][0]) * deti;
+#pragma unroll
+  for (int d = 0; d < 3; d++) g[3][d] = -g[0][d] - g[1][d] - g[2][d];
+  const Law L = make_law(TETRA4, m.e + (size_t)m.mat[t] * m.prop);
+  const double div6 = 0.166666666666667e+00;
+  const double wt1 = L.a * det * div6;
+#pragma unroll
+  for (int a = 0; a < 4; a++)
+#pragma unroll
+    for (int bb = 0; bb <= a; bb++) {
+      double M[3][3], K[3][3];
+#pragma unroll
+      for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) M[r][c] = wt1 * g[a][r] * g[bb][c];
+      block3d(L, M, K);
+      if (a == bb) scatter_diag<4, 3>(E, N, k, a, K, with_u);
+      else scatter_pair<4, 3>(E, N, k, a, bb, K, with_u);
+    }
+  if (with_u) finish_rhs<4, 3>(E, b);
+}
+
+// ---------------------------------------------------------------- HEXA8
+// elmt07_mec (Elmlib02.f:1577-2023): 2x2x2 Gauss with sfhexa8_m
+// (Elmlib.f:1151-1258) and jacob3d_m (Elmlib.f:1942-2036).  The shape
+// function gradients of the 8 points are kept in shared memory, one column
+// per thread ([gp][node][xyz][thread]) so that accesses are bank-conflict free.
+// (one entry at a time: 36 pairs are too many to load ahead)
 // Adds the block K_ab (rows = dofs of local node a, columns = dofs of b) of a
 // node pair a != b into al, and both directions of K u into p.
 template <int NEN, int NDF>
-__device__ __forceinline__ void scatter_pair(Elem<NEN, NDF> &E, const CsrcDev &k,
+__device__ __forceinline__ void scatter_pair_rmw(Elem<NEN, NDF> &E, const CsrcDev &k,
                                              const MeshDev &m, int t, int a, int b,
                                              const double (&K)[NDF][NDF], bool with_u) {
   if (with_u) {
@@ -124,7 +486,7 @@ __device__ __forceinline__ void scatter_pair(Elem<NEN, NDF> &E, const CsrcDev &k
 // Diagonal block of node a: ad and the node's own lower entries, which are
 // the last entries of each of its rows (column c of row r at ia[r+1]-(r-c)).
 template <int NEN, int NDF>
-__device__ __forceinline__ void scatter_diag(Elem<NEN, NDF> &E, const CsrcDev &k, int a,
+__device__ __forceinline__ void scatter_diag_rmw(Elem<NEN, NDF> &E, const CsrcDev &k, int a,
                                              const double (&K)[NDF][NDF], bool with_u) {
   if (with_u) {
 #pragma unroll
@@ -146,237 +508,6 @@ __device__ __forceinline__ void scatter_diag(Elem<NEN, NDF> &E, const CsrcDev &k
   }
 }
 
-template <int NEN, int NDF>
-__device__ __forceinline__ void load_elem(Elem<NEN, NDF> &E, const MeshDev &m, int t,
-                                          const int (&node)[NEN], const double *u) {
-#pragma unroll
-  for (int a = 0; a < NEN; a++) {
-    int f = -1;
-#pragma unroll
-    for (int d = NDF - 1; d >= 0; d--) {
-      const int q = m.eq[(size_t)node[a] * NDF + d];
-      E.eq[a][d] = q;
-      if (q >= 0) f = q;
-      E.u[a][d] = u ? u[(size_t)node[a] * NDF + d] : 0.0;
-      E.p[a][d] = 0.0;
-    }
-    E.first[a] = f;
-  }
-}
-
-// b(k) = b(k) - p(i) for free dofs (Assbly.f:118).
-template <int NEN, int NDF>
-__device__ __forceinline__ void finish_rhs(const Elem<NEN, NDF> &E, double *b) {
-  if (b == nullptr) return;
-#pragma unroll
-  for (int a = 0; a < NEN; a++)
-#pragma unroll
-    for (int d = 0; d < NDF; d++)
-      if (E.eq[a][d] >= 0) b[E.eq[a][d]] -= E.p[a][d];
-}
-
-__device__ __forceinline__ void mark_bad(int32_t *bad, int elnum) { atomicMin(bad, elnum); }
-
-// 2-D block from M = sum wt g_i g_j^T (rows x, y).
-__device__ __forceinline__ void block2d(const Law &L, const double (&M)[2][2],
-                                        double (&K)[2][2]) {
-  K[0][0] = L.d11 * M[0][0] + L.d33 * M[1][1];
-  K[0][1] = L.d12 * M[0][1] + L.d33 * M[1][0];
-  K[1][0] = L.d12 * M[1][0] + L.d33 * M[0][1];
-  K[1][1] = L.d22 * M[1][1] + L.d33 * M[0][0];
-}
-
-// 3-D block from M = sum wt1 g_i g_j^T: b M + c M^T + c tr(M) I.
-__device__ __forceinline__ void block3d(const Law &L, const double (&M)[3][3],
-                                        double (&K)[3][3]) {
-  const double tr = L.c * (M[0][0] + M[1][1] + M[2][2]);
-#pragma unroll
-  for (int r = 0; r < 3; r++)
-#pragma unroll
-    for (int c = 0; c < 3; c++) K[r][c] = L.b * M[r][c] + L.c * M[c][r] + (r == c ? tr : 0.0);
-}
-
-// ---------------------------------------------------------------- TRIA3
-// elmt02_mec / elmt03_mec (Elmlib02.f:50-627): constant-strain triangle,
-// wt1 = det/2; the plane-stress thickness is not applied to K (as there).
-__global__ void tria3_kernel(MeshDev m, CsrcDev k, int begin, int end, int iel,
-                             const double *__restrict__ u, double *__restrict__ b,
-                             int32_t *bad) {
-  const int t = begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= end) return;
-  int node[3];
-#pragma unroll
-  for (int a = 0; a < 3; a++) node[a] = m.conn[(size_t)a * m.numel + t];
-  double xl[3][2];
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    xl[a][0] = m.x[(size_t)node[a] * m.ndm + 0];
-    xl[a][1] = m.x[(size_t)node[a] * m.ndm + 1];
-  }
-  const double xj11 = xl[0][0] - xl[2][0], xj12 = xl[0][1] - xl[2][1];
-  const double xj21 = xl[1][0] - xl[2][0], xj22 = xl[1][1] - xl[2][1];
-  const double det = xj11 * xj22 - xj12 * xj21;
-  if (det <= 0.0) { mark_bad(bad, m.elnum[t]); return; }
-  const double xji11 = xj22 / det, xji12 = -xj12 / det;
-  const double xji21 = -xj21 / det, xji22 = xj11 / det;
-  const double g[3][2] = {{xji11, xji21}, {xji12, xji22},
-                          {-xji11 - xji12, -xji21 - xji22}};
-  const Law L = make_law(iel, m.e + (size_t)m.mat[t] * m.prop);
-  const double wt1 = 0.5 * det;
-  Elem<3, 2> E;
-  load_elem<3, 2>(E, m, t, node, u);
-  const bool with_u = u != nullptr;
-#pragma unroll
-  for (int a = 0; a < 3; a++)
-#pragma unroll
-    for (int bb = 0; bb <= a; bb++) {
-      double M[2][2], K[2][2];
-#pragma unroll
-      for (int r = 0; r < 2; r++)
-#pragma unroll
-        for (int c = 0; c < 2; c++) M[r][c] = wt1 * g[a][r] * g[bb][c];
-      block2d(L, M, K);
-      if (a == bb) scatter_diag<3, 2>(E, k, a, K, with_u);
-      else scatter_pair<3, 2>(E, k, m, t, a, bb, K, with_u);
-    }
-  finish_rhs<3, 2>(E, b);
-}
-
-// ---------------------------------------------------------------- QUAD4
-// elmt04_mec / elmt05_mec (Elmlib02.f:629-1230): 2x2 Gauss with sfquad4_m
-// (Elmlib.f:815-886) and jacob2d_m (Elmlib.f:1769-1852).
-__global__ void quad4_kernel(MeshDev m, CsrcDev k, int begin, int end, int iel,
-                             const double *__restrict__ u, double *__restrict__ b,
-                             int32_t *bad) {
-  const int t = begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= end) return;
-  int node[4];
-#pragma unroll
-  for (int a = 0; a < 4; a++) node[a] = m.conn[(size_t)a * m.numel + t];
-  double xl[4][2];
-#pragma unroll
-  for (int a = 0; a < 4; a++) {
-    xl[a][0] = m.x[(size_t)node[a] * m.ndm + 0];
-    xl[a][1] = m.x[(size_t)node[a] * m.ndm + 1];
-  }
-  const Law L = make_law(iel, m.e + (size_t)m.mat[t] * m.prop);
-  double g[4][4][2];  // [gp][node][x,y]
-  double wt[4];
-#pragma unroll
-  for (int ly = 0; ly < 2; ly++)
-#pragma unroll
-    for (int lx = 0; lx < 2; lx++) {
-      const int gp = ly * 2 + lx;
-      const double r = kPg2[lx], s = kPg2[ly];
-      const double opr = 1.0 + r, ops = 1.0 + s, omr = 1.0 - r, oms = 1.0 - s;
-      const double hr[4] = {ops * 0.25, -(ops * 0.25), -(oms * 0.25), oms * 0.25};
-      const double hs[4] = {opr * 0.25, omr * 0.25, -(omr * 0.25), -(opr * 0.25)};
-      double j11 = 0, j12 = 0, j21 = 0, j22 = 0;
-#pragma unroll
-      for (int a = 0; a < 4; a++) {
-        j11 += hr[a] * xl[a][0];
-        j12 += hr[a] * xl[a][1];
-        j21 += hs[a] * xl[a][0];
-        j22 += hs[a] * xl[a][1];
-      }
-      const double det = j11 * j22 - j21 * j12;
-      if (det <= 1.e-14) { mark_bad(bad, m.elnum[t]); return; }
-      const double i11 = j22 / det, i12 = -j12 / det, i21 = -j21 / det, i22 = j11 / det;
-#pragma unroll
-      for (int a = 0; a < 4; a++) {
-        g[gp][a][0] = i11 * hr[a] + i12 * hs[a];
-        g[gp][a][1] = i21 * hr[a] + i22 * hs[a];
-      }
-      wt[gp] = det * L.thic;  // wg(lx)*wg(ly) = 1
-    }
-  Elem<4, 2> E;
-  load_elem<4, 2>(E, m, t, node, u);
-  const bool with_u = u != nullptr;
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int bb = 0; bb <= a; bb++) {
-      double M[2][2] = {{0, 0}, {0, 0}}, K[2][2];
-#pragma unroll
-      for (int gp = 0; gp < 4; gp++) {
-        const double s0 = wt[gp] * g[gp][a][0], s1 = wt[gp] * g[gp][a][1];
-        M[0][0] += s0 * g[gp][bb][0];
-        M[0][1] += s0 * g[gp][bb][1];
-        M[1][0] += s1 * g[gp][bb][0];
-        M[1][1] += s1 * g[gp][bb][1];
-      }
-      block2d(L, M, K);
-      if (a == bb) scatter_diag<4, 2>(E, k, a, K, with_u);
-      else scatter_pair<4, 2>(E, k, m, t, a, bb, K, with_u);
-    }
-  finish_rhs<4, 2>(E, b);
-}
-
-// --------------------------------------------------------------- TETRA4
-// elmt06_mec (Elmlib02.f:1232-1573) with jtetra4 (Elmlib.f:2636-2713):
-// constant strain, wt1 = a * det * div6 with the literal div6.
-__global__ void tetra4_kernel(MeshDev m, CsrcDev k, int begin, int end,
-                              const double *__restrict__ u, double *__restrict__ b,
-                              int32_t *bad) {
-  const int t = begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= end) return;
-  int node[4];
-#pragma unroll
-  for (int a = 0; a < 4; a++) node[a] = m.conn[(size_t)a * m.numel + t];
-  double xl[4][3];
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int d = 0; d < 3; d++) xl[a][d] = m.x[(size_t)node[a] * 3 + d];
-  double xj[3][3];
-#pragma unroll
-  for (int r = 0; r < 3; r++)
-#pragma unroll
-    for (int d = 0; d < 3; d++) xj[r][d] = xl[r][d] - xl[3][d];
-  const double det = xj[0][0] * xj[1][1] * xj[2][2] + xj[0][1] * xj[1][2] * xj[2][0] +
-                     xj[0][2] * xj[1][0] * xj[2][1] - xj[2][0] * xj[1][1] * xj[0][2] -
-                     xj[0][1] * xj[1][0] * xj[2][2] - xj[0][0] * xj[2][1] * xj[1][2];
-  if (det <= 1.e-14) { mark_bad(bad, m.elnum[t]); return; }
-  const double deti = 1.0 / det;
-  double g[4][3];
-  g[0][0] = (xj[1][1] * xj[2][2] - xj[1][2] * xj[2][1]) * deti;
-  g[1][0] = (xj[0][2] * xj[2][1] - xj[0][1] * xj[2][2]) * deti;
-  g[2][0] = (xj[0][1] * xj[1][2] - xj[0][2] * xj[1][1]) * deti;
-  g[0][1] = (xj[1][2] * xj[2][0] - xj[1][0] * xj[2][2]) * deti;
-  g[1][1] = (xj[0][0] * xj[2][2] - xj[0][2] * xj[2][0]) * deti;
-  g[2][1] = (xj[0][2] * xj[1][0] - xj[0][0] * xj[1][2]) * deti;
-  g[0][2] = (xj[1][0] * xj[2][1] - xj[1][1] * xj[2][0]) * deti;
-  g[1][2] = (xj[0][1] * xj[2][0] - xj[0][0] * xj[2][1]) * deti;
-  g[2][2] = (xj[0][0] * xj[1][1] - xj[0][1] * xj[1][0]) * deti;
-#pragma unroll
-  for (int d = 0; d < 3; d++) g[3][d] = -g[0][d] - g[1][d] - g[2][d];
-  const Law L = make_law(TETRA4, m.e + (size_t)m.mat[t] * m.prop);
-  const double div6 = 0.166666666666667e+00;
-  const double wt1 = L.a * det * div6;
-  Elem<4, 3> E;
-  load_elem<4, 3>(E, m, t, node, u);
-  const bool with_u = u != nullptr;
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int bb = 0; bb <= a; bb++) {
-      double M[3][3], K[3][3];
-#pragma unroll
-      for (int r = 0; r < 3; r++)
-#pragma unroll
-        for (int c = 0; c < 3; c++) M[r][c] = wt1 * g[a][r] * g[bb][c];
-      block3d(L, M, K);
-      if (a == bb) scatter_diag<4, 3>(E, k, a, K, with_u);
-      else scatter_pair<4, 3>(E, k, m, t, a, bb, K, with_u);
-    }
-  finish_rhs<4, 3>(E, b);
-}
-
-// ---------------------------------------------------------------- HEXA8
-// elmt07_mec (Elmlib02.f:1577-2023): 2x2x2 Gauss with sfhexa8_m
-// (Elmlib.f:1151-1258) and jacob3d_m (Elmlib.f:1942-2036).  The shape
-// function gradients of the 8 points are kept in shared memory, one column
-// per thread ([gp][node][xyz][thread]) so that accesses are bank-conflict free.
 constexpr int kHexThreads = 64;
 constexpr size_t kHexSmem = sizeof(double) * 8 * 8 * 3 * kHexThreads;
 
@@ -446,8 +577,7 @@ hexa8_kernel(MeshDev m, CsrcDev k, int begin, int end, const double *__restrict_
         wt[gp] = det * L.a;  // wg^3 = 1
       }
   Elem<8, 3> E;
-  load_elem<8, 3>(E, m, t, node, u);
-  const bool with_u = u != nullptr;
+  const bool with_u = load_elem<8, 3>(E, m, t, node, u);
   for (int a = 0; a < 8; a++) {
     double sa[8][3];
 #pragma unroll
@@ -467,11 +597,11 @@ hexa8_kernel(MeshDev m, CsrcDev k, int begin, int end, const double *__restrict_
         }
       }
       block3d(L, M, K);
-      if (a == bb) scatter_diag<8, 3>(E, k, a, K, with_u);
-      else scatter_pair<8, 3>(E, k, m, t, a, bb, K, with_u);
+      if (a == bb) scatter_diag_rmw<8, 3>(E, k, a, K, with_u);
+      else scatter_pair_rmw<8, 3>(E, k, m, t, a, bb, K, with_u);
     }
   }
-  finish_rhs<8, 3>(E, b);
+  if (with_u) finish_rhs<8, 3>(E, b);
 #undef SG
 }
 
@@ -776,14 +906,14 @@ void launch_assembly(const MeshDev &m, const CsrcDev &k, const Segment &seg,
   switch (seg.iel) {
     case TRIA3_STRAIN:
     case TRIA3_STRESS:
-      tria3_kernel<<<(n + 127) / 128, 128, 0, st>>>(m, k, seg.begin, seg.end, seg.iel, u, b, bad);
+      tria3_kernel<<<(n + 63) / 64, 64, 0, st>>>(m, k, seg.begin, seg.end, seg.iel, u, b, bad);
       break;
     case QUAD4_STRAIN:
     case QUAD4_STRESS:
-      quad4_kernel<<<(n + 127) / 128, 128, 0, st>>>(m, k, seg.begin, seg.end, seg.iel, u, b, bad);
+      quad4_kernel<<<(n + 63) / 64, 64, 0, st>>>(m, k, seg.begin, seg.end, seg.iel, u, b, bad);
       break;
     case TETRA4:
-      tetra4_kernel<<<(n + 127) / 128, 128, 0, st>>>(m, k, seg.begin, seg.end, u, b, bad);
+      tetra4_kernel<<<(n + 63) / 64, 64, 0, st>>>(m, k, seg.begin, seg.end, u, b, bad);
       break;
     case HEXA8: {
       static const bool team = !getenv("ELX_HEX_TEAM") || atoi(getenv("ELX_HEX_TEAM")) != 0;

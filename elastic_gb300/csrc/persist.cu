@@ -12,8 +12,8 @@
 // dots and the new p.  Arithmetic that does not need a dot runs in the other
 // warps while the first waits for it: x, the slices cut between warps, the
 // stopping test.  Per iteration, launches -> here: 16.2 -> 7.0 us (2,176
-// equations, QUAD4), 19.8 -> 10.3 (90,902, TRIA3), 33.1 -> 11.2 (26,460,
-// HEXA8), 72.2 -> 60.3 (345,744, HEXA8), 142 -> 130 (811,200, HEXA8: the
+// equations, QUAD4), 19.8 -> 9.9 (90,902, TRIA3), 33.1 -> 11.2 (26,460,
+// HEXA8), 72.2 -> 60.3 (345,744, HEXA8), 142 -> 127 (811,200, HEXA8: the
 // FP64 pipe's floor is 110).
 //
 // Up to kGridCols load cases go through one launch: they share the matrix

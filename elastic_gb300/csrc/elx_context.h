@@ -105,6 +105,9 @@ struct elx_ctx {
   bool want_blocks = true;   // node blocks are not switched off
   int persist_grid = 0, persist_rows = 0, persist_slices = 0;
   int persist_mode[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  // the same by one cluster of blocks for one column (0: not used; its cuts
+  // follow the grid's in persist_cta)
+  int cluster_grid = 0, cluster_rows = 0, cluster_slices = 0;
   elx::PersistCol *h_cols = nullptr;  // pinned, 2 slots of 6
 
   int64_t launches = 0;  // kernels of this library launched by this context

@@ -26,7 +26,7 @@ namespace elx {
 constexpr int kGridMaxBlocks = 160;
 constexpr uint64_t kGridWaitNs = 2000000000ull;  // bound of every grid wait
 constexpr int kDigits = 5;
-
+constexpr int kClusterBlocks = 16;  // the most that a cluster has
 
 // Shared by the blocks of a launch; zeroed before each launch.
 struct alignas(128) GridWords {
@@ -293,6 +293,63 @@ __device__ __forceinline__ bool sum(Team team, const V (&v)[NC], GridSync *gs, i
   return sh.ok != 0;
 }
 
+// The same for the blocks of one cluster: every block writes its partials into
+// all blocks' shared memory, and the hardware's cluster barrier stands for the
+// polls.  `slots` alternate with `which`; between two uses of one lies another
+// barrier, which a block reaches after reading the first.
+template <int NC>
+struct Cluster {
+  int me, n;
+  FixSum (*slots)[NC][kClusterBlocks];  // [2], shared memory
+};
+
+template <int T, int NC, class V, class F, class H>
+__device__ __forceinline__ bool sum(Cluster<NC> team, const V (&v)[NC], GridSync *, int which,
+                                    const double *, unsigned long long &, uint64_t,
+                                    Scratch<T, NC> &sh, F then, H meanwhile) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int c = 0; c < NC; c++) {
+    const FixSum s = warp_sum(fix_of(v[c]));
+    if (lane == 0) sh.part[c][w] = s;
+  }
+  __syncthreads();
+  if (w == 0) {
+    FixSum mine;
+    mine.m = 0;
+    mine.e = -4096;
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+      FixSum t;
+      t.m = 0;
+      t.e = -4096;
+      if (lane < T / 32) t = sh.part[c][lane];
+      t = warp_sum(t);  // in every lane: one for each block
+      if (lane < team.n) ptx::store_cluster(&team.slots[which][c][team.me], lane, t.m, t.e);
+    }
+    __syncwarp();
+    ptx::cluster_arrive();
+    ptx::cluster_wait();
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+      FixSum t;
+      t.m = 0;
+      t.e = -4096;
+      if (lane < team.n) t = team.slots[which][c][lane];
+      t = warp_sum(t);
+      if (lane == c) mine = t;
+    }
+    if (lane < NC) then(fix_value(mine));
+  } else {
+    ptx::cluster_arrive();
+    meanwhile();
+    __syncwarp();
+    ptx::cluster_wait();
+  }
+  __syncthreads();
+  return true;
+}
+
 // Makes the blocks' global stores visible to one another.  The fences on both
 // sides order the data (and drop stale L1 lines).  `count`: barriers passed
 // in this launch, this one included.
@@ -313,6 +370,14 @@ __device__ __forceinline__ bool barrier(Team team, GridSync *gs, uint32_t count,
   }
   __syncthreads();
   return sh.ok != 0;
+}
+
+template <int T, int NC>
+__device__ __forceinline__ bool barrier(Cluster<NC>, GridSync *, uint32_t, Scratch<T, NC> &) {
+  __syncwarp();
+  ptx::cluster_arrive();
+  ptx::cluster_wait();
+  return true;
 }
 
 }  // namespace grid

@@ -38,11 +38,11 @@ size_t persist_smem(int rows, int slices) {
          sizeof(int32_t) * ((size_t)(slices + 1) + (kPW + 1) + kPW);
 }
 
-// Block `team.me` of a solve's blocks (T threads): up to `steps` iterations,
-// the first of a solve with `start`.  `epoch` is above that of any earlier use
+// Block `team.me` of a solve's blocks (T threads; grid::Team or grid::Cluster):
+// up to `steps` iterations, the first of a solve with `start`.  `epoch` is above that of any earlier use
 // of a.gs's slots; a.gs's words are zero.
-template <int T, int B, int NC, bool SMEM>
-__device__ __forceinline__ void persist_pcg(const PersistArgs &a, const grid::Team team,
+template <int T, int B, int NC, bool SMEM, class Blocks>
+__device__ __forceinline__ void persist_pcg(const PersistArgs &a, const Blocks team,
                                             const int start, const int steps, uint64_t epoch) {
   constexpr int kPT = T, kPW = T / 32;
   constexpr int BB = B * B, R = kSliceRows, RB = R * B, RBC = RB * NC;

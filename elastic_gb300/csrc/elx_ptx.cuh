@@ -105,6 +105,25 @@ __device__ __forceinline__ void named_barrier(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// The hardware barrier over a cluster's threads (whole warps); memory written
+// before the arrival is visible after the wait.
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// 16 bytes to the place of `p` (this block's shared memory) in block `rank`.
+__device__ __forceinline__ void store_cluster(void *p, int rank, int64_t a, int64_t b) {
+  asm volatile(
+      "{\n\t.reg .u32 t;\n\tmapa.shared::cluster.u32 t, %0, %1;\n\t"
+      "st.shared::cluster.v2.b64 [t], {%2, %3};\n\t}" ::"r"(smem_addr(p)),
+      "r"(rank), "l"(a), "l"(b)
+      : "memory");
+}
+
 // Streaming loads of read-only data that is used once (matrix values and
 // indices): not kept in L1, and issued in program order (volatile), so that a
 // group of them is in flight before the first use.

@@ -24,6 +24,11 @@
 // start and the end of a solve: the same kernel in place of the scalar gather
 // (205,556 equations with rollers: 68 against 38 us an iteration).
 //
+// A small matrix and one load case run as one cluster of up to 16 blocks:
+// the sums go through the blocks' shared memory and the hardware's cluster
+// barrier takes the place of the polls in L2 (2,176 equations: 7.4 -> 5.4 us an
+// iteration; 512 threads a block measured as good as 256, 128 slower).
+//
 // Inside a block every warp takes the same number of slot groups (the FP64
 // pipe is charged per warp instruction; one group in flight measured faster
 // than two, 130 against 134 us at 811,200 equations); a slice cut between
@@ -38,11 +43,30 @@ namespace elx {
 namespace {
 
 constexpr int kPT = 512;  // threads of a block
+// Clocks that an iteration's waits are shorter in a cluster than in a grid
+// (net of its longer vector passes).  Either side of the line, clocks that
+// the products are longer and us an iteration as grid / cluster: 1,200 (3,720
+// TRIA3 equations) 6.84 / 5.47, 1,700 (2,187, HEXA8) 9.24 / 8.92, then 3,100
+// (8,160, TRIA3) 7.07 / 7.23, 3,500 (7,140, QUAD4) 7.23 / 7.34, 3,900 (3,000,
+// HEXA8) 9.21 / 9.28.  With two columns nothing is left at 2,176 equations
+// (8.9 / 8.7).
+constexpr double kClusterGain = 2800;
 
 template <int B, int NC, bool SMEM>
 __global__ void __launch_bounds__(kPT, 1)
 pcg_persist_kernel(PersistArgs a, int start, int steps) {
   persist_pcg<kPT, B, NC, SMEM>(a, grid::Team{(int)blockIdx.x, (int)gridDim.x}, start, steps, 0);
+}
+
+// The same by one cluster: grid::Cluster's sums and barrier.
+template <int B>
+__global__ void __launch_bounds__(kPT, 1)
+pcg_cluster_kernel(PersistArgs a, int start, int steps) {
+  __shared__ __align__(16) FixSum slots[2][1][kClusterBlocks];
+  ptx::cluster_arrive();  // the other blocks' shared memory is there
+  ptx::cluster_wait();
+  persist_pcg<kPT, B, 1, true>(a, grid::Cluster<1>{(int)blockIdx.x, (int)gridDim.x, slots}, start,
+                               steps, 0);
 }
 
 template <int B, int NC>
@@ -60,6 +84,38 @@ void launch(const PersistArgs &a, int grid, bool in_smem, int start, int steps, 
   PersistArgs arg = a;
   void *args[] = {&arg, &start, &steps};
   ELX_CUDA(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(kPT), args, bytes, st));
+}
+
+// `n` blocks as one cluster: the launch, or with `fit` whether the GPU takes
+// it (*fit > 0).
+template <int B>
+cudaError_t cluster_call(const PersistArgs &a, int n, int start, int steps, cudaStream_t st,
+                         int *fit) {
+  auto f = pcg_cluster_kernel<B>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(n);
+  cfg.blockDim = dim3(kPT);
+  cfg.dynamicSmemBytes = persist_smem<kPT, B, 1, true>(a.rows, a.slices);
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = n;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)cfg.dynamicSmemBytes);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  return fit ? cudaOccupancyMaxActiveClusters(fit, f, &cfg)
+             : cudaLaunchKernelEx(&cfg, f, a, start, steps);
+}
+
+cudaError_t cluster_call(int B, const PersistArgs &a, int n, int start, int steps,
+                         cudaStream_t st, int *fit) {
+  return B == 3 ? cluster_call<3>(a, n, start, steps, st, fit)
+                : cluster_call<2>(a, n, start, steps, st, fit);
 }
 
 #define ELX_NC_DISPATCH(nc, call)                             \
@@ -120,7 +176,9 @@ bool ensure_persist(elx_ctx *c) {
     const std::vector<int32_t> &ptr = padded ? s.p_ptr : s.sell_ptr;
     const int nslices = (int)ptr.size() - 1, B = padded ? s.p_bsize : s.bsize;
     const int grid = std::min({elx::sm_count(), elx::kGridMaxBlocks, nslices});
-    const std::vector<int32_t> cuts = elx::persist_cuts(ptr, grid);
+    std::vector<int32_t> cuts = elx::persist_cuts(ptr, grid);
+    const int cl = std::min(elx::kClusterBlocks, nslices);
+    const std::vector<int32_t> ccuts = elx::persist_cuts(ptr, cl);
     int slices = 0;
     for (int k = 0; k < grid; k++) slices = std::max(slices, cuts[k + 1] - cuts[k]);
     const int rows = slices * elx::kSliceRows * B;
@@ -132,6 +190,21 @@ bool ensure_persist(elx_ctx *c) {
                             : elx::smem_bytes(B, nc, false, rows, slices) <= (size_t)limit ? 1
                                                                                            : 0;
     if (!c->persist_mode[1]) return false;
+    // one cluster in place of the grid, for a small matrix
+    cuts.insert(cuts.end(), ccuts.begin(), ccuts.end());
+    elx::PersistArgs ca = {};
+    for (int k = 0; k < cl; k++) ca.slices = std::max(ca.slices, ccuts[k + 1] - ccuts[k]);
+    ca.rows = ca.slices * elx::kSliceRows * B;
+    // by how many clocks its blocks' products are longer: 16 of an SM's FP64
+    // pipe for each entry of a group
+    const double longer = ptr[nslices] * (1.0 / cl - 1.0 / grid) * 16 * B * B;
+    int fit = 0;
+    if (longer <= elx::kClusterGain &&
+        elx::smem_bytes(B, 1, true, ca.rows, ca.slices) <= (size_t)limit &&
+        elx::cluster_call(B, ca, cl, 0, 0, c->stream, &fit) != cudaSuccess) {
+      cudaGetLastError();  // no such cluster on this device
+      fit = 0;
+    }
     try {
       c->upload(c->persist_cta, cuts.data(), cuts.size());
       c->alloc(c->persist_sync, sizeof(elx::GridSync) + sizeof(elx::PersistCol) * elx::kGridCols);
@@ -155,6 +228,9 @@ bool ensure_persist(elx_ctx *c) {
     c->persist_rows = rows;
     c->persist_slices = slices;
     c->persist_grid = grid;
+    c->cluster_grid = fit > 0 ? cl : 0;
+    c->cluster_rows = ca.rows;
+    c->cluster_slices = ca.slices;
   }
   if (padded && !c->have_padded) {
     elx::launch_fill_padded64(c->csrc_dev(), s.p_bsize, s.p_nb, (int)s.p_ptr.size() - 1,
@@ -204,19 +280,29 @@ void persist_solve(elx_ctx *c, int nc, double tol, int maxit, const double *b, d
   a.maxit = maxit;
   a.rows = c->persist_rows;
   a.slices = c->persist_slices;
+  const bool cluster = nc == 1 && c->cluster_grid;
+  if (cluster) {
+    a.cta += c->persist_grid + 1;
+    a.rows = c->cluster_rows;
+    a.slices = c->cluster_slices;
+  }
   const bool in_smem = c->persist_mode[nc] == 2;
   const int max_launches = maxit / steps + 2;
   int launched = 0, checked = 0;
   auto go = [&] {
     const int slot = launched & 1, start = launched == 0;
-    ELX_CUDA(cudaMemsetAsync(a.gs, 0, sizeof(elx::GridSync), c->stream));
+    if (cluster) {
+      ELX_CUDA(elx::cluster_call(B, a, c->cluster_grid, start, steps, c->stream, nullptr));
+    } else {
+      ELX_CUDA(cudaMemsetAsync(a.gs, 0, sizeof(elx::GridSync), c->stream));
 #define CALL(NC)                                                                     \
   if (B == 3)                                                                        \
     elx::launch<3, NC>(a, c->persist_grid, in_smem, start, steps, c->stream);        \
   else                                                                               \
     elx::launch<2, NC>(a, c->persist_grid, in_smem, start, steps, c->stream)
-    ELX_NC_DISPATCH(nc, CALL)
+      ELX_NC_DISPATCH(nc, CALL)
 #undef CALL
+    }
     c->launches += 1;
     ELX_CUDA(cudaMemcpyAsync(c->h_cols + slot * elx::kGridCols, a.cols,
                              sizeof(elx::PersistCol) * nc, cudaMemcpyDeviceToHost, c->stream));

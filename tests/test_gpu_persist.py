@@ -187,3 +187,40 @@ def test_pack_with_teams_and_packed_launches(built_lib):
                 x, i = ctx.solve(b, tol=1e-10, maxit=50000)
                 assert abs(infos[k]["iters"] - i["iters"]) <= max(2, 0.01 * i["iters"])
                 assert rel_inf(ctx.update(x, u0), U[k]) <= 1e-8
+
+
+# one column of a small matrix runs as one cluster of up to 16 blocks: one
+# slice, 15 to 17, a last slice that is not full, partly fixed nodes, and the
+# sizes on both sides of the rule (the larger of each pair runs as a grid)
+SMALL = {
+    "quad4 1 slice": lambda: M.box2d(4, 7, etype=M.QUAD4_STRESS),
+    "quad4 15 slices": lambda: M.box2d(24, 19, etype=M.QUAD4_STRAIN),
+    "tria3 16 slices": lambda: M.box2d(32, 15, etype=M.TRIA3_STRESS),
+    "quad4 17 slices": lambda: M.box2d(32, 16, etype=M.QUAD4_STRESS),
+    "quad4 rollers": lambda: rollers(M.box2d(23, 17, etype=M.QUAD4_STRAIN), 1),
+    "hexa8 rollers": lambda: rollers(M.box_hexa8(7, 5, 6, jitter=0.1), 0),
+    "tria3 cluster": lambda: M.box2d(60, 58, etype=M.TRIA3_STRESS),
+    "tria3 grid": lambda: M.box2d(80, 56, etype=M.TRIA3_STRESS),
+    "hexa8 cluster": lambda: M.box_hexa8(8, 8, 9),
+    "hexa8 grid": lambda: M.box_hexa8(9, 10, 10),
+}
+
+
+@pytest.mark.parametrize("name", sorted(SMALL))
+def test_small_matrices(gpu_ctx, name):
+    s, ad, al, b = _system(gpu_ctx, SMALL[name]())
+    x_o, i_o = O.pcg(s, ad, al, b, tol=1e-12, maxit=20000)
+    x, i = gpu_ctx.solve(b, tol=1e-12, maxit=20000)
+    assert rel_inf(x_o, x) <= 1e-10 and abs(i["iters"] - i_o["iters"]) <= 2
+    for e in (-400, 0, 400):
+        xs, js = gpu_ctx.solve(np.ldexp(b, e), tol=1e-12, maxit=20000)
+        assert js["iters"] == i["iters"] and np.array_equal(np.ldexp(x, e), xs)
+    for maxit in (1, 7, i["iters"] - 1):
+        _, j = gpu_ctx.solve(b, tol=1e-12, maxit=maxit, raise_on_error=False)
+        assert j["status"] == E.ERR_NO_CONVERGENCE and j["iters"] == maxit
+    c = b.copy()
+    c[-1] = np.nan
+    _, j = gpu_ctx.solve(c, tol=1e-12, maxit=50, raise_on_error=False)
+    assert j["status"] == E.ERR_NO_CONVERGENCE
+    z, j = gpu_ctx.solve(0 * b, tol=1e-12)
+    assert j["status"] == 0 and j["iters"] == 0 and not z.any()

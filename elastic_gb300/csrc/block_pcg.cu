@@ -279,7 +279,7 @@ sell_spmm_kernel(int nb, int nslices, const int32_t *__restrict__ sell_ptr,
                  const int32_t *__restrict__ sell_col, const int16_t *__restrict__ col16,
                  const T *__restrict__ sval, const T *__restrict__ X, T *__restrict__ Y,
                  ColScalars *cols, BlockHeader *hdr, double *partials, unsigned int *counter,
-                 const int32_t *gate) {
+                 const int32_t *gate, int per_sm) {
   constexpr int VC = (16 / (int)sizeof(T)) < W ? (16 / (int)sizeof(T)) : W;
   constexpr int G = W / VC;
   constexpr int BB = B * B, R = kSliceRows;
@@ -298,10 +298,14 @@ sell_spmm_kernel(int nb, int nslices, const int32_t *__restrict__ sell_ptr,
   T v[VC];  // this thread's share of (x_c, y_c), in T (the FP64 pipe is narrow)
 #pragma unroll
   for (int j = 0; j < VC; j++) v[j] = T(0);
-  // passes of SPC slices, every gridDim.x-th for this CTA (contiguous runs
-  // of passes per CTA measured slower: 265 against 247 us, W = 16 FP32 on the
-  // 96x96x48 plate)
-  for (int sl = blockIdx.x * SPC + (int)threadIdx.x / (R * G); sl < nslices;
+  // Passes of SPC slices, every gridDim.x-th for this CTA (contiguous runs of
+  // passes per CTA lose the x rows that the CTAs share in L2).  CTAs b,
+  // b + SMs, b + 2 SMs, which one SM holds, take neighbouring passes: six
+  // slices then gather 918 distinct x rows instead of 1,510 and the SM's L1
+  // holds them (214 -> 208 us, W = 16 FP32 on the 96x96x48 plate).
+  const int sms = gridDim.x / per_sm;
+  const int first = (blockIdx.x % sms) * per_sm + blockIdx.x / sms;
+  for (int sl = first * SPC + (int)threadIdx.x / (R * G); sl < nslices;
        sl += gridDim.x * SPC) {
     const int g0 = sell_ptr[sl], g1 = sell_ptr[sl + 1];
     T acc[B][VC];
@@ -320,10 +324,9 @@ sell_spmm_kernel(int nb, int nslices, const int32_t *__restrict__ sell_ptr,
       for (int u = 0; u < U; u++)
         if (u < nu) sell_load<T, B, LD>(sval + (size_t)(g + u) * BB * R, t, bv[u]);
       // x of each group loaded just before its FMAs (mostly L1 hits): the
-      // registers go to more groups of matrix loads in flight (244 against
-      // 299.5 us for W = 16 FP32 on the 96x96x48 plate with all loads issued
-      // first; 3 groups at 3 CTAs per SM measured best of 3 / 4 / 6 / 8
-      // groups at 1-3 CTAs per SM, 244-301 us)
+      // registers go to more groups of matrix loads in flight (with all loads
+      // issued first 22 % slower for W = 16 FP32 on the 96x96x48 plate; us
+      // there, CTAs per SM x groups: 3 x 3 208, 4 x 2 215, 4 x 1 237, 2 x 5 246)
 #pragma unroll
       for (int u = 0; u < U; u++)
         if (u < nu) {
@@ -842,7 +845,13 @@ void spmm_w(const CsrcDev &k, const T *X, T *Y, ColScalars *cols, BlockHeader *h
   ELX_REQUIRE(val != nullptr && k.sell_ptr != nullptr, ELX_ERR_STATE,
               "sliced node blocks missing for the block product");
   const bool d16 = k.sell_d16 != nullptr;
-  const int grid = std::max(1, std::min((k.nslices + SPC - 1) / SPC, k.max_grid));
+  // FP32: one resident wave.  A CTA that starts when another ends is out of step
+  // with its neighbours, and the x rows that it reads have left L1 and L2 (W =
+  // 16, 8 CTAs per SM / one wave: 243 / 207 us on the 96x96x48 plate, 55 / 48 on
+  // the HEXA8 cube 40^3, 32 / 23 on QUAD4 300x200; W = 1 and 2 the same).  FP64
+  // products wait for the pipe, and an even share counts more (W = 4, 40^3:
+  // 141 / 205 us).
+  const int passes = (k.nslices + SPC - 1) / SPC;
   // slot groups of matrix loads per step: ELX_SPMM_UNROLL, else the
   // autotuner's choice for this width, else three in FP32 and one in FP64
   // (FP64-pipe bound)
@@ -851,9 +860,16 @@ void spmm_w(const CsrcDev &k, const T *X, T *Y, ColScalars *cols, BlockHeader *h
   const int u = k.spmm_unroll > 0 ? k.spmm_unroll : tuned > 0 ? tuned : (sizeof(T) == 4 ? 3 : 1);
 #define ELX_SPMM(B_, DOT_, U_, LD_, D16_)                                                  \
   do {                                                                                      \
-    sell_spmm_kernel<T, B_, W, DOT_, false, U_, LD_, D16_><<<grid, kThreads, 0, st>>>(      \
-        k.nb, k.nslices, k.sell_ptr, k.sell_col, k.sell_d16, val, X, Y, cols, hdr, partials, \
-        counter, gate);                                                                     \
+    const auto f = sell_spmm_kernel<T, B_, W, DOT_, false, U_, LD_, D16_>;                  \
+    int per_sm = 1;                                                                         \
+    if (sizeof(T) == 4)                                                                     \
+      ELX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, kThreads, 0));     \
+    const int wave = per_sm * sm_count();                                                   \
+    const bool full = sizeof(T) == 4 && wave <= std::min(passes, k.max_grid);               \
+    const int grid = full ? wave : std::max(1, std::min(passes, k.max_grid));               \
+    f<<<grid, kThreads, 0, st>>>(k.nb, k.nslices, k.sell_ptr, k.sell_col, k.sell_d16, val,  \
+                                 X, Y, cols, hdr, partials, counter, gate,                  \
+                                 full ? per_sm : 1);                                        \
   } while (0)
 #define ELX_SPMM_LD(B_, DOT_, U_)           \
   if (ld && d16)                            \

@@ -224,3 +224,21 @@ def test_small_matrices(gpu_ctx, name):
     assert j["status"] == E.ERR_NO_CONVERGENCE
     z, j = gpu_ctx.solve(0 * b, tol=1e-12)
     assert j["status"] == 0 and j["iters"] == 0 and not z.any()
+
+
+# FP32 block products as one resident wave: 3 CTAs per SM on 152 SMs, 64, 32
+# and 16 block rows a CTA at W = 16, 8 and 4; matrices whose passes are below
+# the wave, equal to it at W = 16, above it, and several times it
+@pytest.mark.parametrize("nz", [23, 24, 25])
+@pytest.mark.parametrize("width", [4, 8, 16])
+def test_block_products_of_one_wave(gpu_ctx, nz, width):
+    s, ad, al, b = _system(gpu_ctx, M.box_hexa8(31, 37, nz))
+    assert s.neq == 3 * 32 * 38 * nz
+    B = np.random.default_rng(nz).standard_normal((b.size, width))
+    X, infos = gpu_ctx.solve_block(B, precision=E.PREC_MIXED, tol=1e-9, maxit=20000, width=width)
+    for i in infos:
+        assert i["status"] == 0 and i["norm_m_r"] <= 3.16 * i["conv"]
+    x_o, _ = O.pcg_omp(s, ad, al, B[:, -1], tol=1e-12, maxit=20000)
+    assert rel_inf(x_o, X[:, -1]) <= 1e-6
+    X2, _ = gpu_ctx.solve_block(B, precision=E.PREC_MIXED, tol=1e-9, maxit=20000, width=width)
+    assert np.array_equal(X, X2)

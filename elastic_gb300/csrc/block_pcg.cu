@@ -526,7 +526,9 @@ brel_start_kernel(int n, const double *__restrict__ b, const double *__restrict_
 // direction pass, which reads p anyway: 8 passes over the multi-vectors in an
 // iteration instead of 9 (87 MB each at 1,354,896 equations x 16).  Each
 // thread takes VC consecutive columns of a row (16-byte accesses), two rows in
-// flight.
+// flight.  From the last row to the first: the product has just written the
+// last rows of q, which are still in L2, and the direction pass then finds the
+// first rows of r there (61.8 -> 58.2 us, the direction 67.6 -> 66.4).
 template <int W>
 __global__ void __launch_bounds__(kThreads)
 brel_update_kernel(int n, const float *__restrict__ qv, const float *__restrict__ m32,
@@ -559,7 +561,7 @@ brel_update_kernel(int n, const float *__restrict__ qv, const float *__restrict_
   if (any) {
     size_t t = (size_t)blockIdx.x * kThreads + threadIdx.x;
     for (; t + step < ng; t += 2 * step) {
-      const size_t row0 = t / G, row1 = (t + step) / G;
+      const size_t row0 = n - 1 - t / G, row1 = n - 1 - (t + step) / G;
       const ColVec<float, VC> q0 = load_cols<float, VC>(qv + row0 * W + c0);
       const ColVec<float, VC> q1 = load_cols<float, VC>(qv + row1 * W + c0);
       ColVec<float, VC> r0 = load_cols<float, VC>(r + row0 * W + c0);
@@ -569,7 +571,7 @@ brel_update_kernel(int n, const float *__restrict__ qv, const float *__restrict_
       one(row1, r1, q1, m1);
     }
     if (t < ng) {
-      const size_t row = t / G;
+      const size_t row = n - 1 - t / G;
       const ColVec<float, VC> q0 = load_cols<float, VC>(qv + row * W + c0);
       ColVec<float, VC> r0 = load_cols<float, VC>(r + row * W + c0);
       one(row, r0, q0, m32[row]);
@@ -615,6 +617,25 @@ brel_update_kernel(int n, const float *__restrict__ qv, const float *__restrict_
   }
 }
 
+// x_lo is read and written once an iteration: streamed, it leaves L2 to the
+// other vectors (66.4 -> 64.8 us).
+template <int VC>
+__device__ __forceinline__ ColVec<float, VC> load_cs(const float *p) {
+  if constexpr (VC == 4) {
+    const float4 t = __ldcs(reinterpret_cast<const float4 *>(p));
+    return ColVec<float, VC>{{t.x, t.y, t.z, t.w}};
+  } else {
+    return load_cols<float, VC>(p);
+  }
+}
+template <int VC>
+__device__ __forceinline__ void store_cs(float *p, const ColVec<float, VC> &x) {
+  if constexpr (VC == 4)
+    __stcs(reinterpret_cast<float4 *>(p), make_float4(x.v[0], x.v[1], x.v[2], x.v[3]));
+  else
+    store_cols<float, VC>(p, x);
+}
+
 // p = M r + beta p and x_lo += alpha p (the old p) for the active columns.
 template <int W>
 __global__ void __launch_bounds__(kThreads)
@@ -646,7 +667,7 @@ brel_direction_kernel(int n, const float *__restrict__ r, const float *__restric
         pv.v[j] = rv.v[j] * mi + beta[j] * pv.v[j];
       }
     store_cols<float, VC>(p + row * W + c0, pv);
-    store_cols<float, VC>(xlo + row * W + c0, xv);
+    store_cs<VC>(xlo + row * W + c0, xv);
   };
   size_t t = (size_t)blockIdx.x * kThreads + threadIdx.x;
   for (; t + step < ng; t += 2 * step) {
@@ -655,8 +676,8 @@ brel_direction_kernel(int n, const float *__restrict__ r, const float *__restric
     ColVec<float, VC> p1 = load_cols<float, VC>(p + row1 * W + c0);
     const ColVec<float, VC> r0 = load_cols<float, VC>(r + row0 * W + c0);
     const ColVec<float, VC> r1 = load_cols<float, VC>(r + row1 * W + c0);
-    ColVec<float, VC> x0 = load_cols<float, VC>(xlo + row0 * W + c0);
-    ColVec<float, VC> x1 = load_cols<float, VC>(xlo + row1 * W + c0);
+    ColVec<float, VC> x0 = load_cs<VC>(xlo + row0 * W + c0);
+    ColVec<float, VC> x1 = load_cs<VC>(xlo + row1 * W + c0);
     const float m0 = m32[row0], m1 = m32[row1];
     one(row0, p0, x0, r0, m0);
     one(row1, p1, x1, r1, m1);
@@ -665,7 +686,7 @@ brel_direction_kernel(int n, const float *__restrict__ r, const float *__restric
     const size_t row = t / G;
     ColVec<float, VC> p0 = load_cols<float, VC>(p + row * W + c0);
     const ColVec<float, VC> r0 = load_cols<float, VC>(r + row * W + c0);
-    ColVec<float, VC> x0 = load_cols<float, VC>(xlo + row * W + c0);
+    ColVec<float, VC> x0 = load_cs<VC>(xlo + row * W + c0);
     one(row, p0, x0, r0, m32[row]);
   }
 }
@@ -824,6 +845,17 @@ int bgrid(size_t nw) {
   return (int)std::max<size_t>(1, std::min<size_t>(g, (size_t)grid_cap(8)));
 }
 
+// At most g blocks of f, and no more than are resident: blocks of a second wave
+// find a third of the GPU's places taken (brel_update_kernel, 40 registers, 6
+// of 8 blocks per SM resident: 58.2 us, one wave 51.3; brel_direction_kernel, 4
+// of 8: 64.8 and 63.7; W = 16 on the 96x96x48 plate).
+template <class F>
+int wave(F f, int g) {
+  int per = 1;
+  ELX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, kThreads, 0));
+  return std::min(g, per * sm_count());
+}
+
 // Y = K X on the sliced copy of precision T: one CTA pass per SPC slices,
 // at most the context's grid bound (the partial sums of the dots hold one
 // row per CTA).
@@ -918,9 +950,9 @@ void iteration_w(const CsrcDev &k, const BlockVecs &v, bool mixed, bool replacem
   } else {
     spmm_w<float, W>(k, v.p32, v.q32, v.cols, v.hdr, v.partials, cnt + 0, nullptr, true,
                      st);
-    brel_update_kernel<W><<<g, kThreads, 0, st>>>(n, v.q32, v.m32, v.r32, v.cols, v.hdr,
+    brel_update_kernel<W><<<wave(brel_update_kernel<W>, g), kThreads, 0, st>>>(n, v.q32, v.m32, v.r32, v.cols, v.hdr,
                                                   v.partials, cnt + 1);
-    brel_direction_kernel<W><<<g, kThreads, 0, st>>>(n, v.r32, v.m32, v.p32, v.xlo, v.cols,
+    brel_direction_kernel<W><<<wave(brel_direction_kernel<W>, g), kThreads, 0, st>>>(n, v.r32, v.m32, v.p32, v.xlo, v.cols,
                                                      v.hdr);
     if (replacement_point) {
       brel_accumulate_kernel<W><<<g, kThreads, 0, st>>>(n, v.x, v.xlo, v.cols, v.hdr);

@@ -2,6 +2,11 @@
 // the diagonal preconditioner of Solv.f:65-69 / Precond.f:22-45), and its
 // mixed-precision form: FP32 inner PCG inside FP64 iterative refinement.
 //
+// These launches solve what the resident ones (persist.cu, persist_mixed.cu)
+// do not take: matrices whose vectors do not fit a block's shared memory even
+// without the copies, partly fixed nodes in mixed precision, the tiled
+// product, and contexts whose memory budget has no room for the plan.
+//
 // One PCG iteration is three kernels that keep every scalar on the device,
 // so the host never waits inside the loop:
 //   1. q = K p (spmv.cu) fused with the dot (p, q); the last block to finish

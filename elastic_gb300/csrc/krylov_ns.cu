@@ -14,6 +14,9 @@
 //     projection + norm + rotations, one normalisation; then the
 //     back-substitution (one thread: k is small) and x += sum y_j g_j.
 //
+// GMRES cycles that fit a resident launch go through persist_gmres.cu instead;
+// these launches take the others (long restarts, the tiled product).
+//
 // Every kernel returns at once when the solve (or, inside a GMRES cycle, the
 // Arnoldi loop) has stopped, so a captured graph runs to its end harmlessly.
 // All reductions are the deterministic two-level ones of elx_reduce.cuh.

@@ -77,7 +77,7 @@ namespace {
 // The pack as one cooperative launch: a team of kPackThreads-thread blocks for
 // each load case, `steps` PCG iterations of every one (elx_persist.cuh).
 // Teams wait only for their own blocks, so load cases of every size go on at
-// their own pace; three blocks share an SM, and one team's arithmetic runs in
+// their own pace; four blocks share an SM, and one team's arithmetic runs in
 // another's waits.  A team has a block per kPackRows rows of its matrix,
 // whatever else is in the pack: a result is bitwise the same alone and in a
 // mix.  As three launches an iteration over all slots (48 us on a burst of 27

@@ -545,8 +545,8 @@ void launch_gather_epi64(const CsrcDev &k, int epi, const double *x, double *y, 
 // cudaMalloc is not allowed or would synchronise the device in the middle of
 // an asynchronous pipeline.  elx_spmv_dot_noalloc serves them: the caller
 // passes every input and output as device pointers, and the only scratch the
-// kernel needs -- one partial sum per block, the last-block ticket and the
-// scalar slot of the fused dot product -- lives in the file-scope array
+// kernel needs -- one partial sum per block and the last-block ticket --
+// lives in the file-scope array
 // below, which every GPU that loads this library holds until the process
 // exits.
 namespace elx {

@@ -219,9 +219,9 @@ int elx_block_tiling(elx_ctx *ctx, int32_t precision, int32_t *unroll);
  * reference runs one deck per process).  Requests are solved with the
  * reference's FP64 Jacobi PCG; structures are built on host threads while
  * the GPU works; a request is admitted when its device memory fits the HBM
- * budget; the PCG iterations of all admitted requests (every load case) run
- * as one packed set of kernels per iteration, each load case with its own
- * scalars and stopping test; requests join and leave between polls
+ * budget; the PCG iterations of all admitted requests run as packed launches
+ * of several iterations, each load case in its own team of blocks with its
+ * own scalars and stopping test; requests join and leave between polls
  * (continuous batching).  Requests of large_dofs equations or more are
  * instead solved whole, several at once on their own streams, by the block
  * PCG over all their load cases (see large_mode).
@@ -392,8 +392,7 @@ int elx_fortran_e(const double *x, int32_t n, int32_t w, int32_t d, int32_t e, c
  *                   order), e.g. from a counting sort of ja;
  *   x (neq), y (neq), xy (1 double); stream: a cudaStream_t (NULL = default).
  * Limit: neq <= 1048576 (ELX_ERR_ARG above; nothing is launched).  The
- * scratch (one partial sum per 64 rows, a ticket and a scalar slot, about
- * 130 KB) is a static device array that every GPU loading this library
+ * scratch (the blocks' partial sums and a ticket, about 130 KB) is a static device array that every GPU loading this library
  * holds until the process exits.  The first call on a device looks up that
  * array's device address (with the device current): make that first call
  * before any stream capture.  The address is that of the device's primary

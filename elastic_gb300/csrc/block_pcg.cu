@@ -301,8 +301,8 @@ sell_spmm_kernel(int nb, int nslices, const int32_t *__restrict__ sell_ptr,
   // Passes of SPC slices, every gridDim.x-th for this CTA (contiguous runs of
   // passes per CTA lose the x rows that the CTAs share in L2).  CTAs b,
   // b + SMs, b + 2 SMs, which one SM holds, take neighbouring passes: six
-  // slices then gather 918 distinct x rows instead of 1,510 and the SM's L1
-  // holds them (214 -> 208 us, W = 16 FP32 on the 96x96x48 plate).
+  // slices then gather 918 distinct x rows instead of 1,510 (L1 hits 58 -> 60 %,
+  // 214 -> 208 us, W = 16 FP32 on the 96x96x48 plate).
   const int sms = gridDim.x / per_sm;
   const int first = (blockIdx.x % sms) * per_sm + blockIdx.x / sms;
   for (int sl = first * SPC + (int)threadIdx.x / (R * G); sl < nslices;
@@ -877,9 +877,9 @@ void spmm_w(const CsrcDev &k, const T *X, T *Y, ColScalars *cols, BlockHeader *h
   ELX_REQUIRE(val != nullptr && k.sell_ptr != nullptr, ELX_ERR_STATE,
               "sliced node blocks missing for the block product");
   const bool d16 = k.sell_d16 != nullptr;
-  // FP32: one resident wave.  A CTA that starts when another ends is out of step
-  // with its neighbours, and the x rows that it reads have left L1 and L2 (W =
-  // 16, 8 CTAs per SM / one wave: 243 / 207 us on the 96x96x48 plate, 55 / 48 on
+  // FP32: one resident wave.  8 CTAs per SM, three of them resident, are 2.67
+  // waves, the last two thirds full, and all CTAs have the same work (W = 16, 8
+  // per SM / one wave: 243 / 207 us on the 96x96x48 plate, 55 / 48 on
   // the HEXA8 cube 40^3, 32 / 23 on QUAD4 300x200; W = 1 and 2 the same).  FP64
   // products wait for the pipe, and an even share counts more (W = 4, 40^3:
   // 141 / 205 us).

@@ -31,6 +31,22 @@ struct Error {
     if (!(cond)) throw ::elx::Error{(code), (what)};                        \
   } while (0)
 
+// Lets launches of f have all the dynamic shared memory that a block can.  The
+// limit belongs to the kernel, not to a launch: set to each launch's own size,
+// one thread's small matrix would lower it under another thread's large one.
+template <class F>
+cudaError_t allow_shared(F *f) {
+  cudaFuncAttributes at;
+  int dev = 0, limit = 0;
+  cudaError_t e = cudaFuncGetAttributes(&at, f);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              limit - (int)at.sharedSizeBytes);
+}
+
 // ------------------------------------------------------- device buffers
 // Owning device allocation; every allocation of a context goes through
 // Ctx::alloc so that the HBM budget is enforced in one place.

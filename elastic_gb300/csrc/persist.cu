@@ -80,7 +80,7 @@ void launch(const PersistArgs &a, int grid, bool in_smem, int start, int steps, 
   const void *f = in_smem ? (const void *)pcg_persist_kernel<B, NC, true>
                           : (const void *)pcg_persist_kernel<B, NC, false>;
   const size_t bytes = smem_of<B, NC>(in_smem, a.rows, a.slices);
-  ELX_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  ELX_CUDA(allow_shared(f));
   PersistArgs arg = a;
   void *args[] = {&arg, &start, &steps};
   ELX_CUDA(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(kPT), args, bytes, st));
@@ -103,8 +103,7 @@ cudaError_t cluster_call(const PersistArgs &a, int n, int start, int steps, cuda
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)cfg.dynamicSmemBytes);
+  cudaError_t e = allow_shared(f);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;

@@ -368,7 +368,7 @@ void gmres_persist_cycle(elx_ctx *c, int k, double *basis, double *xr, void *dot
                          : (const void *)elx::gmres_persist_kernel<2>;
   const size_t bytes = B == 3 ? elx::gmres_smem<3>(a.rows, a.slices, k)
                               : elx::gmres_smem<2>(a.rows, a.slices, k);
-  ELX_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  ELX_CUDA(elx::allow_shared(f));
   void *args[] = {&a};
   ELX_CUDA(cudaLaunchCooperativeKernel(f, dim3(c->persist_grid), dim3(elx::kGT), args, bytes,
                                        c->stream));

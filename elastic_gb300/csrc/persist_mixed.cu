@@ -306,7 +306,7 @@ template <int B, bool LD, bool D16>
 void launch_mixed(const MixedArgs &a, int grid, int replace_every, int steps, cudaStream_t st) {
   const void *f = (const void *)mixed_persist_kernel<B, LD, D16>;
   const size_t bytes = mixed_smem<B>(a.rows, a.slices);
-  ELX_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  ELX_CUDA(allow_shared(f));
   MixedArgs arg = a;
   void *args[] = {&arg, &replace_every, &steps};
   ELX_CUDA(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(kMT), args, bytes, st));

@@ -9,6 +9,8 @@ matrix and a load whose norms differ by many orders, and a load with a NaN.
 Bars: the solver tests' (displacements within 1e-10 of the oracle, iterations
 within 2); a load scaled by a power of two gives the same iterates scaled
 exactly."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -242,3 +244,36 @@ def test_block_products_of_one_wave(gpu_ctx, nz, width):
     assert rel_inf(x_o, X[:, -1]) <= 1e-6
     X2, _ = gpu_ctx.solve_block(B, precision=E.PREC_MIXED, tol=1e-9, maxit=20000, width=width)
     assert np.array_equal(X, X2)
+
+
+@pytest.mark.parametrize("kind", ["fp64", "mixed", "gmres"])
+def test_threads_with_matrices_of_different_sizes(built_lib, kind):
+    """The same kernel launched by several threads for blocks of 3, 12 and 66 KB
+    of vectors: the kernel's shared memory limit is no launch's own."""
+    args = {"fp64": dict(maxit=4), "mixed": dict(precision=E.PREC_MIXED, maxit=4),
+            "gmres": dict(solver=E.SOLVER_GMRES, ngram=4, maxit=1)}[kind]
+    errors = []
+
+    def work(n, count):
+        try:
+            with E.Context(device=0) as ctx:
+                m = M.box_hexa8(n, n, n)
+                ctx.set_mesh(m)
+                ctx.build_structure(True)
+                b, _ = E.pload(m, ctx.structure().id)
+                ctx.assemble(None, b)
+                x0 = None
+                for _ in range(count):
+                    x, i = ctx.solve(b, tol=1e-13, raise_on_error=False, **args)
+                    assert i["status"] in (0, E.ERR_NO_CONVERGENCE) and x.any()
+                    assert x0 is None or np.array_equal(x, x0)
+                    x0 = x
+        except Exception as e:  # noqa: BLE001 - reported by the main thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=a) for a in ((12, 300), (20, 200), (40, 60))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors

@@ -872,13 +872,21 @@ bool solve_block_persist(elx_ctx *c, int nrhs, double tol, int maxit, int width,
   if (c->persist_vec.bytes < 5 * n * nc * 8) c->alloc(c->persist_vec, 5 * n * nc * 8);
   double *work = c->persist_vec.as<double>(), *bs = work + 3 * n * nc, *xs = bs + n * nc;
   const int chunks = (nrhs + nc - 1) / nc;
+  // the caller's two arrays may share memory: the diagnostics read b after x is
+  // written, so b is set aside, and x may lie ahead of b, so chunks then go
+  // from the last to the first
+  const uintptr_t ab = (uintptr_t)b, ax = (uintptr_t)x, len = 8 * n * nrhs;
+  const bool shared = ab < ax + len && ax < ab + len;
+  const bool stage = !device_ptrs || shared;
   int status = ELX_OK;
-  for (int k = 0; k < chunks; k++) {
+  for (int i = 0; i < chunks; i++) {
+    const int k = shared && ax > ab ? chunks - 1 - i : i;
     const int c0 = (int)((int64_t)nrhs * k / chunks), m = (int)((int64_t)nrhs * (k + 1) / chunks) - c0;
-    const double *bd = device_ptrs ? b + (size_t)c0 * n : bs;
+    const double *bd = stage ? bs : b + (size_t)c0 * n;
     double *xd = device_ptrs ? x + (size_t)c0 * n : xs;
-    if (!device_ptrs)
-      ELX_CUDA(cudaMemcpyAsync(bs, b + (size_t)c0 * n, n * m * 8, cudaMemcpyHostToDevice,
+    if (stage)
+      ELX_CUDA(cudaMemcpyAsync(bs, b + (size_t)c0 * n, n * m * 8,
+                               device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                                c->stream));
     elx::PersistCol cols[elx::kGridCols];
     persist_solve(c, m, tol, maxit, bd, xd, work,

@@ -480,10 +480,7 @@ void pcg64(elx_ctx *c, double tol, int maxit, elx_info *info) {
   build_preconditioner(c);
   elx::PcgScalars last{};
   if (ensure_persist(c)) {
-    // x's place holds x between launches too; r and p are the context's
     elx::PersistCol col;
-    const size_t n = (size_t)persist_rows(c);
-    if (c->persist_vec.bytes < 3 * n * 8) c->alloc(c->persist_vec, 3 * n * 8);
     persist_solve(c, 1, tol, maxit, c->b.as<double>(), c->xs.as<double>(),
                   c->persist_vec.as<double>(), c->batch_gate ? kPersistGatedSteps : kPersistSteps,
                   &col);
@@ -852,7 +849,8 @@ int autotune_block_width(elx_ctx *c, bool mixed, double *times_us = nullptr) {
 
 // FP64 load cases by the cooperative PCG, up to nc columns a launch (persist.cu):
 // the columns share the matrix reads and the waits, and none pads a block to a
-// width.  False: the matrix is too large for it.
+// width.  False: the matrix is too large for it, or the memory budget has no
+// room for the vectors of four columns.
 bool solve_block_persist(elx_ctx *c, int nrhs, double tol, int maxit, int width, const double *b,
                          double *x, elx_info *infos, bool device_ptrs) {
   // 3x3 blocks are FP64-bound either way: krylov's product over 8 or 16 columns
@@ -863,13 +861,15 @@ bool solve_block_persist(elx_ctx *c, int nrhs, double tol, int maxit, int width,
   if (c->s.bsize == 3 && nrhs > elx::kGridCols && 21 * nrhs > 20 * ((nrhs + w - 1) / w * w))
     return false;
   const int want = std::min(nrhs, width > 0 ? width : elx::kGridCols);
-  const int nc = persist_columns(c, want);
-  if (nc < std::min(want, 4)) return false;
-  auto t0 = std::chrono::steady_clock::now();
-  build_preconditioner(c);
+  const int least = std::min(want, 4);
   const size_t n = (size_t)c->s.neq;
   // per column: three work vectors, b and x
-  if (c->persist_vec.bytes < 5 * n * nc * 8) c->alloc(c->persist_vec, 5 * n * nc * 8);
+  int nc = persist_columns(c, want);
+  while (nc >= least && !persist_vectors(c, 5 * n * nc * 8))
+    nc = nc > least ? persist_columns(c, nc - 1) : 0;
+  if (nc < least) return false;
+  auto t0 = std::chrono::steady_clock::now();
+  build_preconditioner(c);
   double *work = c->persist_vec.as<double>(), *bs = work + 3 * n * nc, *xs = bs + n * nc;
   const int chunks = (nrhs + nc - 1) / nc;
   // the caller's two arrays may share memory: the diagnostics read b after x is

@@ -96,8 +96,9 @@ struct elx_ctx {
   int32_t *h_flags = nullptr;         // pinned
 
   // cooperative PCG (persist.cu): blocks (0: not planned, -1: not used), their
-  // slices and shared words, the vectors between launches, and per number of
-  // columns where the vectors live (0: too many, 1: L2, 2: shared memory)
+  // slices and shared words, the vectors between launches (those of one column
+  // at least, as long as there is a plan), and per number of columns where the
+  // vectors live (0: too many, 1: L2, 2: shared memory)
   DBuf persist_cta, persist_sync, persist_vec;
   // its matrix when some nodes are only partly fixed (Structure::p_*)
   DBuf p_ptr, p_col, p_off, p_eq, p_val;
@@ -243,6 +244,7 @@ void release_block(elx_ctx *c);
 // Cooperative PCG (persist.cu).
 bool ensure_persist(elx_ctx *c);
 int persist_columns(elx_ctx *c, int want);
+bool persist_vectors(elx_ctx *c, size_t bytes);
 int persist_rows(const elx_ctx *c);
 bool mixed_persist(elx_ctx *c);
 bool ensure_gmres_persist(elx_ctx *c, int k);

@@ -164,6 +164,19 @@ int persist_rows(const elx_ctx *c) {
   return c->use_blocks ? c->s.nb * c->s.bsize : c->s.p_nb * c->s.p_bsize;
 }
 
+namespace {
+
+// Gives the plan's memory back; the launches are used until the next structure.
+void drop_persist(elx_ctx *c) {
+  for (DBuf *d : {&c->persist_cta, &c->persist_sync, &c->persist_vec, &c->p_ptr, &c->p_col,
+                  &c->p_off, &c->p_eq, &c->p_val})
+    c->release(*d);
+  c->have_padded = false;
+  c->persist_grid = -1;
+}
+
+}  // namespace
+
 // Plans the cooperative PCG of the context's matrix (once per structure).
 // False: krylov.cu's launches are used.
 bool ensure_persist(elx_ctx *c) {
@@ -217,10 +230,7 @@ bool ensure_persist(elx_ctx *c) {
       }
     } catch (const Error &e) {
       if (e.code != ELX_ERR_OOM) throw;
-      // a memory budget without room for it
-      for (DBuf *d : {&c->persist_cta, &c->persist_sync, &c->persist_vec, &c->p_ptr, &c->p_col,
-                      &c->p_off, &c->p_eq, &c->p_val})
-        c->release(*d);
+      drop_persist(c);  // a memory budget without room for it
       return false;
     }
     c->sync();
@@ -248,6 +258,23 @@ int persist_columns(elx_ctx *c, int want) {
   int nc = std::min(want, elx::kGridCols);
   while (nc > 0 && !c->persist_mode[nc]) nc--;
   return nc;
+}
+
+// Makes the plan's vectors `bytes` long.  False: the memory budget has no room
+// for that; one column's are there again (alloc gives the old ones back first),
+// or there is no plan any more.
+bool persist_vectors(elx_ctx *c, size_t bytes) {
+  if (c->persist_vec.bytes >= bytes) return true;
+  for (size_t n : {bytes, 3 * 8 * (size_t)persist_rows(c)}) {
+    try {
+      c->alloc(c->persist_vec, n);
+      return n == bytes;
+    } catch (const Error &e) {
+      if (e.code != ELX_ERR_OOM) throw;
+    }
+  }
+  drop_persist(c);
+  return false;
 }
 
 // PCG of nc columns b -> x (device, neq x nc), at most `steps` iterations a

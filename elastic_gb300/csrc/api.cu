@@ -647,30 +647,34 @@ void bicgstab64(elx_ctx *c, double tol, int maxit, elx_info *info, bool plain) {
 void gmres64(elx_ctx *c, int kdim, double tol, int maxit, elx_info *info) {
   auto t0 = std::chrono::steady_clock::now();
   require(kdim >= 1 && kdim <= kMaxGmresK, ELX_ERR_ARG, "GMRES restart length out of range");
+  if (!c->gstate.p) c->alloc(c->gstate, sizeof(elx::GmresState));
   bool persist = ensure_gmres_persist(c, kdim);
+  size_t n = 0;
   // the basis by equations, or by rows of the sliced matrix
-  size_t n = persist ? (size_t)persist_rows(c) : (size_t)c->s.neq;
-  if (c->gmres_k == kdim && c->gbasis.p) {
+  auto rows = [&] { return persist ? (size_t)persist_rows(c) : (size_t)c->s.neq; };
+  if (c->gmres_k == kdim && c->gbasis.p && (persist || !c->gmres_persist)) {
     persist = c->gmres_persist;
-    n = persist ? (size_t)persist_rows(c) : (size_t)c->s.neq;
+    n = rows();
   } else {
     if (c->gmres_graph) cudaGraphExecDestroy(c->gmres_graph);
     c->gmres_graph = nullptr;
     c->gmres_k = 0;
-    try {
+    auto take = [&] {
+      n = rows();
       c->alloc(c->gbasis, n * 8 * (size_t)(kdim + 1));
       c->alloc(c->garrays,
                persist ? gmres_persist_bytes(kdim) : elx::gmres_array_doubles(kdim) * 8);
+    };
+    try {
+      take();
     } catch (const Error &e) {
       if (e.code != ELX_ERR_OOM || !persist) throw;
-      // a memory budget without room for the cooperative cycle's words
+    }
+    if (persist && c->persist_grid <= 0) {  // the plan made way
       persist = false;
-      n = (size_t)c->s.neq;
-      c->alloc(c->gbasis, n * 8 * (size_t)(kdim + 1));
-      c->alloc(c->garrays, elx::gmres_array_doubles(kdim) * 8);
+      take();
     }
     c->gmres_persist = persist;
-    if (!c->gstate.p) c->alloc(c->gstate, sizeof(elx::GmresState));
     c->gmres_k = kdim;
   }
   build_preconditioner(c);

@@ -127,6 +127,26 @@ struct elx_ctx {
   void alloc(DBuf &d, size_t bytes) {
     release(d);
     if (bytes == 0) bytes = 16;
+    try {
+      take(d, bytes);
+    } catch (const Error &) {
+      // the resident solvers have launches to fall back on: their plan makes
+      // way for what does not fit beside it
+      if (persist_grid <= 0 || &d == &persist_vec) throw;
+      drop_persist(0);
+      take(d, bytes);
+    }
+  }
+  // Gives the resident solvers' plan back; `state`: 0 to plan again at the next
+  // solve, -1 for the launches until the next structure.
+  void drop_persist(int state) {
+    for (DBuf *d : {&persist_cta, &persist_sync, &persist_vec, &p_ptr, &p_col, &p_off, &p_eq,
+                    &p_val})
+      release(*d);
+    have_padded = false;
+    persist_grid = state;
+  }
+  void take(DBuf &d, size_t bytes) {
     if (budget > 0 && used + (int64_t)bytes > budget)
       throw Error{ELX_ERR_OOM, "HBM budget exceeded: need " + std::to_string(bytes) +
                                    " more bytes, " + std::to_string(budget - used) + " left"};

@@ -164,19 +164,6 @@ int persist_rows(const elx_ctx *c) {
   return c->use_blocks ? c->s.nb * c->s.bsize : c->s.p_nb * c->s.p_bsize;
 }
 
-namespace {
-
-// Gives the plan's memory back; the launches are used until the next structure.
-void drop_persist(elx_ctx *c) {
-  for (DBuf *d : {&c->persist_cta, &c->persist_sync, &c->persist_vec, &c->p_ptr, &c->p_col,
-                  &c->p_off, &c->p_eq, &c->p_val})
-    c->release(*d);
-  c->have_padded = false;
-  c->persist_grid = -1;
-}
-
-}  // namespace
-
 // Plans the cooperative PCG of the context's matrix (once per structure).
 // False: krylov.cu's launches are used.
 bool ensure_persist(elx_ctx *c) {
@@ -230,7 +217,7 @@ bool ensure_persist(elx_ctx *c) {
       }
     } catch (const Error &e) {
       if (e.code != ELX_ERR_OOM) throw;
-      drop_persist(c);  // a memory budget without room for it
+      c->drop_persist(-1);  // a memory budget without room for it
       return false;
     }
     c->sync();
@@ -273,7 +260,7 @@ bool persist_vectors(elx_ctx *c, size_t bytes) {
       if (e.code != ELX_ERR_OOM) throw;
     }
   }
-  drop_persist(c);
+  c->drop_persist(-1);
   return false;
 }
 

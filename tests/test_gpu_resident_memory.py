@@ -68,3 +68,22 @@ def test_block_solve_that_does_not_fit_leaves_the_context_usable(system):
         y, i = ctx.solve(b, solver=E.SOLVER_GMRES, ngram=2, tol=1e-11, maxit=1, raise_on_error=False)
         assert i["status"] in (E.OK, E.ERR_NO_CONVERGENCE) and np.isfinite(y).all() and y.any()
         assert rel_inf(x, ctx.solve(b, tol=1e-11)[0]) <= 1e-9
+
+
+def test_other_solvers_take_the_place_of_the_plan(system):
+    """Budgets that hold one solver's vectors but not the plan beside them."""
+    base, n, b, x = system
+    ctx, _, _ = _start(base + 24 * n + (64 << 10))
+    with ctx:
+        assert rel_inf(x, ctx.solve(b, tol=1e-11)[0]) <= 1e-9
+        y, _ = ctx.solve(b, solver=E.SOLVER_BICGSTAB, tol=1e-11)  # 16 n bytes
+        assert rel_inf(x, y) <= 1e-8
+        assert rel_inf(x, ctx.solve(b, tol=1e-11)[0]) <= 1e-9
+    k = 40
+    ctx, _, _ = _start(base + 8 * n * (k + 1) + (128 << 10))
+    with ctx:
+        assert rel_inf(x, ctx.solve(b, tol=1e-11)[0]) <= 1e-9
+        y, _ = ctx.solve(b, solver=E.SOLVER_GMRES, ngram=k, tol=1e-11)
+        assert rel_inf(x, y) <= 1e-8
+        y2, _ = ctx.solve(b, solver=E.SOLVER_GMRES, ngram=k, tol=1e-11)
+        assert np.array_equal(y, y2)

@@ -35,6 +35,7 @@
 // warps is summed by its first warp and the heads of the following ones, in
 // warp order, so results do not depend on timing.
 #include <algorithm>
+#include <cstdlib>
 
 #include "elx_context.h"
 #include "elx_persist.cuh"
@@ -117,6 +118,25 @@ cudaError_t cluster_call(int B, const PersistArgs &a, int n, int start, int step
                 : cluster_call<2>(a, n, start, steps, st, fit);
 }
 
+// A block of it has an SM to itself, as the resident kernels' blocks have.
+__global__ void residency_kernel() {}
+
+// Whether `grid` blocks of one per SM can run at the same time: not in a process
+// that has a part of the GPU's SMs, which the occupancy calls do not know of.
+bool resident_together(int grid, cudaStream_t st) {
+  cudaFuncAttributes at;
+  ELX_CUDA(allow_shared(residency_kernel));
+  ELX_CUDA(cudaFuncGetAttributes(&at, residency_kernel));
+  const cudaError_t e =
+      cudaLaunchCooperativeKernel((const void *)residency_kernel, dim3(grid), dim3(kPT), nullptr,
+                                  at.maxDynamicSharedSizeBytes, st);
+  if (e == cudaSuccess) return true;
+  cudaGetLastError();
+  ELX_REQUIRE(e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported, ELX_ERR_CUDA,
+              cudaGetErrorString(e));
+  return false;
+}
+
 #define ELX_NC_DISPATCH(nc, call)                             \
   switch (nc) {                                               \
     case 1: call(1); break;                                   \
@@ -174,7 +194,10 @@ bool ensure_persist(elx_ctx *c) {
     c->persist_grid = -1;
     const std::vector<int32_t> &ptr = padded ? s.p_ptr : s.sell_ptr;
     const int nslices = (int)ptr.size() - 1, B = padded ? s.p_bsize : s.bsize;
-    const int grid = std::min({elx::sm_count(), elx::kGridMaxBlocks, nslices});
+    const char *env = getenv("ELX_RESIDENT_BLOCKS");
+    const int want = env ? std::max(1, atoi(env)) : elx::sm_count();
+    const int grid = std::min({want, elx::kGridMaxBlocks, nslices});
+    if (!elx::resident_together(grid, c->stream)) return false;
     std::vector<int32_t> cuts = elx::persist_cuts(ptr, grid);
     const int cl = std::min(elx::kClusterBlocks, nslices);
     const std::vector<int32_t> ccuts = elx::persist_cuts(ptr, cl);

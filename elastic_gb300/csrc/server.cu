@@ -91,6 +91,7 @@ constexpr int kPackRows = 768;  // five vectors of it in shared memory: 37 KB a 
 
 __global__ void __launch_bounds__(kPackThreads, kPackPerSm)
 packed_pcg_kernel(const PackSlot *d, int nslots, int steps, uint64_t epoch) {
+  if (nslots == 0) return;
   int lo = 0, hi = nslots - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -1083,7 +1084,23 @@ int elx_server_create(elx_server **out, const elx_server_opts *opts) {
                                                       elx::kPackThreads, elx::pack_smem());
   if (e == cudaSuccess)
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, sv->device);
-  sv->pack_capacity = per_sm * sms;
+  const char *res_env = std::getenv("ELX_RESIDENT_BLOCKS");
+  sv->pack_capacity = res_env ? std::max(1, std::atoi(res_env)) : per_sm * sms;
+  if (e == cudaSuccess) {
+    // a process that has a part of the GPU's SMs cannot run that many at once:
+    // the packed launches then
+    const elx::PackSlot *none = nullptr;
+    int n = 0, st = 0;
+    uint64_t ep = 0;
+    void *args[] = {&none, &n, &st, &ep};
+    e = cudaLaunchCooperativeKernel((const void *)elx::packed_pcg_kernel, dim3(sv->pack_capacity),
+                                    dim3(elx::kPackThreads), args, elx::pack_smem(), sv->stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+      (void)cudaGetLastError();
+      sv->pack_capacity = 0;
+      e = cudaSuccess;
+    }
+  }
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sv->ev_poll, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     (void)cudaGetLastError();

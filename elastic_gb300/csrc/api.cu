@@ -369,14 +369,19 @@ void capture_pcg_graph(elx_ctx *c) {
 
 // Launches batches of `size` iterations (`launch`) until the scalars' stopping
 // flag is set (two batches in flight; the host reads the flag of the older one).
+// With `waits` the batches can give up in a bounded wait of theirs (flags[2]):
+// no more are launched then, and the caller's check of the flag reports it.
 template <class F>
-elx::PcgScalars run_batches(elx_ctx *c, int size, int maxit, F launch) {
+elx::PcgScalars run_batches(elx_ctx *c, int size, int maxit, F launch, bool waits = false) {
   elx::PcgScalars *d_sc = c->scal.as<elx::PcgScalars>();
   int launched = 0, checked = 0;
   auto launch_batch = [&](int slot) {
     launch();
     ELX_CUDA(cudaMemcpyAsync(&c->h_scal[slot], d_sc, sizeof(elx::PcgScalars),
                              cudaMemcpyDeviceToHost, c->stream));
+    if (waits)
+      ELX_CUDA(cudaMemcpyAsync(c->h_wait + slot, c->flags.as<int32_t>() + 2, sizeof(int32_t),
+                               cudaMemcpyDeviceToHost, c->stream));
     ELX_CUDA(cudaEventRecord(c->ev[slot], c->stream));
   };
   const int max_batches = maxit / size + 2;
@@ -390,7 +395,7 @@ elx::PcgScalars run_batches(elx_ctx *c, int size, int maxit, F launch) {
     const int slot = checked & 1;
     ELX_CUDA(cudaEventSynchronize(c->ev[slot]));
     checked++;
-    if (c->h_scal[slot].done) break;
+    if (c->h_scal[slot].done || (waits && c->h_wait[slot])) break;
     if (launched >= max_batches) break;  // guard; the kernels stop at maxit themselves
     launch_batch(launched & 1);
     launched++;
@@ -434,16 +439,18 @@ void spmv64(elx_ctx *c, const double *x, double *y) {
   c->launches += c->spmv_kind == elx::kSpmvTiled ? 2 : 1;
 }
 
-// A bounded device wait of the pipelined (tiled) SpMV that gave up leaves
-// its code in flags[2]; reported, and cleared, as ELX_ERR_TIMEOUT.
-void check_pipe_waits(elx_ctx *c) {
+// A bounded device wait of the pipelined (tiled) SpMV or of a resident mixed or
+// GMRES launch that gave up leaves its code in flags[2]; reported, and cleared,
+// as ELX_ERR_TIMEOUT.
+void check_pipe_waits(elx_ctx *c,
+                      const char *what = "a bounded device wait of the SpMV pipeline gave up") {
   ELX_CUDA(cudaMemcpyAsync(c->h_flags + 2, c->flags.as<int32_t>() + 2, sizeof(int32_t),
                            cudaMemcpyDeviceToHost, c->stream));
   c->sync();
   if (c->h_flags[2] != 0) {
     ELX_CUDA(cudaMemsetAsync(c->flags.as<int32_t>() + 2, 0, sizeof(int32_t), c->stream));
     c->sync();
-    throw Error{ELX_ERR_TIMEOUT, "a bounded device wait of the SpMV pipeline gave up"};
+    throw Error{ELX_ERR_TIMEOUT, what};
   }
 }
 
@@ -547,8 +554,9 @@ void pcg_mixed(elx_ctx *c, double tol, int maxit, elx_info *info) {
   c->launches += 2;
   elx::PcgScalars last =
       persist ? run_batches(c, kPersistSteps, maxit,
-                            [&] { mixed_persist_steps(c, kReplaceEvery, kPersistSteps); })
+                            [&] { mixed_persist_steps(c, kReplaceEvery, kPersistSteps); }, true)
               : run_batches(c, c->pcg32_graph, 3 + 3.0 / kReplaceEvery, maxit);
+  if (persist) check_pipe_waits(c, kResidentWait);
   // fold the last FP32 piece (zero unless maxit stopped the iteration)
   elx::launch_refine_accumulate(n, c->xs.as<double>(), c->x32.as<float>(), false, c->stream);
   c->launches += 1;
@@ -714,7 +722,7 @@ void gmres64(elx_ctx *c, int kdim, double tol, int maxit, elx_info *info) {
     if (persist) {
       gmres_persist_cycle(c, kdim, c->gbasis.as<double>(), c->persist_vec.as<double>(),
                           c->garrays.p);
-      check_pipe_waits(c);
+      check_pipe_waits(c, kResidentWait);
       continue;
     }
     ELX_CUDA(cudaGraphLaunch(c->gmres_graph, c->stream));
@@ -1284,10 +1292,10 @@ int elx_create(elx_ctx **out, const elx_opts *opts) {
     c->pool = elx::device_pool(c->device);
     elx::pool_users(c->device, 1);
     c->pool_user = true;
-    // h_scal (2 PcgScalars), h_diag (8 doubles), h_flags (4 ints) in one
-    // recycled pinned block
+    // h_scal (2 PcgScalars), h_diag (8 doubles), h_flags (4 ints), h_state,
+    // h_wait (2 ints) in one recycled pinned block
     static_assert(2 * sizeof(elx::PcgScalars) + 8 * sizeof(double) + 4 * sizeof(int32_t) +
-                          12 * sizeof(elx::PersistCol) <=
+                          2 * sizeof(elx::PersistState) + 2 * sizeof(int32_t) <=
                       elx::kPinnedBlock,
                   "pinned block too small");
     c->pinned = elx::pinned_block_get();
@@ -1295,8 +1303,9 @@ int elx_create(elx_ctx **out, const elx_opts *opts) {
     c->h_scal = reinterpret_cast<elx::PcgScalars *>(pb);
     c->h_diag = reinterpret_cast<double *>(pb + 2 * sizeof(elx::PcgScalars));
     c->h_flags = reinterpret_cast<int32_t *>(pb + 2 * sizeof(elx::PcgScalars) + 8 * sizeof(double));
-    c->h_cols = reinterpret_cast<elx::PersistCol *>(pb + 2 * sizeof(elx::PcgScalars) +
-                                                    8 * sizeof(double) + 4 * sizeof(int32_t));
+    c->h_state = reinterpret_cast<elx::PersistState *>(pb + 2 * sizeof(elx::PcgScalars) +
+                                                       8 * sizeof(double) + 4 * sizeof(int32_t));
+    c->h_wait = reinterpret_cast<int32_t *>(c->h_state + 2);
     for (auto &e : c->ev) ELX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     for (auto &e : c->ev_t) ELX_CUDA(cudaEventCreate(&e));
   });

@@ -109,7 +109,8 @@ struct elx_ctx {
   // the same by one cluster of blocks for one column (0: not used; its cuts
   // follow the grid's in persist_cta)
   int cluster_grid = 0, cluster_rows = 0, cluster_slices = 0;
-  elx::PersistCol *h_cols = nullptr;  // pinned, 2 slots of 6
+  elx::PersistState *h_state = nullptr;  // pinned, 2 slots
+  int32_t *h_wait = nullptr;             // pinned, 2 slots of flags[2]
 
   int64_t launches = 0;  // kernels of this library launched by this context
 
@@ -262,6 +263,7 @@ void assemble_resident(elx_ctx *c);
 void build_preconditioner(elx_ctx *c);
 void release_block(elx_ctx *c);
 // Cooperative PCG (persist.cu).
+constexpr const char *kResidentWait = "a bounded device wait of the resident solver gave up";
 bool ensure_persist(elx_ctx *c);
 int persist_columns(elx_ctx *c, int want);
 bool persist_vectors(elx_ctx *c, size_t bytes);

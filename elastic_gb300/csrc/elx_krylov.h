@@ -38,6 +38,14 @@ struct PersistCol {
   double d, conv;
   int32_t iters, done, status, started;
 };
+// The columns and the word of a wait that ran out, read together by the host.
+struct PersistState {
+  PersistCol col[kGridCols];
+  int32_t err, pad[3];
+};
+// ELX_GRID_STALL_TEST=1: the resident launches wait for a block too many (tests
+// of the timeouts; read at every solve).
+int grid_stall();
 // Cuts slices into one run per block with equal numbers of slot groups.
 std::vector<int32_t> persist_cuts(const std::vector<int32_t> &sell_ptr, int grid);
 

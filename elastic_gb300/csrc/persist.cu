@@ -56,7 +56,7 @@ constexpr double kClusterGain = 2800;
 template <int B, int NC, bool SMEM>
 __global__ void __launch_bounds__(kPT, 1)
 pcg_persist_kernel(PersistArgs a, int start, int steps) {
-  persist_pcg<kPT, B, NC, SMEM>(a, grid::Team{(int)blockIdx.x, (int)gridDim.x}, start, steps, 0);
+  persist_pcg<kPT, B, NC, SMEM>(a, grid::Team((int)blockIdx.x, (int)gridDim.x, a.stall), start, steps, 0);
 }
 
 // The same by one cluster: grid::Cluster's sums and barrier.
@@ -158,6 +158,11 @@ size_t smem_bytes(int B, int nc, bool in_smem, int rows, int slices) {
 
 }  // namespace
 
+int grid_stall() {
+  const char *env = getenv("ELX_GRID_STALL_TEST");
+  return env && atoi(env) == 1 ? 1 : 0;
+}
+
 std::vector<int32_t> persist_cuts(const std::vector<int32_t> &sell_ptr, int grid) {
   const int nslices = (int)sell_ptr.size() - 1;
   std::vector<int32_t> t(grid + 1, 0);
@@ -229,7 +234,7 @@ bool ensure_persist(elx_ctx *c) {
     }
     try {
       c->upload(c->persist_cta, cuts.data(), cuts.size());
-      c->alloc(c->persist_sync, sizeof(elx::GridSync) + sizeof(elx::PersistCol) * elx::kGridCols);
+      c->alloc(c->persist_sync, sizeof(elx::GridSync) + sizeof(elx::PersistState));
       c->alloc(c->persist_vec, 3 * 8 * (size_t)persist_rows(c));
       if (padded) {
         c->upload(c->p_ptr, s.p_ptr.data(), s.p_ptr.size());
@@ -310,8 +315,10 @@ void persist_solve(elx_ctx *c, int nc, double tol, int maxit, const double *b, d
   a.sr = work + n * nc;
   a.p = work + 2 * n * nc;
   a.gs = c->persist_sync.as<elx::GridSync>();
-  a.cols = reinterpret_cast<elx::PersistCol *>(a.gs + 1);
-  a.err = c->flags.as<int32_t>() + 2;
+  elx::PersistState *state = reinterpret_cast<elx::PersistState *>(a.gs + 1);
+  a.cols = state->col;
+  a.err = &state->err;
+  a.stall = elx::grid_stall();
   a.tol = tol;
   a.maxit = maxit;
   a.rows = c->persist_rows;
@@ -330,7 +337,10 @@ void persist_solve(elx_ctx *c, int nc, double tol, int maxit, const double *b, d
     if (cluster) {
       ELX_CUDA(elx::cluster_call(B, a, c->cluster_grid, start, steps, c->stream, nullptr));
     } else {
-      ELX_CUDA(cudaMemsetAsync(a.gs, 0, sizeof(elx::GridSync), c->stream));
+      // a solve's first launch finds no states and no error of an earlier one
+      ELX_CUDA(cudaMemsetAsync(a.gs, 0,
+                               sizeof(elx::GridSync) + (start ? sizeof(elx::PersistState) : 0),
+                               c->stream));
 #define CALL(NC)                                                                     \
   if (B == 3)                                                                        \
     elx::launch<3, NC>(a, c->persist_grid, in_smem, start, steps, c->stream);        \
@@ -340,8 +350,8 @@ void persist_solve(elx_ctx *c, int nc, double tol, int maxit, const double *b, d
 #undef CALL
     }
     c->launches += 1;
-    ELX_CUDA(cudaMemcpyAsync(c->h_cols + slot * elx::kGridCols, a.cols,
-                             sizeof(elx::PersistCol) * nc, cudaMemcpyDeviceToHost, c->stream));
+    ELX_CUDA(cudaMemcpyAsync(c->h_state + slot, state, sizeof(elx::PersistState),
+                             cudaMemcpyDeviceToHost, c->stream));
     ELX_CUDA(cudaEventRecord(c->ev[slot], c->stream));
     launched++;
   };
@@ -361,9 +371,14 @@ void persist_solve(elx_ctx *c, int nc, double tol, int maxit, const double *b, d
   go();
   for (;;) {
     if (launched < max_launches && !c->batch_gate) go();
-    const elx::PersistCol *h = c->h_cols + (checked & 1) * elx::kGridCols;
+    const elx::PersistState &hs = c->h_state[checked & 1];
+    const elx::PersistCol *h = hs.col;
     ELX_CUDA(cudaEventSynchronize(c->ev[checked & 1]));
     checked++;
+    if (hs.err && !cluster) {  // the states were not written; a cluster has no such waits
+      c->sync();
+      throw Error{ELX_ERR_TIMEOUT, kResidentWait};
+    }
     bool all = true;
     for (int k = 0; k < nc; k++) all = all && h[k].done;
     if (all || checked >= max_launches) {

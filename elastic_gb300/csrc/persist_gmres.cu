@@ -46,7 +46,7 @@ struct GmresArgs {
   GridSync *sync;
   GmresDot *dots;  // (2, k)
   int32_t *err;
-  int rows, slices;
+  int rows, slices, stall;
 };
 
 // Shared memory: w and M by rows, the warps' heads, the Hessenberg columns and
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kGT, 1) gmres_persist_kernel(GmresArgs a) {
   __shared__ double snorm;
   __shared__ int32_t sncut, scut[kGW], srun, sbad;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const grid::Team team{(int)blockIdx.x, (int)gridDim.x};
+  const grid::Team team((int)blockIdx.x, (int)gridDim.x, a.stall);
   if (!a.gs->live) return;  // block 0 writes the state after the last wait
   const double econv = a.gs->econv;
   const int s0 = a.cta[blockIdx.x], s1 = a.cta[blockIdx.x + 1], ns = s1 - s0;
@@ -362,6 +362,7 @@ void gmres_persist_cycle(elx_ctx *c, int k, double *basis, double *xr, void *dot
   a.err = c->flags.as<int32_t>() + 2;
   a.rows = c->persist_rows;
   a.slices = c->persist_slices;
+  a.stall = elx::grid_stall();
   ELX_CUDA(cudaMemsetAsync(a.sync, 0, sizeof(elx::GridSync), c->stream));
   ELX_CUDA(cudaMemsetAsync(dots, 0, gmres_persist_bytes(k), c->stream));
   const void *f = B == 3 ? (const void *)elx::gmres_persist_kernel<3>

@@ -41,7 +41,7 @@ struct MixedArgs {
   PcgScalars *sc;
   GridSync *gs;
   int32_t *err;
-  int rows, slices;
+  int rows, slices, stall;
 };
 
 template <int B>
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kMT, 1) mixed_persist_kernel(MixedArgs a, int 
   int32_t *sptr = reinterpret_cast<int32_t *>(shead + kMW * RB);
   int32_t *sga = sptr + a.slices + 1, *swsl = sga + kMW + 1;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const grid::Team team{(int)blockIdx.x, (int)gridDim.x};
+  const grid::Team team((int)blockIdx.x, (int)gridDim.x, a.stall);
   // block 0 writes the scalars after the last wait
   if (a.sc->done) return;
   const int s0 = a.cta[blockIdx.x], s1 = a.cta[blockIdx.x + 1], ns = s1 - s0;
@@ -349,6 +349,7 @@ void mixed_persist_steps(elx_ctx *c, int replace_every, int steps) {
   a.err = c->flags.as<int32_t>() + 2;
   a.rows = c->persist_rows;
   a.slices = c->persist_slices;
+  a.stall = elx::grid_stall();
   ELX_CUDA(cudaMemsetAsync(a.gs, 0, sizeof(elx::GridSync), c->stream));
   const int g = c->persist_grid;
   if (c->s.bsize == 3) {

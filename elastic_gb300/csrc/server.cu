@@ -98,7 +98,7 @@ packed_pcg_kernel(const PackSlot *d, int nslots, int steps, uint64_t epoch) {
     if (d[mid].cta0 <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
   }
   const PackSlot &S = d[lo];
-  const grid::Team team{(int)blockIdx.x - S.cta0, S.ncta};
+  const grid::Team team((int)blockIdx.x - S.cta0, S.ncta, S.a.stall);
   // every block reads the state before its first wait, and the team's first
   // block writes it after the last
   const int start = !S.a.cols[0].started;
@@ -893,6 +893,7 @@ void gpu_loop(elx_server *sv) {
               a.maxit = q->maxit;
               a.rows = elx::kPackRows;
               a.slices = elx::pack_slices(c->s.bsize);
+              a.stall = elx::grid_stall();
               d.bsize = c->s.bsize;
               d.cta0 = L.blocks;
               d.ncta = q->blocks;

@@ -24,9 +24,7 @@
 namespace elx {
 
 constexpr int kGridMaxBlocks = 160;
-// Bound of every grid wait, and its length in a launch that waits for a block
-// too many on purpose (ELX_GRID_STALL_TEST)
-constexpr int kGridWaitMs = 2000, kGridStallMs = 50;
+constexpr uint64_t kGridWaitNs = 1000000000ull;  // bound of every grid wait
 constexpr int kDigits = 5;
 constexpr int kClusterBlocks = 16;  // the most that a cluster has
 
@@ -84,25 +82,25 @@ __device__ __forceinline__ FixSum fix_shfl(FixSum f, int lane) {
   return r;
 }
 
-// The blocks that work together: all of a launch, or some.  `stall`: one more is
-// waited for, so that the waits run out (tests).
-struct Team {
-  int me, n, wait_ms;
-  __device__ __forceinline__ Team(int me_, int n_, int stall)
-      : me(me_), n(n_ + stall), wait_ms(stall ? kGridStallMs : kGridWaitMs) {}
-};
-
 // Counts polls and bounds them by the GPU's clock.
 struct Bound {
-  const int ms;
   uint64_t t0 = 0;
   uint32_t it = 0;
-  __device__ __forceinline__ explicit Bound(const Team &t) : ms(t.wait_ms) {}
   __device__ __forceinline__ bool over() {
     if (++it & 1023u) return false;
     const uint64_t now = ptx::global_ns();
     if (!t0) t0 = now;
-    return now - t0 > (uint64_t)ms * 1000000u;
+    return now - t0 > kGridWaitNs;
+  }
+};
+
+// The blocks that work together: all of a launch, or some.
+struct Team {
+  int me, n;
+  // With `stall` (ELX_GRID_STALL_TEST) a team's last block does not take part,
+  // and the others' waits run out.
+  __device__ __forceinline__ bool missing(int stall) const {
+    return stall && n > 1 && me == n - 1;
   }
 };
 
@@ -117,7 +115,7 @@ __device__ __forceinline__ bool slot_sum(Team t, GridSlot (*slots)[kGridMaxBlock
     store_slot(slots[lane] + t.me, f.m,
                epoch << 24 | (uint64_t)(uint32_t)(f.e + 4096));
   bool ok = true;
-  Bound bound(t);
+  Bound bound;
   for (int c = 0; c < NC; c++) {
     FixSum v[K];
 #pragma unroll
@@ -198,7 +196,7 @@ __device__ __forceinline__ bool digit_read(Team t, GridSlot (*slots)[kGridMaxBlo
   unsigned long long w = 0;
   bool ok = true;
   if (lane < NC * kDigits) {
-    Bound bound(t);
+    Bound bound;
     for (;;) {
       w = load_relaxed(words->digit + lane);
       if (((w - seen) >> 48 & 0xff) == (unsigned)n) break;
@@ -370,7 +368,7 @@ __device__ __forceinline__ bool barrier(Team team, GridSync *gs, uint32_t count,
     red_add(p, 1);
     const unsigned long long want = (unsigned long long)count * team.n;
     bool ok = true;
-    Bound bound(team);
+    Bound bound;
     while (ok && load_relaxed(p) < want) ok = !bound.over();
     fence();
     sh.ok = ok;

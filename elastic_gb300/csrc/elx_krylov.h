@@ -43,8 +43,8 @@ struct PersistState {
   PersistCol col[kGridCols];
   int32_t err, pad[3];
 };
-// ELX_GRID_STALL_TEST=1: the resident launches wait for a block too many (tests
-// of the timeouts; read at every solve).
+// ELX_GRID_STALL_TEST=1: a block of each resident launch does not take part
+// (tests of the timeouts; read at every solve).
 int grid_stall();
 // Cuts slices into one run per block with equal numbers of slot groups.
 std::vector<int32_t> persist_cuts(const std::vector<int32_t> &sell_ptr, int grid);

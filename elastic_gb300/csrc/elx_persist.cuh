@@ -26,7 +26,7 @@ struct PersistArgs {
   double tol;
   int maxit;
   int rows, slices;  // of the largest block
-  int stall = 0;     // grid::Team's
+  int stall = 0;     // grid::Team::missing
 };
 
 // Shared memory: the block's rows of q (and of x, r, p, M), the warps' heads

@@ -56,7 +56,9 @@ constexpr double kClusterGain = 2800;
 template <int B, int NC, bool SMEM>
 __global__ void __launch_bounds__(kPT, 1)
 pcg_persist_kernel(PersistArgs a, int start, int steps) {
-  persist_pcg<kPT, B, NC, SMEM>(a, grid::Team((int)blockIdx.x, (int)gridDim.x, a.stall), start, steps, 0);
+  const grid::Team team{(int)blockIdx.x, (int)gridDim.x};
+  if (team.missing(a.stall)) return;
+  persist_pcg<kPT, B, NC, SMEM>(a, team, start, steps, 0);
 }
 
 // The same by one cluster: grid::Cluster's sums and barrier.

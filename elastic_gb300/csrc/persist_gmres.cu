@@ -75,7 +75,8 @@ __global__ void __launch_bounds__(kGT, 1) gmres_persist_kernel(GmresArgs a) {
   __shared__ double snorm;
   __shared__ int32_t sncut, scut[kGW], srun, sbad;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const grid::Team team((int)blockIdx.x, (int)gridDim.x, a.stall);
+  const grid::Team team{(int)blockIdx.x, (int)gridDim.x};
+  if (team.missing(a.stall)) return;
   if (!a.gs->live) return;  // block 0 writes the state after the last wait
   const double econv = a.gs->econv;
   const int s0 = a.cta[blockIdx.x], s1 = a.cta[blockIdx.x + 1], ns = s1 - s0;

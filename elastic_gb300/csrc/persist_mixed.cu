@@ -65,7 +65,8 @@ __global__ void __launch_bounds__(kMT, 1) mixed_persist_kernel(MixedArgs a, int 
   int32_t *sptr = reinterpret_cast<int32_t *>(shead + kMW * RB);
   int32_t *sga = sptr + a.slices + 1, *swsl = sga + kMW + 1;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const grid::Team team((int)blockIdx.x, (int)gridDim.x, a.stall);
+  const grid::Team team{(int)blockIdx.x, (int)gridDim.x};
+  if (team.missing(a.stall)) return;
   // block 0 writes the scalars after the last wait
   if (a.sc->done) return;
   const int s0 = a.cta[blockIdx.x], s1 = a.cta[blockIdx.x + 1], ns = s1 - s0;

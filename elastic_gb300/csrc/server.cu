@@ -98,7 +98,8 @@ packed_pcg_kernel(const PackSlot *d, int nslots, int steps, uint64_t epoch) {
     if (d[mid].cta0 <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
   }
   const PackSlot &S = d[lo];
-  const grid::Team team((int)blockIdx.x - S.cta0, S.ncta, S.a.stall);
+  const grid::Team team{(int)blockIdx.x - S.cta0, S.ncta};
+  if (team.missing(S.a.stall)) return;
   // every block reads the state before its first wait, and the team's first
   // block writes it after the last
   const int start = !S.a.cols[0].started;

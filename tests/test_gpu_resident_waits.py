@@ -1,7 +1,7 @@
-"""The bounded waits of the resident solvers: with a block expected that is not
-there (ELX_GRID_STALL_TEST=1; the waits then run out after 50 ms) each solve
-returns ELX_ERR_TIMEOUT after the launches in flight, whatever maxit is, and
-the same context solves correctly once the stall is lifted."""
+"""The bounded waits of the resident solvers: with one block that does not take
+part (ELX_GRID_STALL_TEST=1; the others' waits run out after a second) each
+solve returns ELX_ERR_TIMEOUT after the two launches in flight, whatever maxit
+is, and the same context solves correctly once the stall is lifted."""
 import time
 
 import numpy as np
@@ -43,19 +43,17 @@ def test_a_wait_that_runs_out(built_lib, monkeypatch, kind):
                 return X[:, 2] / 4, infos[2]
             return ctx.solve(b, maxit=kw.get("maxit", 20000), tol=1e-10, **KINDS.get(kind, {}))
 
-        for _ in range(2):
-            monkeypatch.setenv("ELX_GRID_STALL_TEST", "1")
-            t0 = time.monotonic()
-            with pytest.raises(E.ElasticError) as e:
-                solve()
-            assert e.value.code == E.ERR_TIMEOUT and "resident" in str(e.value)
-            assert time.monotonic() - t0 < 1.5
-            monkeypatch.delenv("ELX_GRID_STALL_TEST")
-            if kind == "gmres":
-                continue
+        monkeypatch.setenv("ELX_GRID_STALL_TEST", "1")
+        t0 = time.monotonic()
+        with pytest.raises(E.ElasticError) as e:
+            solve()
+        assert e.value.code == E.ERR_TIMEOUT and "resident" in str(e.value)
+        assert time.monotonic() - t0 < 4
+        monkeypatch.delenv("ELX_GRID_STALL_TEST")
+        if kind != "gmres":
             x, i = solve()
             assert i["status"] == 0 and rel_inf(x_o, x) <= (1e-5 if kind == "mixed" else 1e-8)
-        if kind == "gmres":
+        else:
             g_o, _ = O.gmres(s, ad, al, b, k=17, tol=1e-14, maxit=1)
             x, _ = ctx.solve(b, solver=E.SOLVER_GMRES, ngram=17, tol=1e-14, maxit=1,
                              raise_on_error=False)

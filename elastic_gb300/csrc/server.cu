@@ -89,6 +89,13 @@ constexpr int kPackThreads = 256;
 constexpr int kPackPerSm = 4;
 constexpr int kPackRows = 768;  // five vectors of it in shared memory: 37 KB a block
 
+// Zeroes the words (not the slots) of every team's sums before a launch.
+__global__ void pack_words_kernel(const PackSlot *d) {
+  constexpr int kWords = offsetof(GridSync, slot) / 8;
+  unsigned long long *w = reinterpret_cast<unsigned long long *>(d[blockIdx.x].a.gs);
+  for (int i = threadIdx.x; i < kWords; i += blockDim.x) w[i] = 0;
+}
+
 __global__ void __launch_bounds__(kPackThreads, kPackPerSm)
 packed_pcg_kernel(const PackSlot *d, int nslots, int steps, uint64_t epoch) {
   if (nslots == 0) return;
@@ -340,6 +347,7 @@ struct SrvRequest {
   DBuf vecs;  // b (nrhs x neq), then per load case x, r, p, q
   int blocks = 0;  // of each load case in the cooperative pack (0: packed launches)
   DBuf cuts;       // its slices' cuts between them
+  DBuf sync;       // a GridSync for each load case
   cudaEvent_t ready = nullptr;
   std::vector<int> slots;  // indices into the server's slot scalars
   // result
@@ -384,11 +392,9 @@ struct elx_server {
   std::vector<std::shared_ptr<SrvRequest>> active;
   void *d_desc = nullptr, *d_part = nullptr;
   size_t desc_bytes = 0, part_bytes = 0;
-  // the cooperative pack: slot states (the error word first), the grids'
-  // words, descriptors; blocks that fit the GPU at once
+  // the cooperative pack: slot states (the error word first), descriptors;
+  // blocks that fit the GPU at once
   elx::PersistCol *d_col = nullptr, *h_col = nullptr;  // 1 + max_slots
-  elx::GridSync *d_sync = nullptr;
-  int sync_slots = 0;
   elx::PackSlot *d_pack = nullptr, *h_pack = nullptr;  // max_slots
   int pack_capacity = 0;
   uint64_t epoch = 0;
@@ -447,7 +453,7 @@ int64_t estimate_bytes(const SrvRequest &q) {
     b += 4 * slots * s.bsize * s.bsize + 5 * 4 * n;
     b += 8 * 2 * 16 * elx::grid_cap(8) + (64 << 10);
   } else {
-    b += 5 * 8 * n * q.nrhs;                           // per load case
+    b += (5 * 8 * n + sizeof(elx::GridSync)) * q.nrhs;  // per load case
   }
   b += 160 << 10;                                      // scalars, partials, padding
   return b;
@@ -551,6 +557,7 @@ void release_request(elx_server *sv, SrvRequest &q) {
   if (q.ctx) {
     q.ctx->release(q.vecs);
     q.ctx->release(q.cuts);
+    q.ctx->release(q.sync);
     elx_destroy(q.ctx);
     q.ctx = nullptr;
   }
@@ -621,6 +628,8 @@ void admit(elx_server *sv, SrvRequest &q) {
     std::vector<int32_t> cuts(q.blocks + 1);
     for (int k = 0; k <= q.blocks; k++) cuts[k] = (int32_t)((int64_t)nsl * k / q.blocks);
     c->upload(q.cuts, cuts.data(), cuts.size());
+    c->alloc(q.sync, sizeof(elx::GridSync) * q.nrhs);
+    ELX_CUDA(cudaMemsetAsync(q.sync.p, 0, q.sync.bytes, c->stream));
     for (int k = 0; k < q.nrhs; k++)
       ELX_CUDA(cudaMemsetAsync(sv->d_col + 1 + q.slots[k], 0, sizeof(elx::PersistCol), c->stream));
     c->sync();  // the cuts' host copy
@@ -888,7 +897,7 @@ void gpu_loop(elx_server *sv) {
               a.sr = x + n;
               a.p = x + 2 * n;
               a.cols = sv->d_col + 1 + q->slots[k];
-              a.gs = nullptr;  // below, once there is one for each slot
+              a.gs = q->sync.as<elx::GridSync>() + k;
               a.err = reinterpret_cast<int32_t *>(sv->d_col);
               a.tol = q->tol;
               a.maxit = q->maxit;
@@ -931,16 +940,6 @@ void gpu_loop(elx_server *sv) {
           }
         }
         sv->peak_slots = std::max<int64_t>(sv->peak_slots.load(), nslots + npack);
-        if (npack > sv->sync_slots) {
-          if (sv->d_sync) cudaFree(sv->d_sync);
-          sv->d_sync = nullptr;
-          sv->sync_slots = 0;
-          const int want = std::min(sv->max_slots, std::max(64, 2 * npack));
-          ELX_CUDA(cudaMalloc(&sv->d_sync, sizeof(elx::GridSync) * want));
-          ELX_CUDA(cudaMemsetAsync(sv->d_sync, 0, sizeof(elx::GridSync) * want, sv->stream));
-          sv->sync_slots = want;
-        }
-        for (int k = 0; k < npack; k++) sv->h_pack[k].a.gs = sv->d_sync + k;
         if (npack)
           ELX_CUDA(cudaMemcpyAsync(sv->d_pack, sv->h_pack, npack * sizeof(elx::PackSlot),
                                    cudaMemcpyHostToDevice, sv->stream));
@@ -962,9 +961,7 @@ void gpu_loop(elx_server *sv) {
       // vectors come from and go to L2 once a launch)
       const int steps = npack ? 4 * sv->poll_steps : sv->poll_steps;
       if (npack) {
-        // the words (not the slots) of each team's sums
-        ELX_CUDA(cudaMemset2DAsync(sv->d_sync, sizeof(elx::GridSync), 0,
-                                   offsetof(elx::GridSync, slot), npack, sv->stream));
+        elx::pack_words_kernel<<<npack, 96, 0, sv->stream>>>(sv->d_pack);
         for (const PackLaunch &L : packs) {
           const elx::PackSlot *d = sv->d_pack + L.first;
           int n = L.n, st = steps;
@@ -1151,7 +1148,6 @@ void elx_server_destroy(elx_server *sv) {
   if (sv->d_desc) cudaFree(sv->d_desc);
   if (sv->d_part) cudaFree(sv->d_part);
   if (sv->d_col) cudaFree(sv->d_col);
-  if (sv->d_sync) cudaFree(sv->d_sync);
   if (sv->d_pack) cudaFree(sv->d_pack);
   if (sv->h_col) cudaFreeHost(sv->h_col);
   if (sv->h_pack) cudaFreeHost(sv->h_pack);

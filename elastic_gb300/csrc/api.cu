@@ -859,24 +859,40 @@ int autotune_block_width(elx_ctx *c, bool mixed, double *times_us = nullptr) {
   return best;
 }
 
+// Whether nrhs FP64 load cases cost less in resident launches of up to nc columns
+// than in blocks of w.  A resident launch pads nothing and waits less, but a
+// chunk beyond the first waits again, where a block of w takes them all in one
+// iteration.  Both sides as us an iteration and load, fitted to 1 to 6 columns
+// and blocks of 8 and 16 on TRIA3, QUAD4, TETRA4 and HEXA8 of 240 to 390,150
+// equations, the solve's fixed part spread over 100 iterations: a latency floor
+// that grows with the entries of a row, and work per equation.  Resident /
+// launches at 8, 12, 13 and 16 load cases: 1.06, 1.33, 1.66, 1.83 (640 equations
+// of TRIA3), 0.86, 0.77, 0.92, 1.05 (21,840), 0.77, 0.62, 0.69, 0.84 (240,800);
+// 0.76, 1.00, 1.19, 1.36 (1,944 of HEXA8), 0.85, 0.82, 0.88, 1.08 (63,504), 0.98,
+// 0.76, 0.84, 1.02 (201,720).  Of 544 measured pairs the line takes none to the
+// side that is slower by more than 5 %.
+bool resident_chunks_pay(const elx::Structure &s, int nrhs, int nc, int w) {
+  const double row = (2.0 * s.nad + s.neq) / s.neq, meq = 1e-6 * s.neq;
+  const int chunks = (nrhs + nc - 1) / nc, blocks = (nrhs + w - 1) / w;
+  const double resident = chunks * 3.7 + nrhs * (1.1 + 0.031 * row + meq * (15.0 + 2.67 * row));
+  const double launches = blocks * (11.8 + 0.44 * row + w * meq * (41.0 + 2.3 * row));
+  return resident < 0.95 * launches;
+}
+
 // FP64 load cases by the cooperative PCG, up to nc columns a launch (persist.cu):
 // the columns share the matrix reads and the waits, and none pads a block to a
 // width.  False: the matrix is too large for it, or the memory budget has no
 // room for the vectors of four columns.
 bool solve_block_persist(elx_ctx *c, int nrhs, double tol, int maxit, int width, const double *b,
                          double *x, elx_info *infos, bool device_ptrs) {
-  // 3x3 blocks are FP64-bound either way: krylov's product over 8 or 16 columns
-  // is 5 % faster per column when none of its columns is padding (205,320
-  // equations, 16 columns: 388 against 405 ms; 6 columns: 206 against 152)
   int w = 1;
   while (w < 16 && w < nrhs && (width == 0 || w < width)) w *= 2;
-  if (c->s.bsize == 3 && nrhs > elx::kGridCols && 21 * nrhs > 20 * ((nrhs + w - 1) / w * w))
-    return false;
   const int want = std::min(nrhs, width > 0 ? width : elx::kGridCols);
   const int least = std::min(want, 4);
   const size_t n = (size_t)c->s.neq;
   // per column: three work vectors, b and x
   int nc = persist_columns(c, want);
+  if (nrhs > nc && w > nc && nc > 0 && !resident_chunks_pay(c->s, nrhs, nc, w)) return false;
   while (nc >= least && !persist_vectors(c, 5 * n * nc * 8))
     nc = nc > least ? persist_columns(c, nc - 1) : 0;
   if (nc < least) return false;
@@ -906,16 +922,19 @@ bool solve_block_persist(elx_ctx *c, int nrhs, double tol, int maxit, int width,
     if (!device_ptrs)
       ELX_CUDA(cudaMemcpyAsync(x + (size_t)c0 * n, xs, n * m * 8, cudaMemcpyDeviceToHost,
                                c->stream));
+    double(*dg)[4] = persist_state(c)->diag;
     for (int j = 0; j < m; j++) {
       spmv64(c, xd + (size_t)j * n, c->z.as<double>());
       elx::launch_diagnostics(c->s.neq, xd + (size_t)j * n, c->z.as<double>(),
-                              bd + (size_t)j * n, c->m.as<double>(), c->diag.as<double>(),
+                              bd + (size_t)j * n, c->m.as<double>(), dg[j],
                               c->partials.as<double>(), c->counters.as<unsigned int>() + 3,
                               c->stream);
       c->launches += 1;
-      ELX_CUDA(cudaMemcpyAsync(c->h_diag, c->diag.p, 4 * sizeof(double), cudaMemcpyDeviceToHost,
-                               c->stream));
-      check_pipe_waits(c);
+    }
+    ELX_CUDA(cudaMemcpyAsync(c->h_state->diag, dg, sizeof(c->h_state->diag),
+                             cudaMemcpyDeviceToHost, c->stream));
+    c->sync();
+    for (int j = 0; j < m; j++) {
       const int st = cols[j].done ? cols[j].status : ELX_ERR_NO_CONVERGENCE;
       if (st != ELX_OK && status == ELX_OK) status = st;
       if (!infos) continue;
@@ -923,10 +942,11 @@ bool solve_block_persist(elx_ctx *c, int nrhs, double tol, int maxit, int width,
       std::memset(&in, 0, sizeof(in));
       in.iters = cols[j].iters;
       in.status = st;
-      in.xkx = c->h_diag[0];
-      in.norm_x = std::sqrt(c->h_diag[1]);
-      in.norm_m_r = std::sqrt(std::fabs(c->h_diag[2]));
-      in.norm_r = std::sqrt(c->h_diag[3]);
+      const double *hd = c->h_state->diag[j];
+      in.xkx = hd[0];
+      in.norm_x = std::sqrt(hd[1]);
+      in.norm_m_r = std::sqrt(std::fabs(hd[2]));
+      in.norm_r = std::sqrt(hd[3]);
       in.conv = cols[j].conv;
     }
     const double secs =

@@ -267,6 +267,7 @@ constexpr const char *kResidentWait = "a bounded device wait of the resident sol
 bool ensure_persist(elx_ctx *c);
 int persist_columns(elx_ctx *c, int want);
 bool persist_vectors(elx_ctx *c, size_t bytes);
+elx::PersistState *persist_state(const elx_ctx *c);  // device
 int persist_rows(const elx_ctx *c);
 bool mixed_persist(elx_ctx *c);
 bool ensure_gmres_persist(elx_ctx *c, int k);

@@ -161,7 +161,7 @@ void pool_users(int device, int delta);
 // A context's small pinned host scalars: blocks of kPinnedBlock bytes,
 // carved from larger pinned allocations and recycled, so that creating and
 // destroying contexts pins and unpins no memory once warm.
-constexpr size_t kPinnedBlock = 1024;
+constexpr size_t kPinnedBlock = 2048;
 void *pinned_block_get();
 void pinned_block_put(void *p);
 // Grid bound of the grid-stride kernels: per_sm CTAs on every SM.

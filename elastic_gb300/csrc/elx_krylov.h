@@ -38,10 +38,12 @@ struct PersistCol {
   double d, conv;
   int32_t iters, done, status, started;
 };
-// The columns and the word of a wait that ran out, read together by the host.
+// The columns and the word of a wait that ran out, read together by the host,
+// and what a block solve reports of each column (launch_diagnostics).
 struct PersistState {
   PersistCol col[kGridCols];
   int32_t err, pad[3];
+  double diag[kGridCols][4];
 };
 // ELX_GRID_STALL_TEST=1: a block of each resident launch does not take part
 // (tests of the timeouts; read at every solve).

@@ -35,6 +35,7 @@
 // warps is summed by its first warp and the heads of the following ones, in
 // warp order, so results do not depend on timing.
 #include <algorithm>
+#include <cstddef>
 #include <cstdlib>
 
 #include "elx_context.h"
@@ -294,6 +295,10 @@ bool persist_vectors(elx_ctx *c, size_t bytes) {
   return false;
 }
 
+elx::PersistState *persist_state(const elx_ctx *c) {
+  return reinterpret_cast<elx::PersistState *>(c->persist_sync.as<elx::GridSync>() + 1);
+}
+
 // PCG of nc columns b -> x (device, neq x nc), at most `steps` iterations a
 // launch, two launches in flight; `work` holds 3 n nc doubles.  The columns'
 // results into out.
@@ -317,7 +322,7 @@ void persist_solve(elx_ctx *c, int nc, double tol, int maxit, const double *b, d
   a.sr = work + n * nc;
   a.p = work + 2 * n * nc;
   a.gs = c->persist_sync.as<elx::GridSync>();
-  elx::PersistState *state = reinterpret_cast<elx::PersistState *>(a.gs + 1);
+  elx::PersistState *state = persist_state(c);
   a.cols = state->col;
   a.err = &state->err;
   a.stall = elx::grid_stall();
@@ -341,7 +346,7 @@ void persist_solve(elx_ctx *c, int nc, double tol, int maxit, const double *b, d
     } else {
       // a solve's first launch finds no states and no error of an earlier one
       ELX_CUDA(cudaMemsetAsync(a.gs, 0,
-                               sizeof(elx::GridSync) + (start ? sizeof(elx::PersistState) : 0),
+                               sizeof(elx::GridSync) + (start ? offsetof(elx::PersistState, diag) : 0),
                                c->stream));
 #define CALL(NC)                                                                     \
   if (B == 3)                                                                        \
@@ -352,7 +357,7 @@ void persist_solve(elx_ctx *c, int nc, double tol, int maxit, const double *b, d
 #undef CALL
     }
     c->launches += 1;
-    ELX_CUDA(cudaMemcpyAsync(c->h_state + slot, state, sizeof(elx::PersistState),
+    ELX_CUDA(cudaMemcpyAsync(c->h_state + slot, state, offsetof(elx::PersistState, diag),
                              cudaMemcpyDeviceToHost, c->stream));
     ELX_CUDA(cudaEventRecord(c->ev[slot], c->stream));
     launched++;

@@ -43,24 +43,22 @@ __device__ __forceinline__ double gather_columns(const double *partials, int nbl
   constexpr int S = kThreads / NC;
   __shared__ double sh[kThreads];
   const int c = threadIdx.x % NC, sl = threadIdx.x / NC;
-  // eight loads in flight, four chains of adds (76 adds a thread of 1216 blocks'
-  // partials: a chain of FP64 adds is 64 clocks each)
-  double t0 = 0.0, t1 = 0.0, t2 = 0.0, t3 = 0.0;
-  const double *pc = partials + (size_t)c * nblocks;
-  int b = sl;
-#pragma unroll 2
-  for (; b + 3 * S < nblocks; b += 4 * S) {
-    t0 += __ldcg(pc + b);
-    t1 += __ldcg(pc + b + S);
-    t2 += __ldcg(pc + b + 2 * S);
-    t3 += __ldcg(pc + b + 3 * S);
-  }
-  for (; b < nblocks; b += S) t0 += __ldcg(pc + b);
-  sh[threadIdx.x] = (t0 + t1) + (t2 + t3);
+  double t = 0.0;
+#pragma unroll 4
+  for (int b = sl; b < nblocks; b += S) t += __ldcg(partials + (size_t)c * nblocks + b);
+  sh[threadIdx.x] = t;
   __syncthreads();
   double u = 0.0;
-  if (threadIdx.x < NC)
-    for (int k = 0; k < S; k++) u += sh[k * NC + threadIdx.x];
+  if (threadIdx.x < NC) {
+    // A small grid fills the first slices only: the rest are zeros, and a chain
+    // of 256 FP64 adds at W = 1 (mixed solves of 2,480 equations of QUAD4, us an
+    // iteration: 33.3 -> 15.0 at W = 1, 26.8 -> 17.2 at 2, 24.9 -> 20.2 at 4)
+    if (nblocks < S) {
+      for (int k = 0; k < nblocks; k++) u += sh[k * NC + threadIdx.x];
+    } else {
+      for (int k = 0; k < S; k++) u += sh[k * NC + threadIdx.x];
+    }
+  }
   return u;
 }
 
@@ -218,36 +216,53 @@ __device__ __forceinline__ bool column_reduce_v(double (&v)[VC], double *partial
 }
 
 // The same for FP32 values, in integers (FixSum): the FP64 shuffle trees of
-// eight blocks per SM held its FP64 pipe for 8 of the update's 50 us.  Warp w
-// adds columns w, w + 8, ... of the block's values from shared memory.
+// eight blocks per SM held its FP64 pipe for 8 of the update's 50 us.  Of one
+// column a warp adds its own lanes' values; of more, warp w adds columns w, w + 8
+// of the block's values from shared memory.  The block's sums are
+// published together: one fence (W = 16 with one for each of a warp's columns
+// 23.8 us an iteration at 2,480 equations of QUAD4, 21.9 here).
 template <int W, int VC>
 __device__ __forceinline__ bool column_reduce_v(const float (&v)[VC], double *partials,
                                                 unsigned int *counter, double &out) {
-  constexpr int G = W / VC, N = kThreads / G, K = N / 32;  // values of a column, per lane
-  __shared__ float sv[VC][kThreads];
+  constexpr int G = W / VC, NW = kThreads / 32;
+  constexpr int P = W == 1 ? NW : 1;  // warps that share a column
+  __shared__ double sh[P][W];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if constexpr (W == 1) {
+    const double s = fix_value(warp_sum(fix_of(v[0])));
+    if (lane == 0) sh[warp][0] = s;
+  } else {
+    constexpr int N = kThreads / G, K = N / 32;  // values of a column, per lane
+    __shared__ float sv[VC][kThreads];
 #pragma unroll
-  for (int j = 0; j < VC; j++) sv[j][threadIdx.x] = v[j];
+    for (int j = 0; j < VC; j++) sv[j][threadIdx.x] = v[j];
+    __syncthreads();
+#pragma unroll
+    for (int c = warp; c < W; c += NW) {
+      FixSum f[K];
+      int e = -4096;
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        f[k] = fix_of(sv[c % VC][c / VC + G * (lane + 32 * k)]);
+        e = max(e, f[k].e);
+      }
+      FixSum t;
+      t.m = 0;
+#pragma unroll
+      for (int k = 0; k < K; k++) t.m += fix_align(f[k], e, 3);
+      t.e = e >= kFixBad ? e : e + 3;
+      const double s = fix_value(warp_sum(t));
+      if (lane == 0) sh[0][c] = s;
+    }
+  }
   __syncthreads();
-  for (int c = warp; c < W; c += kThreads / 32) {
-    FixSum f[K];
-    int e = -4096;
+  if (threadIdx.x < W) {
+    double t = sh[0][threadIdx.x];
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      f[k] = fix_of(sv[c % VC][c / VC + G * (lane + 32 * k)]);
-      e = max(e, f[k].e);
-    }
-    FixSum t;
-    t.m = 0;
-#pragma unroll
-    for (int k = 0; k < K; k++) t.m += fix_align(f[k], e, 3);
-    t.e = e >= kFixBad ? e : e + 3;
-    const double s = fix_value(warp_sum(t));
-    if (lane == 0) {
-      partials[(size_t)c * gridDim.x + blockIdx.x] = s;
-      __threadfence();
-    }
+    for (int p = 1; p < P; p++) t += sh[p][threadIdx.x];
+    partials[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = t;
+    __threadfence();
   }
   __syncthreads();
   if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
@@ -304,7 +319,8 @@ sell_spmm_kernel(int nb, int nslices, const int32_t *__restrict__ sell_ptr,
   // slices then gather 918 distinct x rows instead of 1,510 (L1 hits 58 -> 60 %,
   // 214 -> 208 us, W = 16 FP32 on the 96x96x48 plate).
   const int sms = gridDim.x / per_sm;
-  const int first = (blockIdx.x % sms) * per_sm + blockIdx.x / sms;
+  const int first =
+      sizeof(T) == 8 ? (int)blockIdx.x : (blockIdx.x % sms) * per_sm + blockIdx.x / sms;
   for (int sl = first * SPC + (int)threadIdx.x / (R * G); sl < nslices;
        sl += gridDim.x * SPC) {
     const int g0 = sell_ptr[sl], g1 = sell_ptr[sl + 1];

@@ -442,10 +442,13 @@ void spmv64(elx_ctx *c, const double *x, double *y) {
 // A bounded device wait of the pipelined (tiled) SpMV or of a resident mixed or
 // GMRES launch that gave up leaves its code in flags[2]; reported, and cleared,
 // as ELX_ERR_TIMEOUT.
+// `state` (nullable): read in the same wait.
 void check_pipe_waits(elx_ctx *c,
-                      const char *what = "a bounded device wait of the SpMV pipeline gave up") {
+                      const char *what = "a bounded device wait of the SpMV pipeline gave up",
+                      void *state = nullptr, const void *d_state = nullptr, size_t bytes = 0) {
   ELX_CUDA(cudaMemcpyAsync(c->h_flags + 2, c->flags.as<int32_t>() + 2, sizeof(int32_t),
                            cudaMemcpyDeviceToHost, c->stream));
+  if (state) ELX_CUDA(cudaMemcpyAsync(state, d_state, bytes, cudaMemcpyDeviceToHost, c->stream));
   c->sync();
   if (c->h_flags[2] != 0) {
     ELX_CUDA(cudaMemsetAsync(c->flags.as<int32_t>() + 2, 0, sizeof(int32_t), c->stream));
@@ -716,13 +719,16 @@ void gmres64(elx_ctx *c, int kdim, double tol, int maxit, elx_info *info) {
   }
   elx::GmresState st{};
   for (int cyc = 0; cyc <= maxit; cyc++) {
-    ELX_CUDA(cudaMemcpyAsync(&st, gs, sizeof(st), cudaMemcpyDeviceToHost, c->stream));
-    c->sync();
+    if (persist) {
+      check_pipe_waits(c, kResidentWait, &st, gs, sizeof(st));
+    } else {
+      ELX_CUDA(cudaMemcpyAsync(&st, gs, sizeof(st), cudaMemcpyDeviceToHost, c->stream));
+      c->sync();
+    }
     if (!st.live) break;
     if (persist) {
       gmres_persist_cycle(c, kdim, c->gbasis.as<double>(), c->persist_vec.as<double>(),
                           c->garrays.p);
-      check_pipe_waits(c, kResidentWait);
       continue;
     }
     ELX_CUDA(cudaGraphLaunch(c->gmres_graph, c->stream));

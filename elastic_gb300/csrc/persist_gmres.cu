@@ -324,10 +324,27 @@ __global__ void __launch_bounds__(kGT, 1) gmres_persist_kernel(GmresArgs a) {
 
 namespace elx_api {
 
+// Whether a resident cycle of GMRES(k) costs less than its launches.  It saves
+// the launches of k (k + 1) / 2 projections and reads the basis four times a
+// step where they read it twice, which weighs more the larger the matrix and
+// the shorter the cycle; with k = 1 it saves three launches and pays its own
+// start.  Launches / resident, us a cycle: QUAD4 of 9,728 equations k = 1 50 / 52,
+// k = 2 74 / 68; TRIA3 of 401,000 k = 3 191 / 206, 6 399 / 371; QUAD4 of 701,400
+// k = 8 803 / 816, 12 1,381 / 1,271; TRIA3 of 1,261,800 k = 24 6,219 / 6,356, 32
+// 10,109 / 9,851; HEXA8 of 9,450 k = 1 78 / 55; of 285,660 k = 1 164 / 155; of
+// 669,780 k = 8 1,449 / 1,482, 12 2,304 / 2,260; of 1,299,600 k = 24 9,931 /
+// 12,043.  With partly fixed nodes the launches' product is the scalar gather:
+// TRIA3 of 1,261,600 k = 1 359 / 240, HEXA8 of 9,450 k = 1 49 / 57, 2 76 / 68.
+static bool gmres_cycle_pays(const elx_ctx *c, int k) {
+  const double n = c->s.neq;
+  if (!c->use_blocks) return k > 1 || n > 1.5e5;
+  return k >= (c->s.bsize == 3 ? 0.5 + n * n / 5e10 : 2.0 + n * n / 6e10);
+}
+
 // Plans the cooperative cycle of GMRES(k) (its basis by rows of the sliced
 // matrix); false: krylov_ns.cu's launches are used.
 bool ensure_gmres_persist(elx_ctx *c, int k) {
-  if (!ensure_persist(c)) return false;
+  if (!gmres_cycle_pays(c, k) || !ensure_persist(c)) return false;
   int limit = 0;
   ELX_CUDA(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
   const int B = c->use_blocks ? c->s.bsize : c->s.p_bsize;

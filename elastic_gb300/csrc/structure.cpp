@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <memory>
 #include <numeric>
 #include <thread>
 
@@ -697,82 +698,103 @@ void build_padded(Structure &s, int bsize) {
   const int B = bsize, R = kSliceRows;
   const int nnode = (int)(s.id.size() / B);
   if (B < 2 || B > 3 || s.neq < 1) return;
-  std::vector<int32_t> node_at(s.neq, -1);  // the node whose first equation it is
-  for (int no = 0; no < nnode; no++) {
-    int32_t first = 0, next = 0;
-    for (int d = 0; d < B; d++) {
-      const int32_t q = s.id[(size_t)no * B + d];
-      if (q <= 0) continue;
-      if (!first) first = next = q;
-      if (q != next++) return;
+  // the node whose first equation it is, and how many it has
+  std::vector<int32_t> node_at(s.neq, -1);
+  std::vector<uint8_t> count(s.neq, 0);
+  std::atomic<bool> bad{false};
+  std::atomic<int32_t> nodes{0};
+  parallel_chunks(nnode, 65536, [&](int64_t a, int64_t b) {
+    int32_t n_free = 0;
+    for (int64_t no = a; no < b; no++) {
+      int32_t first = 0, n = 0;
+      bool ok = true;
+      for (int d = 0; d < B; d++) {
+        const int32_t q = s.id[no * B + d];
+        if (q <= 0) continue;
+        if (!first) first = q;
+        ok = ok && q == first + n++;
+      }
+      if (!first) continue;
+      n_free++;
+      if (!ok || first - 1 + n > s.neq) {
+        bad = true;
+        return;
+      }
+      node_at[first - 1] = (int32_t)no;
+      count[first - 1] = (uint8_t)n;
     }
-    if (!first) continue;
-    if (node_at[first - 1] >= 0) return;
-    node_at[first - 1] = no;
-  }
-  std::vector<int32_t> first, count, blk(s.neq, -1);
-  s.p_eq.clear();
-  for (int32_t q = 0; q < s.neq;) {
-    const int no = node_at[q];
-    if (no < 0) return;
-    const int I = (int)first.size();
+    nodes += n_free;
+  });
+  if (bad) return;
+  std::vector<int32_t> first, blk(s.neq);
+  first.reserve(nodes + 1);
+  for (int32_t q = 0; q < s.neq; q += count[q]) {
+    if (node_at[q] < 0) return;
     first.push_back(q);
-    int n = 0;
-    for (int d = 0; d < B; d++) {
-      const int32_t e = s.id[(size_t)no * B + d];
-      s.p_eq.push_back(e > 0 ? e - 1 : -1);
-      if (e <= 0) continue;
-      if (e - 1 >= s.neq || blk[e - 1] >= 0) return;
-      blk[e - 1] = I;
-      n++;
-    }
-    count.push_back(n);
-    q += n;
   }
   const int nb = (int)first.size();
-  struct Low { int32_t J, off; };
-  std::vector<std::vector<Low>> low(nb);
-  std::atomic<bool> bad{false};
+  if (nb != nodes) return;  // nodes that share equations
+  s.p_eq.resize((size_t)nb * B);
+  parallel_chunks(nb, 65536, [&](int64_t a, int64_t b) {
+    for (int64_t I = a; I < b; I++)
+      for (int d = 0; d < B; d++) {
+        const int32_t e = s.id[(size_t)node_at[first[I]] * B + d] - 1;
+        s.p_eq[I * B + d] = e >= 0 ? e : -1;
+        if (e >= 0) blk[e] = (int32_t)I;
+      }
+  });
+  first.push_back(s.neq);
+  auto width = [&](int I) { return first[I + 1] - first[I]; };  // equations of a node
+  // the lower blocks of every row block, counted and checked, then listed from
+  // each row's start in one array
+  std::vector<int32_t> nlow(nb), nup(nb, 0);
   parallel_chunks(nb, 4096, [&](int64_t I0, int64_t I1) {
     for (int64_t I = I0; I < I1 && !bad.load(std::memory_order_relaxed); I++) {
       const int32_t r0 = first[I], k0 = s.ia[r0] - 1, len0 = s.ia[r0 + 1] - s.ia[r0];
       bool ok = true;
-      for (int32_t k = 0; ok && k < len0;) {
+      int n = 0;
+      for (int32_t k = 0; ok && k < len0; n++) {
         const int32_t c = s.ja[k0 + k] - 1;
-        const int32_t J = blk[c];
-        ok = J < I && first[J] == c && k + count[J] <= len0;
-        for (int b = 1; ok && b < count[J]; b++) ok = s.ja[k0 + k + b] - 1 == c + b;
-        if (!ok) break;
-        low[I].push_back({J, k});
-        k += count[J];
+        const int32_t J = blk[c], w = width(J);
+        ok = J < I && first[J] == c && k + w <= len0;
+        for (int b = 1; ok && b < w; b++) ok = s.ja[k0 + k + b] - 1 == c + b;
+        if (ok) __atomic_fetch_add(&nup[J], 1, __ATOMIC_RELAXED);
+        k += w;
       }
-      for (int a = 0; ok && a < count[I]; a++) {
+      for (int a = 0; ok && a < width((int)I); a++) {
         const int32_t ka = s.ia[r0 + a] - 1;
         ok = s.ia[r0 + a + 1] - s.ia[r0 + a] == len0 + a;
         for (int32_t k = 0; ok && k < len0; k++) ok = s.ja[ka + k] == s.ja[k0 + k];
         for (int t = 0; ok && t < a; t++) ok = s.ja[ka + len0 + t] - 1 == r0 + t;
       }
+      nlow[I] = n;
       if (!ok) bad = true;
     }
   });
   if (bad) return;
   std::vector<int32_t> bia(nb + 1, 0);
-  for (int I = 0; I < nb; I++) {
-    bia[I + 1] += (int32_t)low[I].size() + 1;
-    for (const Low &l : low[I]) bia[l.J + 1]++;
-  }
-  for (int I = 0; I < nb; I++) bia[I + 1] += bia[I];
-  std::vector<Low> row(bia[nb]);
-  std::vector<int32_t> up(nb);
-  for (int I = 0; I < nb; I++) up[I] = bia[I] + (int32_t)low[I].size() + 1;
-  for (int I = 0; I < nb; I++) {
-    int32_t k = bia[I];
-    for (const Low &l : low[I]) {
-      row[k++] = l;
-      row[up[l.J]++] = {I, l.off};
+  for (int I = 0; I < nb; I++) bia[I + 1] = bia[I] + nlow[I] + 1 + nup[I];
+  struct Slot { int32_t J, off; };
+  const std::unique_ptr<Slot[]> row(new Slot[bia[nb]]);
+  parallel_chunks(nb, 8192, [&](int64_t I0, int64_t I1) {
+    for (int64_t I = I0; I < I1; I++) {
+      Slot *r = row.get() + bia[I];
+      const int32_t *c = s.ja.data() + s.ia[first[I]] - 1;
+      int32_t off = 0;
+      for (int q = 0; q < nlow[I]; q++) {
+        const int J = blk[c[off] - 1];
+        *r++ = {J, off};
+        off += width(J);
+      }
+      *r = {(int32_t)I, 0};
     }
-    row[k] = {I, 0};
-  }
+  });
+  // the mirrors, rows in ascending order, so that the upper blocks are sorted
+  std::vector<int32_t> &up = nup;
+  for (int I = 0; I < nb; I++) up[I] = bia[I] + nlow[I] + 1;
+  for (int I = 0; I < nb; I++)
+    for (const Slot *r = row.get() + bia[I], *e = r + nlow[I]; r < e; r++)
+      row[up[r->J]++] = {I, r->off};
   const int ns = (nb + R - 1) / R;
   s.p_ptr.assign(ns + 1, 0);
   for (int sl = 0; sl < ns; sl++) {

@@ -215,10 +215,16 @@ bool ensure_persist(elx_ctx *c) {
     int limit = 0;
     ELX_CUDA(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
     limit -= 2048;  // the kernel's static arrays
-    for (int nc = 1; nc <= elx::kGridCols; nc++)
-      c->persist_mode[nc] = elx::smem_bytes(B, nc, true, rows, slices) <= (size_t)limit    ? 2
-                            : elx::smem_bytes(B, nc, false, rows, slices) <= (size_t)limit ? 1
-                                                                                           : 0;
+    // ELX_RESIDENT_MODE=1: the vectors in L2 whatever fits shared memory, 0: the
+    // launches
+    const char *mode_env = getenv("ELX_RESIDENT_MODE");
+    const int most = mode_env ? atoi(mode_env) : 2;
+    for (int nc = 1; nc <= elx::kGridCols; nc++) {
+      const int mode = elx::smem_bytes(B, nc, true, rows, slices) <= (size_t)limit    ? 2
+                       : elx::smem_bytes(B, nc, false, rows, slices) <= (size_t)limit ? 1
+                                                                                      : 0;
+      c->persist_mode[nc] = std::min(mode, most);
+    }
     if (!c->persist_mode[1]) return false;
     // one cluster in place of the grid, for a small matrix
     cuts.insert(cuts.end(), ccuts.begin(), ccuts.end());
@@ -229,7 +235,7 @@ bool ensure_persist(elx_ctx *c) {
     // pipe for each entry of a group
     const double longer = ptr[nslices] * (1.0 / cl - 1.0 / grid) * 16 * B * B;
     int fit = 0;
-    if (longer <= elx::kClusterGain &&
+    if (longer <= elx::kClusterGain && most == 2 &&
         elx::smem_bytes(B, 1, true, ca.rows, ca.slices) <= (size_t)limit &&
         elx::cluster_call(B, ca, cl, 0, 0, c->stream, &fit) != cudaSuccess) {
       cudaGetLastError();  // no such cluster on this device

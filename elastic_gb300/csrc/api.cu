@@ -559,7 +559,8 @@ void pcg_mixed(elx_ctx *c, double tol, int maxit, elx_info *info) {
       persist ? run_batches(c, kPersistSteps, maxit,
                             [&] { mixed_persist_steps(c, kReplaceEvery, kPersistSteps); }, true)
               : run_batches(c, c->pcg32_graph, 3 + 3.0 / kReplaceEvery, maxit);
-  if (persist) check_pipe_waits(c, kResidentWait);
+  // both slots were read in this solve: two batches at least are launched
+  if (persist && (c->h_wait[0] || c->h_wait[1])) check_pipe_waits(c, kResidentWait);
   // fold the last FP32 piece (zero unless maxit stopped the iteration)
   elx::launch_refine_accumulate(n, c->xs.as<double>(), c->x32.as<float>(), false, c->stream);
   c->launches += 1;

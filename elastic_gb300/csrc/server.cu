@@ -344,10 +344,10 @@ struct SrvRequest {
   bool small_counted = false;  // counted among the gate's small requests
   // device state
   elx_ctx *ctx = nullptr;
-  DBuf vecs;  // b (nrhs x neq), then per load case x, r, p, q
+  // b (nrhs x neq), then per load case x, r, p, q, then a GridSync of each
+  DBuf vecs;
   int blocks = 0;  // of each load case in the cooperative pack (0: packed launches)
   DBuf cuts;       // its slices' cuts between them
-  DBuf sync;       // a GridSync for each load case
   cudaEvent_t ready = nullptr;
   std::vector<int> slots;  // indices into the server's slot scalars
   // result
@@ -427,6 +427,15 @@ double now_s() {
       .count();
 }
 
+// A packed request's vectors, and behind them the words of its teams.
+size_t packed_vec_bytes(size_t n, int nrhs) { return (5 * 8 * n * nrhs + 127) / 128 * 128; }
+size_t packed_bytes(size_t n, int nrhs) {
+  return packed_vec_bytes(n, nrhs) + sizeof(elx::GridSync) * nrhs;
+}
+elx::GridSync *packed_sync(const DBuf &vecs, size_t n, int nrhs) {
+  return reinterpret_cast<elx::GridSync *>(static_cast<char *>(vecs.p) + packed_vec_bytes(n, nrhs));
+}
+
 // Device bytes a request will hold (the allocations of upload_structure,
 // the assembly and the per-load-case vectors), from its prepared structure.
 int64_t estimate_bytes(const SrvRequest &q) {
@@ -453,7 +462,7 @@ int64_t estimate_bytes(const SrvRequest &q) {
     b += 4 * slots * s.bsize * s.bsize + 5 * 4 * n;
     b += 8 * 2 * 16 * elx::grid_cap(8) + (64 << 10);
   } else {
-    b += (5 * 8 * n + sizeof(elx::GridSync)) * q.nrhs;  // per load case
+    b += (int64_t)packed_bytes(n, q.nrhs);             // per load case
   }
   b += 160 << 10;                                      // scalars, partials, padding
   return b;
@@ -557,7 +566,6 @@ void release_request(elx_server *sv, SrvRequest &q) {
   if (q.ctx) {
     q.ctx->release(q.vecs);
     q.ctx->release(q.cuts);
-    q.ctx->release(q.sync);
     elx_destroy(q.ctx);
     q.ctx = nullptr;
   }
@@ -618,7 +626,7 @@ void admit(elx_server *sv, SrvRequest &q) {
     sv->peak_used = std::max<int64_t>(sv->peak_used.load(), sv->used);
     return;  // the estimate stays charged: the block buffers come with the solve
   }
-  c->alloc(q.vecs, 5 * n * q.nrhs * 8);
+  c->alloc(q.vecs, packed_bytes(n, q.nrhs));
   ELX_CUDA(cudaMemcpyAsync(q.vecs.p, q.b0.data(), n * q.nrhs * 8, cudaMemcpyHostToDevice,
                            c->stream));
   q.blocks = sv->pack_capacity > 0 ? elx::pack_blocks(c->s) : 0;
@@ -628,8 +636,8 @@ void admit(elx_server *sv, SrvRequest &q) {
     std::vector<int32_t> cuts(q.blocks + 1);
     for (int k = 0; k <= q.blocks; k++) cuts[k] = (int32_t)((int64_t)nsl * k / q.blocks);
     c->upload(q.cuts, cuts.data(), cuts.size());
-    c->alloc(q.sync, sizeof(elx::GridSync) * q.nrhs);
-    ELX_CUDA(cudaMemsetAsync(q.sync.p, 0, q.sync.bytes, c->stream));
+    ELX_CUDA(cudaMemsetAsync(packed_sync(q.vecs, n, q.nrhs), 0, sizeof(elx::GridSync) * q.nrhs,
+                             c->stream));
     for (int k = 0; k < q.nrhs; k++)
       ELX_CUDA(cudaMemsetAsync(sv->d_col + 1 + q.slots[k], 0, sizeof(elx::PersistCol), c->stream));
     c->sync();  // the cuts' host copy
@@ -897,7 +905,7 @@ void gpu_loop(elx_server *sv) {
               a.sr = x + n;
               a.p = x + 2 * n;
               a.cols = sv->d_col + 1 + q->slots[k];
-              a.gs = q->sync.as<elx::GridSync>() + k;
+              a.gs = packed_sync(q->vecs, n, q->nrhs) + k;
               a.err = reinterpret_cast<int32_t *>(sv->d_col);
               a.tol = q->tol;
               a.maxit = q->maxit;

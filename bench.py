@@ -365,7 +365,9 @@ def run_ours(args, dist: Dist):
             "pcg_ms": pcg_ms, "pcg_iter_gbs": iter_gbs, "spmv_ms": spmv_ms,
             "spmv_gbs": spmv_gbs, "wall_s": wall,
             "roofline": {"bound": "hbm",
-                         "kernel": "sell_spmv_kernel<double> (FP64 sliced node-block SpMV + fused (p, Kp))",
+                         "kernel": "sell_spmv_kernel<double> (FP64 sliced node-block SpMV + fused (p, Kp)), "
+                                   "timed alone; the step's iterations do the same product inside "
+                                   "pcg_persist_kernel",
                          "achieved": spmv_gbs, "peak": peak, "unit": "GB/s",
                          "frac": spmv_gbs / peak, "peak_kind": peak_kind,
                          "algorithmic_bytes_per_launch": spmv_bytes,

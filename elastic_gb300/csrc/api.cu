@@ -479,10 +479,10 @@ void set_scalars(elx_ctx *c, double tol, int maxit) {
                            c->stream));
 }
 
-// Iterations of a launch of the cooperative PCG: long solves stay in launches
-// of some ms, and the state's round trip between two is under 1 % of them.  A
-// server's block solve, whose batches are held back for small requests, takes
-// shorter ones.
+// Iterations of a launch of the resident PCG: 3 ms at 2,176 equations, 65 ms at
+// 811,200, so that the state's round trip between two launches is under 1 % of
+// them.  A server's block solve, whose batches are held back for small requests,
+// takes shorter ones.
 constexpr int kPersistSteps = 512, kPersistGatedSteps = 32;
 
 void pcg64(elx_ctx *c, double tol, int maxit, elx_info *info) {

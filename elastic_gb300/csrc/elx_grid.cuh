@@ -10,8 +10,9 @@
 // block that adds the partials a fence, an atomic and two more round trips.
 // The words are never reset: a total is their difference from the last one.
 //
-// The window reaches 32 bits above the sum's reference (the last residual's
-// norm) and 120 below.  A partial above it, an infinity or a NaN marks the
+// The window reaches 120 bits below the sum's reference (the last residual's
+// norm), and takes partials up to 30 above (two bits are left for the carries of
+// the sum and its sign).  A partial above that, an infinity or a NaN marks the
 // sum, and all blocks repeat it through slots, each with its own exponent.
 #pragma once
 

@@ -5,7 +5,8 @@
 // These launches solve what the resident ones (persist.cu, persist_mixed.cu)
 // do not take: matrices whose vectors do not fit a block's shared memory even
 // without the copies, partly fixed nodes in mixed precision, the tiled
-// product, and contexts whose memory budget has no room for the plan.
+// product, contexts whose memory budget has no room for the plan, and processes
+// in which its blocks cannot all run at once.
 //
 // One PCG iteration is three kernels that keep every scalar on the device,
 // so the host never waits inside the loop:

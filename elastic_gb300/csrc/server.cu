@@ -964,9 +964,9 @@ void gpu_loop(elx_server *sv) {
                                    cudaMemcpyHostToDevice, sv->stream));
         repack = false;
       }
-      // 3. PCG iterations of every active load case, then the poll: poll_steps
-      // of packed launches, four times as many in cooperative ones (a team's
-      // vectors come from and go to L2 once a launch)
+      // 3. PCG iterations of every active load case, then the poll: poll_steps,
+      // or four times as many of both kinds while there are teams (their vectors
+      // come from and go to L2 once a launch)
       const int steps = npack ? 4 * sv->poll_steps : sv->poll_steps;
       if (npack) {
         elx::pack_words_kernel<<<npack, 96, 0, sv->stream>>>(sv->d_pack);

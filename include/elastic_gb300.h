@@ -188,12 +188,16 @@ int elx_solve(elx_ctx *ctx, int32_t solver, int32_t precision, double tol,
               int32_t maxit, int32_t ngram, const double *b, double *x,
               elx_info *info);
 
-/* Block PCG: nrhs load cases of the resident matrix, solved `width`
- * columns at a time over one read of the matrix per iteration (each column is
- * the reference's Jacobi PCG with its own scalars and stopping test; pcg,
- * Iters.f:252-524).  b and x are neq x nrhs, column-major; info has nrhs
- * entries (refinements = FP64 residual replacements of the mixed solver).
- * width 0 = autotuned (elx_autotune_block); otherwise 1, 2, 4, 8 or 16.
+/* Block PCG: nrhs load cases of the resident matrix, several columns at a
+ * time over one read of the matrix per iteration (each column is the
+ * reference's Jacobi PCG with its own scalars and stopping test; pcg,
+ * Iters.f:252-524).  b and x are neq x nrhs, column-major, and may share
+ * memory; info has nrhs entries (refinements = FP64 residual replacements of
+ * the mixed solver).  width is 0, 1, 2, 4, 8 or 16.  ELX_PREC_MIXED solves
+ * blocks of width columns (0 = autotuned, elx_autotune_block).  In FP64 width
+ * is the most columns that go together (0 = no limit): up to six in one
+ * resident launch, or, where more than six cost less that way, blocks of width
+ * (0 = autotuned).
  * Needs node blocks: every node all free or all fixed.  No reference
  * counterpart (the reference solves one load case per solv call,
  * Main.f:820-826).  _device: b and x are device pointers. */
@@ -231,8 +235,9 @@ typedef struct elx_server_opts {
   int32_t device;
   int32_t prep_threads; /* host threads building structures (0: 4)          */
   int64_t hbm_budget;   /* device bytes for admitted requests (0: no limit)  */
-  int32_t poll_steps;   /* PCG iterations between polls (0: 8); the          */
-                        /* cooperative pack takes 2 to 12 times as many      */
+  int32_t poll_steps;   /* PCG iterations between polls (0: 8); teams of      */
+                        /* blocks take 2 to 12 times as many, and load cases */
+                        /* too large for a team 4 times beside them          */
   int32_t max_slots;    /* load cases in flight at most (0: 4096)            */
   int32_t large_dofs;   /* requests with at least this many equations are   */
                         /* solved whole, not packed (0: 100000)             */

@@ -148,7 +148,11 @@ __device__ __forceinline__ void block_sum(double (&v)[NV]) {
 
 // Writes this block's NV partials and returns true in thread 0 of the last
 // block to arrive, after which that thread may read every block's partials.
-template <int NV>
+// The ticket counts to the grid's size and gather_partials sets it back; with
+// MOD (at least the grid's size) a launch adds MOD to it whatever its grid (block
+// 0 the difference beforehand), and the last to arrive completes a multiple:
+// nobody sets it back, and launches that overlapped leave it as any others do.
+template <int NV, unsigned int MOD = 0>
 __device__ __forceinline__ bool publish_partials(const double (&v)[NV], double *partials,
                                                  unsigned int *counter) {
   __shared__ bool last;
@@ -156,16 +160,17 @@ __device__ __forceinline__ bool publish_partials(const double (&v)[NV], double *
 #pragma unroll
     for (int i = 0; i < NV; i++) partials[(size_t)i * gridDim.x + blockIdx.x] = v[i];
     __threadfence();
+    if (MOD && blockIdx.x == 0) atomicAdd(counter, MOD - gridDim.x);
     const unsigned int ticket = atomicAdd(counter, 1u);
-    last = ticket == gridDim.x - 1;
+    last = MOD ? ticket % (MOD ? MOD : 1u) == MOD - 1 : ticket == gridDim.x - 1;
   }
   __syncthreads();
   return last;
 }
 
 // In the last block: every thread sums a strided slice of the partials, then
-// a fixed tree; thread 0 gets the totals and resets the counter.
-template <int NV>
+// a fixed tree; thread 0 gets the totals and resets the counter (without MOD).
+template <int NV, unsigned int MOD = 0>
 __device__ __forceinline__ void gather_partials(double (&tot)[NV], const double *partials,
                                                 unsigned int *counter) {
   __threadfence();
@@ -180,7 +185,7 @@ __device__ __forceinline__ void gather_partials(double (&tot)[NV], const double 
     tot[i] = s;
   }
   block_sum<NV>(tot);
-  if (threadIdx.x == 0) *counter = 0u;
+  if (MOD == 0 && threadIdx.x == 0) *counter = 0u;
 }
 
 

@@ -265,6 +265,8 @@ spmv_pipe_kernel(const T *__restrict__ al, const T *__restrict__ ad, const int32
   }
 }
 
+constexpr int kNoAllocMaxBlocks = 16384;  // partial sums in the scratch of kEpiDot
+
 // Two-sided gather: LANES threads per row stride over the row's lower
 // entries and over its upper entries (column i of L through the transposed
 // copy), UNROLL entries in flight per thread, then a fixed shuffle tree.
@@ -347,9 +349,10 @@ gather_spmv_kernel(int neq, const int32_t *__restrict__ ia, const int32_t *__res
   if (!DOT) return;
   double vb[NV];
   block_sum_widen<NV>(v, vb);
-  if (!publish_partials<NV>(vb, partials, counter)) return;
+  constexpr unsigned int MOD = EPI == kEpiDot ? kNoAllocMaxBlocks : 0;
+  if (!publish_partials<NV, MOD>(vb, partials, counter)) return;
   double tot[NV];
-  gather_partials<NV>(tot, partials, counter);
+  gather_partials<NV, MOD>(tot, partials, counter);
   if (threadIdx.x == 0) {
     if (EPI == kEpiPcg) {
       sc->pq = tot[0];
@@ -552,17 +555,16 @@ void launch_gather_epi64(const CsrcDev &k, int epi, const double *x, double *y, 
 namespace elx {
 namespace {
 
-constexpr int kNoAllocMaxBlocks = 16384;       // partial sums in the scratch
 constexpr int64_t kNoAllocMaxRows = 1 << 20;   // the documented limit
 // Two lanes per row, eight entries in flight each: the columns are 32-bit here
 // (no offsets), and fewer lanes per row idle less in a row's last step and need
 // one shuffle add instead of two (330,750 rows of 74 entries: 99.5 us; lanes x
 // entries 4 x 4 102.5, 4 x 2 106.7, 2 x 4 108.9, 1 x 8 120, 8 x 4 149).  Shorter
-// rows gain too; with integer block sums and one launch beside the ticket's
-// reset, us a call before and now, repeated / with a cold L2: HEXA8 of 285,660
-// rows 91.9 / 98.3 and 76.2 / 80.9, TETRA4 of 147,852 43.1 / 49.2 and 27.6 / 39.9,
-// QUAD4 of 701,400 117.6 / 120.8 and 71.7 / 76.8, TRIA3 of 401,000 69.9 / 73.8 and
-// 37.9 / 48.1, TRIA3 of 32 13.8 / 16.5 and 8.4 / 11.3.
+// rows gain too; with integer block sums as one launch, us a call before and
+// now, repeated / with a cold L2: HEXA8 of 285,660 rows 91.9 / 98.3 and 75.2 / 79.9,
+// TETRA4 of 147,852 43.1 / 49.2 and 26.9 / 38.7, QUAD4 of 701,400 117.6 / 120.8
+// and 70.0 / 75.8, TRIA3 of 401,000 69.9 / 73.8 and 37.1 / 47.1, TRIA3 of 32 13.8 /
+// 16.5 and 7.2 / 10.2.
 constexpr int kNoAllocLanes = 2;
 constexpr int kNoAllocRowsPerBlock = 256 / kNoAllocLanes;
 static_assert(kNoAllocMaxRows / kNoAllocRowsPerBlock <= kNoAllocMaxBlocks, "scratch too small");
@@ -600,12 +602,10 @@ extern "C" int elx_spmv_dot_noalloc(int32_t neq, const int32_t *ia, const int32_
     g_noalloc_addr[dev].store(sc, std::memory_order_release);
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // The ticket is set to zero for each call, although a launch leaves it there:
-  // calls that overlapped (they race for the scratch) may not have, and every
-  // later call of the process would then add its dot too early or never.  The
-  // last block writes *xy.
-  if (cudaMemsetAsync(&sc->counter, 0, sizeof(unsigned int), st) != cudaSuccess)
-    return ELX_ERR_CUDA;
+  // One launch, whose last block writes *xy.  Calls that overlap race for the
+  // scratch; the ticket is a multiple of kNoAllocMaxBlocks after them as after
+  // any others, so that the next call by itself is right (set to zero by a memset
+  // for each call: up to 2 us more).
   const int grid = (neq + kNoAllocRowsPerBlock - 1) / kNoAllocRowsPerBlock;
   gather_spmv_kernel<double, kNoAllocLanes, 8, kEpiDot, 1><<<grid, 256, 0, st>>>(
       neq, ia, ja, al, iat, jat, alt, ad, x, y, nullptr, nullptr, sc->partials, &sc->counter,

@@ -382,7 +382,10 @@ void derive_structure(const Mesh &m, Structure &s) {
       int q = s.id[(size_t)v * m.ndf + d];
       if (q > 0) first[v] = q;  // smallest free equation of the node
     }
-  std::atomic<bool> missing{false};
+  // An element that names a node with free dofs twice has no slot for that pair
+  // (the assembly kernels would write before the node's rows) and its entries
+  // are not distinct; with the node fixed nothing is added for it.
+  std::atomic<bool> missing{false}, twice{false};
   parallel_chunks(m.numel, 16384, [&](int64_t t0, int64_t t1) {
     for (int64_t t = t0; t < t1; t++) {
       int el = s.elem_order[t];
@@ -393,7 +396,11 @@ void derive_structure(const Mesh &m, Structure &s) {
         for (int b = a + 1; b < nen; b++, pair++) {
           if (a >= nv || b >= nv) continue;
           int va = c[a] - 1, vb = c[b] - 1;
-          if (!first[va] || !first[vb] || va == vb) continue;
+          if (!first[va] || !first[vb]) continue;
+          if (va == vb) {
+            twice = true;
+            continue;
+          }
           int hi = first[va] > first[vb] ? va : vb;
           int lo = hi == va ? vb : va;
           int32_t r = first[hi] - 1;  // 0-based row of the higher node's first dof
@@ -408,6 +415,7 @@ void derive_structure(const Mesh &m, Structure &s) {
         }
     }
   });
+  ELX_REQUIRE(!twice, ELX_ERR_ARG, "an element names a node with free dofs twice");
   ELX_REQUIRE(!missing, ELX_ERR_ARG, "CSRC pattern does not contain an element's node pair");
 }
 
